@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cmath>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -65,7 +66,6 @@ struct Status {
     uint32_t spin_where;
     uint32_t density_passes;       // density passes executed (not skipped after convergence)
     uint32_t converged;            // set by a density pass whose error met the target
-    uint32_t done_blocks;          // last-block counter of the density pass reduction
     uint32_t converged_substeps;   // substeps in which a density pass met the target
     uint32_t pass_index;           // solve loop graph: index of the first pass of the current body run
     uint32_t loop_iters;           // solve loop graph: body runs since the context was created
@@ -78,6 +78,41 @@ struct Status {
     uint32_t bar_gen;              // persistent solve: grid barriers released so far
     unsigned long long loop_e1;    // persistent solve: error sums of the current pass (2^-24 fixed point)
     unsigned long long loop_e2;
+};
+
+// Sums of one density pass, handed to the position update behind it without a last
+// block: every density block adds its two integer error sums and whether a kernel width
+// differed to the current slot, striped over 16 lines (the two dies' L2 passes one line
+// back and forth at about 25 ns a write, so 8 000 warps storing a flag to one word cost
+// 150 us), and the position update reads them.  Two slots alternate: the density pass
+// adds to slot `cur_density` and copies that number to `cur_update` (its block 0); the
+// position update reads slot `cur_update`, clears the other slot and makes it
+// `cur_density`.  No kernel writes a word that its own blocks read, and no host state is
+// involved, so any sequence of passes may be captured and replayed.
+constexpr int kSumStripes = 16;
+struct PassSync {
+    // [slot][stripe]: compression error, absolute error (2^-24 fixed point), blocks that met
+    // a kernel width other than particle 0's; one 128-byte line each
+    unsigned long long e[2][kSumStripes][16];
+    uint32_t cur_density;
+    uint32_t cur_update;
+    uint32_t pool_used[2];  // entries taken of the two tile plans' pools
+    uint32_t pad[28];
+};
+
+// The neighbour rows of a substep rewritten for the tiled passes (solver.cu).
+constexpr int kTileHalo = 640;  // halo entries of a tile; one that fills it reads the list's own rows
+constexpr int kTileDepth = 64;  // row entries rewritten as offsets; the rest of a longer row goes to the pool
+constexpr uint32_t kHaloOver = 0xffffffffu, kNoParticle = 0xffffffffu;
+struct TilePlan {
+    uint32_t *halo;        // [tile * kTileHalo + slot]: particles outside the tile
+    uint4 *tile;           // per tile: halo entries (kHaloOver: they did not fit), particles, largest |radius|, 0
+    uint32_t *lane;        // [tile * T + rank]: the tile's particles by falling row length, place in the tile
+                           // | row length << 8; kNoParticle past the list's end
+    uint2 *rows;           // [(tile * kTileDepth / 4 + q) * T + rank]: entries 4q..4q+3 as 16-bit record offsets
+    uint32_t *tail;        // per particle with a longer row: where its rest starts in the pool (all ones: not there)
+    uint32_t *pool, *pool_used;
+    uint32_t pool_size;
 };
 
 // Device length block.
@@ -227,6 +262,8 @@ struct apbf_ctx {
     uint32_t *t_keep = nullptr;    // per transfer: kept after particle_transfer
     uint32_t *t_scan = nullptr;    // per transfer: inclusive scan of t_keep
 
+    apbf::TilePlan tile_plan[2] = {};     // of the neighbour rows, of the transposed rows
+    apbf::PassSync *pass_sync = nullptr;  // density sums on their way to the position update
     double *red_partials = nullptr;
     double *red_out = nullptr;
     int red_blocks = 0;
@@ -257,6 +294,7 @@ struct apbf_ctx {
     apbf::ProfSlot *prof_open = nullptr;
     bool capturing = false;        // launches go into a graph being built: not counted
 
+    bool shape_set = false;  // launch shapes given by apbf_set_tuning / apbf_autotune: pass_shape() leaves them alone
     apbf_tuning tuning = {1u, 256u, 8u, 0u, 0u, 0u, 0u, 0u};  // launch shapes (apbf_set_tuning / apbf_autotune)
 
     // solve loop graphs (graph.cu)
@@ -359,6 +397,25 @@ inline int grid_for(const apbf_ctx *ctx, uint32_t n, int block = kBlock, int per
     return (int)(need < cap ? need : cap);
 }
 
+// target = m 2^-(s + 24) with m < 2^24, for error_meets_target.  s is clamped to 63
+// (then n m < 2^55 gives the limit 0) and to -8 (a target of 256 and more: every term
+// saturates at 128, so with the largest m any sum meets it).
+inline void split_target(float target, uint32_t &m, int &s) {
+    m = 0;
+    s = 0;
+    if (!(target > 0.0f)) return;
+    int e = 0;
+    const float f = std::isinf(target) ? 0.5f : std::frexp(target, &e);  // target = f 2^e, f in [0.5, 1)
+    if (std::isinf(target) || e > 8) {
+        m = 1u << 23;
+        s = -8;
+        return;
+    }
+    m = (uint32_t)std::ldexp(f, 24);
+    s = -e;  // m 2^(e - 24) = m 2^-(s + 24)
+    if (s > 63) s = 63;
+}
+
 // float -> int32 truncating toward zero, saturating, NaN -> 0 (rule C4), on the host
 inline int32_t f2i_host(float x) {
     if (!(x == x)) return 0;
@@ -398,10 +455,17 @@ struct SolveOpts {
     int prev_mode = 0;        // lambda_prev: 0 off, 1 reset, 2 add the applied lambda
     bool projected = false;   // with prev_mode 2: pull-back up to the substep's accumulated push
     bool later_pass = false;  // not the first pass of a substep (the widths' uniformity is known)
+    bool behind = true;       // a pass behind another one's position update in the stream
+    bool tiles = false;       // over the tiles of tile_rows (the substep's rows, unchanged since)
     int loop_offset = -1;     // >= 0: a pass of the solve loop graph, number = pass_index + offset;
     uint32_t max_passes = 0;  //   skipped from max_passes on, box after it unless it is the last
 };
 apbf_status incompressibility(apbf_ctx *ctx, cudaStream_t s, const SolveOpts &o = SolveOpts());
+// The tiled passes: whether the solve qualifies, and the rewriting of the rows the
+// search left (with the transposed rows too where the update may need them).
+apbf_status tiles_prepare_device();  // kernel attributes on the current device
+bool tiles_eligible(const apbf_ctx *ctx);
+apbf_status tile_rows(apbf_ctx *ctx, cudaStream_t s, bool transposed);
 // Passes 1.. of a substep as one persistent cooperative kernel with grid barriers
 // between the density and position phases; APBF_ERR_INVALID_ARG when the solve
 // does not qualify (then the caller uses the per-pass or graph forms).
@@ -444,7 +508,8 @@ apbf_status mlp_train_step(float *P, float *m, float *v, float *partials, const 
                            uint32_t nrows, float lr, float over_weight, uint32_t step, float *grad_out,
                            float *loss_out, cudaStream_t s);
 uint32_t mlp_partials_floats(uint32_t nrows);
-apbf_status mlp_lambda(apbf_ctx *ctx, cudaStream_t s, bool early_exit);
+// target > 0 (with its split_target form): no update when the pass's density met it.
+apbf_status mlp_lambda(apbf_ctx *ctx, cudaStream_t s, float target, uint32_t target_m, int target_s);
 // Packs a parameter vector into the inference kernel's shared-memory image
 // (mlp_image_bytes() bytes, 16-byte aligned).
 apbf_status mlp_pack(const float *P, void *image, cudaStream_t s);
@@ -478,6 +543,46 @@ __device__ __forceinline__ uint32_t wait_limit(const Status *st, uint32_t dflt, 
     return l ? l : dflt;
 }
 
+// The sums of a density pass (see PassSync), read by one whole warp.
+struct PassTotals {
+    unsigned long long e1, e2;
+    bool kw_diff;
+};
+__device__ __forceinline__ PassTotals pass_totals(const PassSync *sync, uint32_t slot) {
+    const uint32_t lane = threadIdx.x & 31u;
+    PassTotals t = {0ull, 0ull, false};
+    unsigned long long d = 0ull;
+    if (lane < (uint32_t)kSumStripes) {
+        const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2 *>(sync->e[slot][lane]));
+        d = __ldcg(&sync->e[slot][lane][2]);
+        t.e1 = v.x;
+        t.e2 = v.y;
+    }
+#pragma unroll
+    for (int off = kSumStripes / 2; off > 0; off >>= 1) {
+        t.e1 += __shfl_xor_sync(0xffffffffu, t.e1, off);
+        t.e2 += __shfl_xor_sync(0xffffffffu, t.e2, off);
+    }
+    t.e1 = __shfl_sync(0xffffffffu, t.e1, 0);
+    t.e2 = __shfl_sync(0xffffffffu, t.e2, 0);
+    t.kw_diff = __any_sync(0xffffffffu, d != 0ull);
+    return t;
+}
+
+// Whether the mean compression error of a density pass, fl(t1 2^-24 / n) in FP64, is
+// at most the target = target_m 2^-(target_s + 24) (split_target), as every thread of
+// the kernels behind the pass decides it: in integers, because an FP64 division per
+// warp would cost more than the rest of a small block's work.  t1 <= n target exactly
+// when t1 <= floor(n target_m 2^-target_s); rounding can only pull the next integer
+// down to the target, so that one is divided as the books of the pass divide it.
+__device__ __forceinline__ bool error_meets_target(unsigned long long t1, uint32_t n, float target, uint32_t target_m,
+                                                   int target_s) {
+    if (n == 0u) return true;
+    const unsigned long long nm = (unsigned long long)n * target_m;
+    const unsigned long long limit = target_s >= 0 ? nm >> target_s : nm << -target_s;
+    if (t1 <= limit) return true;
+    return t1 == limit + 1ull && (double)t1 * (1.0 / 16777216.0) / n <= (double)target;
+}
 // Bits of a 10-bit value spread to every third bit (Morton interleave).
 __device__ __host__ __forceinline__ uint32_t spread3(uint32_t x) {
     x &= 0x3ffu;

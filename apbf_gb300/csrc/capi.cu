@@ -298,15 +298,33 @@ apbf_status apbf_create(const apbf_config *cfg, apbf_ctx **out) {
     ctx->coop_blocks = solve_persistent_blocks(ctx->device, ctx->num_sms);
     A(ctx->red_partials, (size_t)6 * ctx->red_blocks);
     A(ctx->red_out, 4);
+    A(ctx->pass_sync, 1);
+    for (int k = 0; k < 2; ++k) {
+        TilePlan &t = ctx->tile_plan[k];
+        const size_t whole = ((size_t)cap + 255u) / 256u * 256u;  // whole tiles of every shape
+        A(t.halo, whole / 32u * kTileHalo);
+        A(t.tile, whole / 32u);
+        A(t.lane, whole);
+        A(t.rows, whole * (kTileDepth / 4));
+        t.pool_size = cfg->max_neighbors > (uint32_t)kTileDepth ? 2u * cap : 0u;
+        A(t.tail, cap);
+        A(t.pool, t.pool_size);
+        t.pool_used = &ctx->pass_sync->pool_used[k];
+    }
     A(ctx->box_min, APBF_MAX_BOXES);
     A(ctx->box_max, APBF_MAX_BOXES);
     A(ctx->box_rot, 3 * APBF_MAX_BOXES);
     A(ctx->emit_state, 8);
     A(ctx->status, 1);
 #undef A
+    if (tiles_prepare_device() != APBF_OK) {
+        apbf_destroy(ctx);
+        return APBF_ERR_CUDA;
+    }
     cudaMemset(ctx->d_len, 0, kLenSlots * sizeof(uint32_t));
     cudaMemset(ctx->status, 0, sizeof(Status));
     cudaMemset(ctx->red_out, 0, 4 * sizeof(double));
+    cudaMemset(ctx->pass_sync, 0, sizeof(PassSync));
     cudaMemset(ctx->nb_count, 0, (size_t)cap * sizeof(uint32_t));
     cudaMemset(ctx->owner, 0xff, (size_t)cap * sizeof(uint32_t));
     for (int k = 0; k < 2; ++k) {
@@ -679,6 +697,14 @@ apbf_status substep_body(apbf_ctx *ctx, float dt, cudaStream_t s, bool capture, 
     // Passes 1.. as one graph launch whose while loop stops on the device (at
     // convergence or after solver_iterations passes), instead of one launch pair per
     // possible pass; not while tracing, debugging or recording.
+    SolveOpts probe;
+    probe.max_passes = (uint32_t)std::max(st.solver_iterations, 0);
+    const bool tiles = tiles_eligible(ctx) && !(defer_loop && batch_solve_eligible(ctx, probe)) &&
+                       !solve_persistent_eligible(ctx, probe);
+    if (tiles) {
+        r = tile_rows(ctx, s, spread || ctx->search_method == APBF_NEIGHBORHOOD_BINARY_SEARCH);
+        if (r != APBF_OK) return r;
+    }
     const bool loop_graph = ctx->use_graphs && !ctx->prof_on && !ctx->debug && !recording &&
                             st.solver_iterations >= 2;
     for (int it = 0; it < st.solver_iterations; ++it) {
@@ -695,6 +721,7 @@ apbf_status substep_body(apbf_ctx *ctx, float dt, cudaStream_t s, bool capture, 
         o.learned = learned && it == 0;
         o.prev_mode = track ? (it == 0 ? 1 : 2) : 0;
         o.projected = projected;
+        o.tiles = tiles;
         if (it == 1 && st.solver_iterations >= 2 && !recording) {
             SolveOpts q = o;
             q.max_passes = (uint32_t)st.solver_iterations;

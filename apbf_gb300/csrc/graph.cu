@@ -57,6 +57,7 @@ static apbf_status capture_loop_body(apbf_ctx *ctx, cudaStream_t cs, cudaGraph_t
         SolveOpts q = o;
         q.loop_offset = k;
         q.box_after = true;  // decided per pass on the device
+        q.behind = k > 0;    // the body starts behind the loop's condition
         r = incompressibility(ctx, cs, q);
     }
     if (r == APBF_OK) {

@@ -337,6 +337,10 @@ struct TcOut {
     int4 *pk;
     int4 *shift;
     Status *st;
+    const PassSync *sync;  // the density pass's error sums
+    float target;          // > 0: the error target, target_m 2^-(target_s + 24)
+    uint32_t target_m;
+    int target_s;
 };
 
 // image != null: the weights arrive by one bulk copy (cp.async.bulk) of the packed
@@ -344,10 +348,14 @@ struct TcOut {
 template <int MODE>
 __global__ void __launch_bounds__(kTcRows) k_mlp_tc(const float *__restrict__ P, const TcImage *image,
                                                     const float *__restrict__ X, uint32_t nrows, const uint32_t *d_len,
-                                                    int early_exit, TcOut o) {
+                                                    TcOut o) {
     __shared__ TcSmem sm;
-    if (MODE == 1 && early_exit && *(volatile const uint32_t *)&o.st->converged) return;  // uniform
     const uint32_t n = MODE == 1 ? d_len[kLenParticles] : nrows;
+    // the density pass before met the target: no update follows (uniform over the grid)
+    if (MODE == 1 && o.target > 0.0f) {
+        const PassTotals t = pass_totals(o.sync, *(volatile const uint32_t *)&o.sync->cur_update & 1u);
+        if (error_meets_target(t.e1, n, o.target, o.target_m, o.target_s)) return;
+    }
     const int tid = threadIdx.x, warp = tid >> 5;
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sm.bar)) : "memory");
@@ -782,7 +790,7 @@ apbf_status mlp_forward(const float *P, const float *X, uint32_t nrows, float *o
     if (nrows == 0) return APBF_OK;
     TcOut o = {};
     o.out = out;
-    k_mlp_tc<0><<<tc_grid(nrows), kTcRows, 0, s>>>(P, nullptr, X, nrows, nullptr, 0, o);
+    k_mlp_tc<0><<<tc_grid(nrows), kTcRows, 0, s>>>(P, nullptr, X, nrows, nullptr, o);
     APBF_CUDA(cudaGetLastError());
     return APBF_OK;
 }
@@ -817,17 +825,20 @@ apbf_status mlp_pack(const float *P, void *image, cudaStream_t s) {
 
 size_t mlp_image_bytes() { return sizeof(TcImage); }
 
-apbf_status mlp_lambda(apbf_ctx *ctx, cudaStream_t s, bool early_exit) {
+apbf_status mlp_lambda(apbf_ctx *ctx, cudaStream_t s, float target, uint32_t target_m, int target_s) {
     TcOut o = {};
     o.selfdir = ctx->selfdir;
     o.rec = ctx->solve_rec;
     o.pk = ctx->solve_pk;
     o.shift = ctx->shift;
     o.st = ctx->status;
+    o.sync = ctx->pass_sync;
+    o.target = target;
+    o.target_m = target_m;
+    o.target_s = target_s;
     APBF_BEFORE_LAUNCH(ctx, s, "k_mlp_tc");
     k_mlp_tc<1><<<tc_grid(ctx->cfg.particle_capacity), kTcRows, 0, s>>>(
-        ctx->mlp_params, reinterpret_cast<const TcImage *>(ctx->mlp_image), ctx->features, 0u, ctx->d_len,
-        early_exit ? 1 : 0, o);
+        ctx->mlp_params, reinterpret_cast<const TcImage *>(ctx->mlp_image), ctx->features, 0u, ctx->d_len, o);
     APBF_AFTER_LAUNCH(ctx, s, "k_mlp_tc");
     return APBF_OK;
 }

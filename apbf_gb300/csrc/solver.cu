@@ -17,6 +17,10 @@
 // as the scatter form, and integer addition is associative, so the gather is
 // bit-identical to the atomic scatter.  Gradients are recomputed in k_delta
 // rather than stored (the reference writes 16 bytes per pair).
+//
+// A substep's passes run over tiles of particles (k_density_tiles, k_delta_tiles: the
+// same terms and sums from shared memory); the direct kernels serve the stage calls, the
+// warm start's feature pass and short solves.
 #include <algorithm>
 #include <cstddef>
 #include <type_traits>
@@ -67,7 +71,7 @@ struct PassA {
     uint32_t *dbg_dens;
     int4 *dbg_grad;
     uint32_t *dbg_sq;
-    long long *partials;  // per block: the two error sums in 2^-24 fixed point, kernel-width bits min << 32 | max
+    PassSync *sync;       // the pass's error sums (2^-24 fixed point) and width uniformity, for the position update
     const uint32_t *d_len;
     Status *st;
     double *red_out;     // [2], [3]: mean compression / absolute error of this pass
@@ -80,9 +84,12 @@ struct PassA {
     uint32_t max_passes;    // loop passes from this number on are skipped
     int4 *filt;             // non-null: Gauss filter deferred to the position pass when rows are symmetric
     float target;        // > 0: set st->converged when the error is at most this
+    uint32_t target_m;   //   = target_m 2^-(target_s + 24) (split_target)
+    int target_s;
     int early_exit;      // skip the pass when st->converged is set
     float rmin3;  // pow(2 * smallestTargetRadius, 3)
     int hk, gk, method, update_b;
+    float one;  // 1, as a value the assembler does not know (see F2)
     float b_speed, b_sgl_factor, b_up_factor;
 };
 
@@ -175,46 +182,6 @@ __device__ __forceinline__ long long err_fix(float x) {
     return x != x ? 0x7fffffffll : (long long)__float2int_rn(__fmul_rn(x, kErrScale));
 }
 
-// Sums of the per-block integer error partials and the min / max of the
-// per-block kernel-width bits (partials of three words per block).
-__device__ __forceinline__ void block_reduce_partials(const long long *partials, int blocks, long long &t1,
-                                                      long long &t2, uint32_t &kmin, uint32_t &kmax) {
-    __shared__ long long s1[32], s2[32];
-    __shared__ uint32_t s3[32], s4[32];
-    long long a = 0, b = 0;
-    uint32_t lo = 0xffffffffu, hi = 0u;
-    for (int k = threadIdx.x; k < blocks; k += blockDim.x) {
-        a += ((volatile const long long *)partials)[3 * k];
-        b += ((volatile const long long *)partials)[3 * k + 1];
-        const unsigned long long w = (unsigned long long)((volatile const long long *)partials)[3 * k + 2];
-        lo = min(lo, (uint32_t)(w >> 32));
-        hi = max(hi, (uint32_t)w);
-    }
-    for (int off = 16; off > 0; off >>= 1) {
-        a += __shfl_down_sync(0xffffffffu, a, off);
-        b += __shfl_down_sync(0xffffffffu, b, off);
-    }
-    lo = __reduce_min_sync(0xffffffffu, lo);
-    hi = __reduce_max_sync(0xffffffffu, hi);
-    if ((threadIdx.x & 31) == 0) {
-        s1[threadIdx.x >> 5] = a;
-        s2[threadIdx.x >> 5] = b;
-        s3[threadIdx.x >> 5] = lo;
-        s4[threadIdx.x >> 5] = hi;
-    }
-    __syncthreads();
-    t1 = 0;
-    t2 = 0;
-    kmin = 0xffffffffu;
-    kmax = 0u;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) {
-        t1 += s1[k];
-        t2 += s2[k];
-        kmin = min(kmin, s3[k]);
-        kmax = max(kmax, s4[k]);
-    }
-}
-
 constexpr int kUnroll = 4;
 
 // L threads per particle ("lanes"): lane s of a particle's group takes row
@@ -228,6 +195,12 @@ __device__ __forceinline__ T group_sum(T v) {
     return v;
 }
 template <int L>
+__device__ __forceinline__ float group_min(float v) {
+#pragma unroll
+    for (int off = L / 2; off > 0; off >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, off));
+    return v;
+}
+template <int L>
 __device__ __forceinline__ int32_t group_wsum(int32_t v) {
 #pragma unroll
     for (int off = L / 2; off > 0; off >>= 1) v = wadd(v, __shfl_xor_sync(0xffffffffu, v, off));
@@ -237,11 +210,142 @@ __device__ __forceinline__ int32_t group_wsum(int32_t v) {
 // XTRA: the warm-start features or the centre-of-mass boundariness sums
 // (method 1) are gathered too; the common pass is compiled without them.
 // Per-thread partial results of a density pass: the two error sums (2^-24 fixed
-// point) and the range of the kernel-width bits.
+// point) and whether a kernel width's bits differed from kw0's.
 struct PassSums {
     long long e1 = 0, e2 = 0;
-    uint32_t kwlo = 0xffffffffu, kwhi = 0u;
+    uint32_t kw0 = 0u;
+    bool kw_diff = false;
 };
+
+// What a density pass has summed over one particle's row.
+struct RowSums {
+    uint32_t dens = 0u, sq = 0u;
+    int32_t gx = 0, gy = 0, gz = 0;
+    int32_t cx = 0, cy = 0, cz = 0, cw = 0;  // method 1: the centre-of-mass sums
+    float div = 0.0f;    // sum_j m_j (v_j - v_i) . gradW_ij  (velocity divergence x density)
+    float nprev = 0.0f;  // sum_j lambda_prev_j (the neighbours' previous-substep lambda sums)
+};
+
+// The rest of a particle's density pass once its row is summed (one thread):
+// incompressibility_2.  Returns whether the boundariness filter is left to the caller
+// (Gauss kernel, not deferred): a neighbour within the cone around ed clears bness[i].
+template <bool GAUSS, bool XTRA>
+__device__ __forceinline__ bool density_finish(const PassA &a, const int4 *pos, uint32_t i, const int4 &p, float kw,
+                                               const KConst &c, const GaussPair &gp, uint32_t cnt, const RowSums &rs,
+                                               float im, float radius, float b, bool feat, bool defer, bool write_rec,
+                                               PassSums &ps, float3 &ed) {
+    bool ask = false;
+    uint32_t dens = rs.dens;
+    const uint32_t sq = rs.sq;
+    const int32_t gx = rs.gx, gy = rs.gy, gz = rs.gz, cx = rs.cx, cy = rs.cy, cz = rs.cz, cw = rs.cw;
+    const float div = rs.div, nprev = rs.nprev;
+    const float W0 = GAUSS ? c.norm : kernel_height(a.hk, 0.0f, kw, c);
+    dens += f2u(W0 / im * APBF_FIX);  // incompressibility_0.comp:32-45 (the self term)
+    // incompressibility_2.comp:77-109
+    const float r2x = 2.0f * radius;
+    const float ird = (r2x * r2x * r2x) * im;
+    const float density = (float)dens * APBF_INV_FIX;
+    const float3 wgs = make_float3((float)gx * APBF_INV_FIX, (float)gy * APBF_INV_FIX, (float)gz * APBF_INV_FIX);
+    float sqs = (float)sq * APBF_INV_FIX;
+    const float wgsq = dot3x(wgs, wgs);
+    const float sgl = sqrtf(wgsq) * ird;
+    sqs += wgsq * im;
+    const float under = 1.0f - density * ird;
+    if (a.update_b) {
+        float bn;
+        if (XTRA && a.method == 1) {
+            float tm = (float)cw * APBF_INV_FIX + 1.0f / im;
+            float3 cv = make_float3((float)cx, (float)cy, (float)cz);
+            bn = sqrtf(dot3x(cv, cv)) / (APBF_FIX * tm) * a.b_sgl_factor;
+        } else {
+            bn = sgl * kw * a.b_sgl_factor + fmaxf(0.0f, under) * a.b_up_factor;
+        }
+        bn = bn >= 1.0f ? 1.0f : 0.0f;
+        float step = bn - b;
+        b = b + fminf(a.b_speed, fmaxf(-a.b_speed, step));
+        b = fminf(1.0f, b);
+    }
+    float lam = under / (ird * ird * (sqs + 0.01f));
+    lam /= a.rmin3 / ird * im;
+    if (a.lambda) a.lambda[i] = lam;
+    // The lambda this pass applies: the reference applies only pushes (lambda < 0,
+    // incompressibility_2.comp:106, incompressibility_3.comp:63).  Projected mode
+    // (warm-started solve) also applies a pull-back lambda > 0 where earlier passes
+    // of this substep pushed, up to their sum, so that an over-push is undone; the
+    // density that pull-back would restore counts as error.
+    float applied = lam < 0.0f ? lam : 0.0f;
+    float pull = 0.0f;
+    if (a.projected && lam > 0.0f) {
+        applied = fminf(lam, -a.lam_prev[i]);  // lam_prev: the sum applied so far (<= 0)
+        if (applied > 0.0f) pull = under * (applied / lam);
+        else applied = 0.0f;
+    }
+    if (write_rec) a.rec[i] = make_float4(applied, c.ivd, c.norm, kw);
+    else if (GAUSS) a.kc[i] = make_float2(gp.ivd36, gp.norm);
+    a.pk[i] = make_int4(p.x, p.y, p.z, __float_as_int(applied));
+    ps.kw_diff = ps.kw_diff || __float_as_uint(kw) != ps.kw0;
+    if (feat) {
+        float *fo = a.features + (size_t)i * 8;
+        fo[0] = (float)cnt;
+        fo[1] = density * ird - 1.0f;
+        fo[2] = kw / radius;
+        fo[3] = lam;
+        fo[4] = density > 0.0f ? div / density : 0.0f;
+        fo[5] = a.lam_prev[i];
+        fo[6] = cnt ? nprev / (float)cnt : 0.0f;
+        fo[7] = 0.0f;
+        a.selfdir[i] = make_float4(-wgs.x * ird, -wgs.y * ird, -wgs.z * ird, im);
+    }
+    int4 sh = make_int4(0, 0, 0, 0);
+    if (applied != 0.0f) {
+        const float sc = applied * im * APBF_FIX;
+        sh.x = f2i(-wgs.x * ird * sc);
+        sh.y = f2i(-wgs.y * ird * sc);
+        sh.z = f2i(-wgs.z * ird * sc);
+    } else if (!(lam >= 0.0f)) {
+        set_flag(a.st, APBF_FLAG_NONFINITE);  // NaN lambda: no shift (int(NaN) = 0)
+    }
+    // incompressibility_3.comp:41-46,60: filter (only changes a non-zero boundariness);
+    // deferred, it is recorded for particles with boundariness, flagged in shift.w
+    if (defer) {
+        if (b > 0.0f) {
+            a.filt[i] = make_int4(gx, gy, gz, 1);
+            sh.w = 1;
+        }
+    } else if (a.method == 2 && b > 0.0f) {
+        if (GAUSS) {
+            ask = filter_dir(gx, gy, gz, ed);
+        } else if (!GAUSS && filter_dir(gx, gy, gz, ed)) {
+            for (uint32_t k = 0; k < cnt; ++k) {
+                const uint32_t j = a.idx[(size_t)k * a.stride + i];
+                const float3 d = fdiff(p, pos[j]);
+                {
+                    float W;
+                    float3 g;
+                    pair_terms<GAUSS>(a.hk, a.gk, d, kw, c, W, g);
+                    float l = sqrtf(dot3x(g, g));
+                    if (!(l > 0.0f)) continue;
+                    float dd = ed.x * (g.x / l) + ed.y * (g.y / l) + ed.z * (g.z / l);
+                    if (dd > 0.6f) {
+                        b = 0.0f;
+                        break;
+                    }
+                }
+            }
+        }
+    }
+    a.shift[i] = sh;
+    a.bness[i] = b;
+    const float ratio = __fmaf_rn(density, ird, -1.0f);  // one rounding of the exact product - 1
+    ps.e1 += err_fix(ratio > 0.0f ? ratio : pull);
+    ps.e2 += err_fix(fabsf(ratio));
+    if (a.dbg_dens) {
+        a.dbg_dens[i] = dens;
+        a.dbg_grad[i] = make_int4(gx, gy, gz, 0);
+        a.dbg_sq[i] = sq;
+    }
+    return ask;
+}
 
 // One particle (row i_raw, lane sub of its group of L) of a density pass:
 // incompressibility_0..2 and the boundariness filter of incompressibility_3.
@@ -264,7 +368,7 @@ __device__ __forceinline__ void density_one(const PassA &a, const int4 *__restri
         // loaded with the particle's other data, so that they are not one more round
         // trip after the neighbour loop
         const float im = a.inv_mass[i], radius = a.radius[i];
-        float b = a.bness[i];
+        const float b = a.bness[i];
         const uint32_t *row = a.idx + i;
         const bool feat = XTRA && a.features != nullptr;
         const float4 vi = feat ? a.vel[i] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -340,182 +444,93 @@ __device__ __forceinline__ void density_one(const PassA &a, const int4 *__restri
             }
         }
         if (!valid || sub != 0) return;
-        const float W0 = GAUSS ? c.norm : kernel_height(a.hk, 0.0f, kw, c);
-        dens += f2u(W0 / im * APBF_FIX);  // incompressibility_0.comp:32-45 (the self term)
-        // incompressibility_2.comp:77-109
-        const float r2x = 2.0f * radius;
-        const float ird = (r2x * r2x * r2x) * im;
-        const float density = (float)dens * APBF_INV_FIX;
-        const float3 wgs = make_float3((float)gx * APBF_INV_FIX, (float)gy * APBF_INV_FIX, (float)gz * APBF_INV_FIX);
-        float sqs = (float)sq * APBF_INV_FIX;
-        const float wgsq = dot3x(wgs, wgs);
-        const float sgl = sqrtf(wgsq) * ird;
-        sqs += wgsq * im;
-        const float under = 1.0f - density * ird;
-        if (a.update_b) {
-            float bn;
-            if (XTRA && a.method == 1) {
-                float tm = (float)cw * APBF_INV_FIX + 1.0f / im;
-                float3 cv = make_float3((float)cx, (float)cy, (float)cz);
-                bn = sqrtf(dot3x(cv, cv)) / (APBF_FIX * tm) * a.b_sgl_factor;
-            } else {
-                bn = sgl * kw * a.b_sgl_factor + fmaxf(0.0f, under) * a.b_up_factor;
+        RowSums rs;
+        rs.dens = dens;
+        rs.sq = sq;
+        rs.gx = gx;
+        rs.gy = gy;
+        rs.gz = gz;
+        rs.cx = cx;
+        rs.cy = cy;
+        rs.cz = cz;
+        rs.cw = cw;
+        rs.div = div;
+        rs.nprev = nprev;
+        float3 ed;
+        if (!density_finish<GAUSS, XTRA>(a, pos, i, p, kw, c, gp, cnt, rs, im, radius, b, feat, defer, write_rec, ps, ed))
+            return;
+        // batches of kUnroll neighbours in row order, software-pipelined as the sums above
+        // (the first hit ends the test, as in the plain loop)
+        uint32_t fj[kUnroll];
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) fj[u] = (uint32_t)u < cnt ? row[(size_t)u * a.stride] : i;
+        bool hit = false;
+        for (uint32_t k0 = 0; k0 < cnt && !hit; k0 += kUnroll) {
+            int4 fq[kUnroll];
+            uint32_t fn[kUnroll];
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) fq[u] = pos[fj[u]];
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) {
+                const uint32_t k = k0 + kUnroll + u;
+                fn[u] = k < cnt ? row[(size_t)k * a.stride] : i;
             }
-            bn = bn >= 1.0f ? 1.0f : 0.0f;
-            float step = bn - b;
-            b = b + fminf(a.b_speed, fmaxf(-a.b_speed, step));
-            b = fminf(1.0f, b);
-        }
-        float lam = under / (ird * ird * (sqs + 0.01f));
-        lam /= a.rmin3 / ird * im;
-        if (a.lambda) a.lambda[i] = lam;
-        // The lambda this pass applies: the reference applies only pushes (lambda < 0,
-        // incompressibility_2.comp:106, incompressibility_3.comp:63).  Projected mode
-        // (warm-started solve) also applies a pull-back lambda > 0 where earlier passes
-        // of this substep pushed, up to their sum, so that an over-push is undone; the
-        // density that pull-back would restore counts as error.
-        float applied = lam < 0.0f ? lam : 0.0f;
-        float pull = 0.0f;
-        if (a.projected && lam > 0.0f) {
-            applied = fminf(lam, -a.lam_prev[i]);  // lam_prev: the sum applied so far (<= 0)
-            if (applied > 0.0f) pull = under * (applied / lam);
-            else applied = 0.0f;
-        }
-        if (write_rec) a.rec[i] = make_float4(applied, c.ivd, c.norm, kw);
-        else if (GAUSS) a.kc[i] = make_float2(gp.ivd36, gp.norm);
-        a.pk[i] = make_int4(p.x, p.y, p.z, __float_as_int(applied));
-        ps.kwlo = min(ps.kwlo, __float_as_uint(kw));
-        ps.kwhi = max(ps.kwhi, __float_as_uint(kw));
-        if (feat) {
-            float *fo = a.features + (size_t)i * 8;
-            fo[0] = (float)cnt;
-            fo[1] = density * ird - 1.0f;
-            fo[2] = kw / radius;
-            fo[3] = lam;
-            fo[4] = density > 0.0f ? div / density : 0.0f;
-            fo[5] = a.lam_prev[i];
-            fo[6] = cnt ? nprev / (float)cnt : 0.0f;
-            fo[7] = 0.0f;
-            a.selfdir[i] = make_float4(-wgs.x * ird, -wgs.y * ird, -wgs.z * ird, im);
-        }
-        int4 sh = make_int4(0, 0, 0, 0);
-        if (applied != 0.0f) {
-            const float sc = applied * im * APBF_FIX;
-            sh.x = f2i(-wgs.x * ird * sc);
-            sh.y = f2i(-wgs.y * ird * sc);
-            sh.z = f2i(-wgs.z * ird * sc);
-        } else if (!(lam >= 0.0f)) {
-            set_flag(a.st, APBF_FLAG_NONFINITE);  // NaN lambda: no shift (int(NaN) = 0)
-        }
-        // incompressibility_3.comp:41-46,60: filter (only changes a non-zero boundariness);
-        // deferred, it is recorded for particles with boundariness, flagged in shift.w
-        if (defer) {
-            if (b > 0.0f) {
-                a.filt[i] = make_int4(gx, gy, gz, 1);
-                sh.w = 1;
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) {
+                if (hit || k0 + u >= cnt) break;
+                hit = gauss_filter_hit(ed, fdiff(p, fq[u]));
             }
-        } else if (a.method == 2 && b > 0.0f) {
-            float3 ed;
-            if (GAUSS && filter_dir(gx, gy, gz, ed)) {
-                // batches of kUnroll neighbours in row order, software-pipelined as the
-                // sums above (the first hit ends the test, as in the plain loop)
-                uint32_t fj[kUnroll];
 #pragma unroll
-                for (int u = 0; u < kUnroll; ++u) fj[u] = (uint32_t)u < cnt ? row[(size_t)u * a.stride] : i;
-                bool hit = false;
-                for (uint32_t k0 = 0; k0 < cnt && !hit; k0 += kUnroll) {
-                    int4 fq[kUnroll];
-                    uint32_t fn[kUnroll];
-#pragma unroll
-                    for (int u = 0; u < kUnroll; ++u) fq[u] = pos[fj[u]];
-#pragma unroll
-                    for (int u = 0; u < kUnroll; ++u) {
-                        const uint32_t k = k0 + kUnroll + u;
-                        fn[u] = k < cnt ? row[(size_t)k * a.stride] : i;
-                    }
-#pragma unroll
-                    for (int u = 0; u < kUnroll; ++u) {
-                        if (hit || k0 + u >= cnt) break;
-                        hit = gauss_filter_hit(ed, fdiff(p, fq[u]));
-                    }
-#pragma unroll
-                    for (int u = 0; u < kUnroll; ++u) fj[u] = fn[u];
-                }
-                if (hit) b = 0.0f;
-            } else if (!GAUSS && filter_dir(gx, gy, gz, ed)) {
-                for (uint32_t k = 0; k < cnt; ++k) {
-                    const uint32_t j = a.idx[(size_t)k * a.stride + i];
-                    const float3 d = fdiff(p, pos[j]);
-                    {
-                        float W;
-                        float3 g;
-                        pair_terms<GAUSS>(a.hk, a.gk, d, kw, c, W, g);
-                        float l = sqrtf(dot3x(g, g));
-                        if (!(l > 0.0f)) continue;
-                        float dd = ed.x * (g.x / l) + ed.y * (g.y / l) + ed.z * (g.z / l);
-                        if (dd > 0.6f) {
-                            b = 0.0f;
-                            break;
-                        }
-                    }
-                }
-            }
+            for (int u = 0; u < kUnroll; ++u) fj[u] = fn[u];
         }
-        a.shift[i] = sh;
-        a.bness[i] = b;
-        const float ratio = __fmaf_rn(density, ird, -1.0f);  // one rounding of the exact product - 1
-        ps.e1 += err_fix(ratio > 0.0f ? ratio : pull);
-        ps.e2 += err_fix(fabsf(ratio));
-        if (a.dbg_dens) {
-            a.dbg_dens[i] = dens;
-            a.dbg_grad[i] = make_int4(gx, gy, gz, 0);
-            a.dbg_sq[i] = sq;
-        }
+        if (hit) a.bness[i] = 0.0f;
     }
 }
 
 // Block sums of the per-thread PassSums, valid in thread 0.
 __device__ __forceinline__ PassSums block_pass_sums(PassSums ps) {
     __shared__ long long s1[8], s2[8];
-    __shared__ uint32_t s3[8], s4[8];
     for (int off = 16; off > 0; off >>= 1) {
         ps.e1 += __shfl_down_sync(0xffffffffu, ps.e1, off);
         ps.e2 += __shfl_down_sync(0xffffffffu, ps.e2, off);
     }
-    ps.kwlo = __reduce_min_sync(0xffffffffu, ps.kwlo);
-    ps.kwhi = __reduce_max_sync(0xffffffffu, ps.kwhi);
     const int w = threadIdx.x >> 5;
     if ((threadIdx.x & 31) == 0) {
         s1[w] = ps.e1;
         s2[w] = ps.e2;
-        s3[w] = ps.kwlo;
-        s4[w] = ps.kwhi;
     }
-    __syncthreads();
     PassSums t;
+    t.kw_diff = __syncthreads_or(ps.kw_diff) != 0;
     if (threadIdx.x == 0) {
         for (int k = 0; k < (int)(blockDim.x >> 5); ++k) {
             t.e1 += s1[k];
             t.e2 += s2[k];
-            t.kwlo = min(t.kwlo, s3[k]);
-            t.kwhi = max(t.kwhi, s4[k]);
         }
     }
     __syncthreads();  // the shared arrays may be reused by the next call
     return t;
 }
 
+// Adds a block's sums to the pass's (one thread).
+__device__ __forceinline__ void add_pass_sums(PassSync *sync, uint32_t slot, const PassSums &bs) {
+    unsigned long long *e = sync->e[slot][blockIdx.x % kSumStripes];
+    if (bs.e1) atomicAdd(&e[0], (unsigned long long)bs.e1);
+    if (bs.e2) atomicAdd(&e[1], (unsigned long long)bs.e2);
+    if (bs.kw_diff) atomicAdd(&e[2], 1ull);
+}
+
 // The end of a density pass, once all its sums are in (one thread): mean errors,
-// width uniformity, pass counter and the convergence flag for the passes that follow.
-__device__ __forceinline__ void finish_pass(const PassA &a, uint32_t n, long long t1, long long t2) {
+// pass counter and, when the error met the target, the flag for the passes that follow.
+__device__ __forceinline__ void finish_pass(double *red_out, Status *st, float target, uint32_t n, long long t1,
+                                            long long t2, bool met) {
     const double inv = 1.0 / (double)kErrScale;
     const double m1 = n ? (double)t1 * inv / n : 0.0, m2 = n ? (double)t2 * inv / n : 0.0;
-    a.red_out[2] = m1;
-    a.red_out[3] = m2;
-    a.st->density_passes += 1u;
-    if (a.target > 0.0f && m1 <= (double)a.target) {
-        a.st->converged = 1u;  // the remaining passes of the substep are skipped
-        a.st->converged_substeps += 1u;
+    red_out[2] = m1;
+    red_out[3] = m2;
+    st->density_passes += 1u;
+    if (target > 0.0f && met) {
+        st->converged = 1u;  // the remaining passes of the substep are skipped
+        st->converged_substeps += 1u;
     }
 }
 
@@ -527,7 +542,11 @@ __global__ void __launch_bounds__(256, GAUSS ? 4 : 3) k_density_lambda(PassA a) 
     // update, which gathers over the same neighbours anyway; filter_tag tells it whether to.
     const bool defer = GAUSS && a.filt && a.method == 2 &&
                        (a.st->range_min == a.st->range_max || a.st->union_rows != 0u);
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.st->filter_tag = (!skip && defer) ? 1u : 0u;
+    const uint32_t slot = *(volatile uint32_t *)&a.sync->cur_density & 1u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a.st->filter_tag = (!skip && defer) ? 1u : 0u;
+        a.sync->cur_update = slot;
+    }
     if (skip) return;  // uniform over the grid
     const uint32_t n = a.d_len[kLenParticles];
     const uint32_t sub = threadIdx.x % L;
@@ -538,31 +557,16 @@ __global__ void __launch_bounds__(256, GAUSS ? 4 : 3) k_density_lambda(PassA a) 
     PassSums ps;
     // the block iterates as a whole (uniform trip count: the group shuffles need every lane)
     const uint32_t gpb = blockDim.x / L;
+    if (blockIdx.x * gpb >= n) return;  // nothing to add
+    ps.kw0 = __float_as_uint(a.kw[0]);
     for (uint32_t base = blockIdx.x * gpb; base < n; base += gridDim.x * gpb)
         density_one<GAUSS, L, XTRA>(a, a.pos, base + threadIdx.x / L, n, sub, defer, write_rec, ps);
+    // The block's sums go to the position update (PassSync), which waits for this kernel
+    // anyway: a last block here (fence, counter, partials read back, FP64 mean) left the
+    // other SMs idle for about 5 us of every pass.
     const PassSums bs = block_pass_sums(ps);
-    __shared__ bool s_last;
     if (threadIdx.x == 0) {
-        const long long t1 = bs.e1, t2 = bs.e2;
-        const uint32_t lo = bs.kwlo, hi = bs.kwhi;
-        a.partials[3 * blockIdx.x] = t1;
-        a.partials[3 * blockIdx.x + 1] = t2;
-        a.partials[3 * blockIdx.x + 2] = (long long)(((unsigned long long)lo << 32) | hi);
-        __threadfence();
-        s_last = atomicAdd(&a.st->done_blocks, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!s_last) return;
-    // the last block: sum of all partials, error and convergence flag for the
-    // passes that follow
-    __threadfence();
-    long long t1, t2;
-    uint32_t kmin, kmax;
-    block_reduce_partials(a.partials, gridDim.x, t1, t2, kmin, kmax);
-    if (threadIdx.x == 0) {
-        a.st->done_blocks = 0u;
-        a.st->kw_uniform = kmin == kmax ? 1u : 0u;  // the position update may gather the packed records
-        finish_pass(a, n, t1, t2);
+        add_pass_sums(a.sync, slot, bs);
     }
 }
 
@@ -583,8 +587,14 @@ struct PassB {
     const uint32_t *ridx;
     uint32_t stride;
     const uint32_t *d_len;
-    const Status *st;
+    Status *st;
+    PassSync *sync;      // this pass's error sums
+    double *red_out;     // [2], [3]: mean compression / absolute error of this pass
+    float target;        // > 0: the error target, target_m 2^-(target_s + 24)
+    uint32_t target_m;
+    int target_s;
     int gk;
+    float one;  // 1, as in PassA
     int early_exit;  // converged: copy the positions unchanged (the buffers swap regardless)
     float *lam_prev;  // prev_mode / acc_mode (0 off, 1 reset, 2 add): accumulate the lambda
     float *lam_acc;   // this pass applied (rec.x: the learned one in a learned pass)
@@ -742,6 +752,26 @@ __device__ __forceinline__ int3 delta_corrections(const PassB &a, const int4 *__
     return acc;
 }
 
+// The end of a particle's position update: the boxes (nboxes > 0), the new position and
+// the books of the lambda lj that this pass applied to it.
+__device__ __forceinline__ void delta_store(const PassB &a, int4 *pos_out, uint32_t j, int4 out, bool hit, float rj,
+                                            float lj, uint32_t nboxes) {
+    if (hit) a.bness[j] = 0.0f;
+    if (nboxes) out = box_push(out, rj, j, a.bmin, a.bmax, a.rot, nboxes);
+    pos_out[j] = out;
+    if (a.prev_mode | a.acc_mode) {
+        accumulate(a.lam_prev, a.prev_mode, j, lj);
+        accumulate(a.lam_acc, a.acc_mode, j, lj);
+    }
+}
+
+// The rest of a particle's position update once its row is summed (one thread).
+__device__ __forceinline__ void delta_finish(const PassB &a, int4 *pos_out, uint32_t j, int4 p, int3 acc, bool hit,
+                                             float rj, float lj, uint32_t nboxes) {
+    int4 out = make_int4(wadd(p.x, acc.x), wadd(p.y, acc.y), wadd(p.z, acc.z), p.w);
+    delta_store(a, pos_out, j, out, hit, rj, lj, nboxes);
+}
+
 // One particle (row j_raw, lane sub of its group of L) of a position update:
 // incompressibility_3 as a gather, the deferred filter, the next iteration's box
 // collision (nboxes > 0) and the lambda bookkeeping.  Every lane of the group
@@ -796,15 +826,9 @@ __device__ __forceinline__ void delta_one(const PassB &a, const int4 *__restrict
             }
         }
         if (!valid || sub != 0) return;
-        if (hit) a.bness[j] = 0.0f;
-        int4 out = make_int4(wadd(p.x, ax), wadd(p.y, ay), wadd(p.z, az), p.w);
-        if (nboxes) out = box_push(out, rj, j, a.bmin, a.bmax, a.rot, nboxes);
-        pos_out[j] = out;
-        if (a.prev_mode | a.acc_mode) {
-            const float lj = __int_as_float(a.pk[j].w);  // applied (learned) lambda
-            accumulate(a.lam_prev, a.prev_mode, j, lj);
-            accumulate(a.lam_acc, a.acc_mode, j, lj);
-        }
+        // applied (learned) lambda
+        const float lj = (a.prev_mode | a.acc_mode) ? __int_as_float(a.pk[j].w) : 0.0f;
+        delta_finish(a, pos_out, j, p, make_int3(ax, ay, az), hit, rj, lj, nboxes);
     }
 }
 
@@ -828,41 +852,870 @@ __device__ __forceinline__ void delta_skip_copy(const PassB &a, uint32_t j) {
     accumulate(a.lam_acc, a.acc_mode, j, 0.0f);
 }
 
-template <bool GAUSS, int L>
-__global__ void __launch_bounds__(256, 4) k_delta(PassB a) {
-    const uint32_t n = a.d_len[kLenParticles];
-    bool skip = a.early_exit && *(volatile const uint32_t *)&a.st->converged;
-    uint32_t nboxes = a.nboxes;
+// What every block of a position update works out before its particles: the list's
+// length, the row forms, whether the pass runs and, in block 0, the books of the
+// density pass behind it (PassSync).  Every calling warp is whole, block 0's first among
+// them.
+struct UpdateHead {
+    uint32_t n, nboxes;
+    bool skip, filter, sym, corr, packed;
+};
+template <bool GAUSS>
+__device__ __forceinline__ UpdateHead update_head(const PassB &a, uint32_t n) {
+    UpdateHead h;
+    h.n = n;
+    const uint32_t slot = *(volatile const uint32_t *)&a.sync->cur_update & 1u;
+    h.skip = a.early_exit && *(volatile const uint32_t *)&a.st->converged;
+    h.nboxes = a.nboxes;
     if (a.loop_offset >= 0) {
         const uint32_t pass = a.st->pass_index + (uint32_t)a.loop_offset;
-        skip = skip || pass >= a.max_passes;
-        if (pass + 1u >= a.max_passes) nboxes = 0u;  // no box collision after the last iteration
+        h.skip = h.skip || pass >= a.max_passes;
+        if (pass + 1u >= a.max_passes) h.nboxes = 0u;  // no box collision after the last iteration
+    }
+    const PassTotals t = pass_totals(a.sync, slot);
+    // every block decides for itself from the sums: block 0 may be setting the flag of
+    // this pass, and reading it early or late gives the same answer
+    const bool ran = !h.skip;
+    if (ran && a.early_exit) h.skip = error_meets_target(t.e1, n, a.target, a.target_m, a.target_s);
+    if (blockIdx.x == 0 && threadIdx.x < 32u) {  // the books of this pass, and the slot of the next
+        if (threadIdx.x < (uint32_t)kSumStripes)
+            for (int k = 0; k < 3; ++k) a.sync->e[slot ^ 1u][threadIdx.x][k] = 0ull;
+        if (threadIdx.x == 0) {
+            if (ran) {
+                a.st->kw_uniform = t.kw_diff ? 0u : 1u;
+                finish_pass(a.red_out, a.st, a.target, n, (long long)t.e1, (long long)t.e2, h.skip);
+            }
+            a.sync->cur_density = slot ^ 1u;
+        }
     }
     // the density pass of this pass deferred the Gauss filter to here (symmetric rows)
-    const bool filter = GAUSS && *(volatile const uint32_t *)&a.st->filter_tag != 0u;
-    if (skip) {
-        if (filter)  // converged: no position update, but the filter still belongs to this pass
-            for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
-                delta_skip_filter(a, a.pos, j);
-        for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
-            delta_skip_copy(a, j);
-        return;
-    }
+    h.filter = GAUSS && *(volatile const uint32_t *)&a.st->filter_tag != 0u;
     // Rows: symmetric (equal radii) or with correction rows (the green search with
     // radii that differ): the particle's own row; transposed rows otherwise.
-    const bool sym = a.st->range_min == a.st->range_max;
-    const bool corr = !sym && a.st->union_rows != 0u;
+    h.sym = a.st->range_min == a.st->range_max;
+    h.corr = !h.sym && a.st->union_rows != 0u;
     // Equal kernel widths (same bits): every neighbour's Gauss constants are this
     // particle's, so one 16-byte record (position, applied lambda) per neighbour is
     // gathered instead of the solve record and the position.
-    const bool packed = GAUSS && a.st->kw_uniform != 0u;
-    const uint32_t *cnt_arr = sym || corr ? a.count : a.rcount;
-    const uint32_t *idx_arr = sym || corr ? a.idx : a.ridx;
+    h.packed = GAUSS && !t.kw_diff;
+    return h;
+}
+// A converged pass: no position update, but its deferred filter still runs.
+__device__ __forceinline__ void update_skipped(const PassB &a, const UpdateHead &h) {
+    if (h.filter)
+        for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < h.n; j += gridDim.x * blockDim.x)
+            delta_skip_filter(a, a.pos, j);
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < h.n; j += gridDim.x * blockDim.x)
+        delta_skip_copy(a, j);
+}
+
+template <bool GAUSS, int L>
+__global__ void __launch_bounds__(256, 4) k_delta(PassB a) {
+    const UpdateHead h = update_head<GAUSS>(a, a.d_len[kLenParticles]);
+    if (h.skip) {
+        update_skipped(a, h);
+        return;
+    }
+    const uint32_t *cnt_arr = h.sym || h.corr ? a.count : a.rcount;
+    const uint32_t *idx_arr = h.sym || h.corr ? a.idx : a.ridx;
     const uint32_t sub = threadIdx.x % L;
     const uint32_t gpb = blockDim.x / L;
-    for (uint32_t base = blockIdx.x * gpb; base < n; base += gridDim.x * gpb)
-        delta_one<GAUSS, L>(a, a.pos, a.pos_out, base + threadIdx.x / L, n, sub, packed, filter, cnt_arr, idx_arr,
-                            corr, nboxes);
+    for (uint32_t base = blockIdx.x * gpb; base < h.n; base += gridDim.x * gpb)
+        delta_one<GAUSS, L>(a, a.pos, a.pos_out, base + threadIdx.x / L, h.n, sub, h.packed, h.filter, cnt_arr, idx_arr,
+                            h.corr, h.nboxes);
+}
+
+// ---- the two passes over tiles of particles ----
+//
+// The direct passes above gather a 16-byte record per pair.  Their warps wait for
+// those gathers (42 % of them leave the L1 at a million particles) and idle a third of
+// their lanes, because neighbouring particles have rows of different lengths.  The rows
+// of a substep do not change between its passes, so for the solve they are rewritten
+// once (k_tile_rows): T consecutive particles are a tile, the particles outside it
+// that its rows name are its halo (1.6 per particle at T = 128, against 14 to 22 row
+// entries), row entries become 16-bit byte offsets of records (the tile's T, T null
+// records that pad odd rows, the halo's), and the tile's particles are dealt to its
+// threads by falling row length.  A pass then loads a
+// tile's records into shared memory once, with every load in flight together, and
+// its pair loop reads shared memory only.  The pair arithmetic and the integer sums are
+// the direct passes' own, so the results are bit-identical.
+//
+// Entries from kTileDepth on and tiles whose halo exceeds kTileHalo are read from the list's
+// own rows.
+
+__device__ __forceinline__ uint32_t tile_hash(uint32_t j, uint32_t mask) { return (j * 2654435761u >> 16) & mask; }
+
+struct TileRowsArgs {
+    const uint32_t *count, *idx;
+    uint32_t stride;
+    const float *radius;
+    const uint32_t *d_len;
+    const Status *st;
+    int reverse;  // transposed rows: needed when neither symmetric nor correction rows hold
+    TilePlan plan;
+};
+
+template <int T>
+__global__ void __launch_bounds__(256) k_tile_rows(TileRowsArgs a) {
+    constexpr uint32_t S = 256 / T;    // threads per particle
+    constexpr uint32_t kSlots = 2048;  // hash table, at most 32 % full
+    constexpr uint32_t kKept = 8;      // row quads whose table slots are kept from the first walk
+    static_assert(kTileHalo * 2 <= kSlots, "the hash table holds the halo with room to probe");
+    __shared__ uint32_t s_key[kSlots];
+    __shared__ uint16_t s_val[kSlots];
+    __shared__ uint2 s_kept[kKept * T];  // four 16-bit codes: 0x8000 | table slot, or the offset of a tile record
+    __shared__ uint32_t s_bin[64];
+    __shared__ uint16_t s_rank[T];
+    __shared__ uint32_t s_halo, s_rmax;
+    if (a.reverse && (a.st->range_min == a.st->range_max || a.st->union_rows != 0u)) return;
+    const uint32_t n = a.d_len[kLenParticles];
+    const uint32_t o = threadIdx.x % T, sub = threadIdx.x / T;  // a warp reads consecutive particles' entries
+    for (uint32_t tile = blockIdx.x; tile * T < n; tile += gridDim.x) {
+        const uint32_t base = tile * T, i = base + o;
+        const uint32_t cnt = i < n ? a.count[i] : 0u;
+        const float r = i < n ? fabsf(a.radius[i]) : 0.0f;
+        for (uint32_t k = threadIdx.x; k < kSlots; k += 256) s_key[k] = 0xffffffffu;
+        if (threadIdx.x < 64) s_bin[threadIdx.x] = 0u;
+        if (threadIdx.x == 0) s_halo = s_rmax = 0u;
+        __syncthreads();
+        const uint32_t depth = min(cnt, (uint32_t)kTileDepth);
+        // falling row length: a counting sort (the order among equal lengths is free)
+        const uint32_t bin = 63u - min(cnt, 63u);
+        if (sub == 0) atomicAdd(&s_bin[bin], 1u);
+        const uint32_t rm = __reduce_max_sync(0xffffffffu, __float_as_uint(r));
+        if ((threadIdx.x & 31u) == 0u) atomicMax(&s_rmax, rm);
+        // the code of entry j: the offset of its record when it lies in the tile, else
+        // its slot in the table of the halo, entered when it is not there yet
+        const auto enter = [&](uint32_t j) -> uint32_t {
+            if (j - base < T) return (j - base) * 16u;
+            uint32_t h = tile_hash(j, kSlots - 1);
+            for (;;) {
+                uint32_t was = *(volatile uint32_t *)&s_key[h];
+                if (was == 0xffffffffu) {
+                    if (*(volatile uint32_t *)&s_halo >= kTileHalo) return 0u;  // overflow: bounds the probing too
+                    was = atomicCAS(&s_key[h], 0xffffffffu, j);
+                    if (was == 0xffffffffu) {
+                        const uint32_t slot = atomicAdd(&s_halo, 1u);
+                        if (slot < kTileHalo) {
+                            s_val[h] = (uint16_t)((2 * T + slot) * 16u);
+                            a.plan.halo[(size_t)tile * kTileHalo + slot] = j;
+                        }
+                        return 0x8000u | h;
+                    }
+                }
+                if (was == j) return 0x8000u | h;
+                h = (h + 1u) & (kSlots - 1);
+            }
+        };
+        const auto load4 = [&](uint32_t q, uint32_t (&j)[4]) {
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) j[u] = 4u * q + u < depth ? a.idx[(size_t)(4u * q + u) * a.stride + i] : i;
+        };
+        uint32_t j[4];
+        load4(sub, j);
+#pragma unroll 1
+        for (uint32_t q = sub; 4u * q < depth; q += S) {
+            uint32_t nx[4];
+            load4(q + S, nx);
+            uint32_t c[4];
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) c[u] = 4u * q + u < depth ? enter(j[u]) : (T + o) * 16u;
+            if (q < kKept) s_kept[q * T + o] = make_uint2(c[0] | c[1] << 16, c[2] | c[3] << 16);
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) j[u] = nx[u];
+        }
+        __syncthreads();
+        if (threadIdx.x < 32) {  // exclusive scan of the 64 bins
+            const uint32_t x0 = s_bin[2 * threadIdx.x], x1 = s_bin[2 * threadIdx.x + 1];
+            uint32_t v = x0 + x1;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, v, off);
+                if ((int)threadIdx.x >= off) v += y;
+            }
+            s_bin[2 * threadIdx.x] = v - x0 - x1;
+            s_bin[2 * threadIdx.x + 1] = v - x1;
+        }
+        const uint32_t halo = s_halo;
+        __syncthreads();
+        // (a tile that fills its halo exactly counts as overflowing: the inserts stop there)
+        const bool over = halo >= kTileHalo;
+        if (sub == 0) {
+            const uint32_t k = atomicAdd(&s_bin[bin], 1u);
+            s_rank[o] = (uint16_t)k;
+            a.plan.lane[base + k] = i < n ? o | cnt << 8 : kNoParticle;
+        }
+        // the rest of the long rows, each in one run of the pool: read through the list's
+        // own rows, every entry would touch another page
+        if (sub == 0)
+            for (uint32_t left = __ballot_sync(0xffffffffu, cnt > kTileDepth); left; left &= left - 1u) {
+                const int src = __ffs(left) - 1;
+                const uint32_t li = __shfl_sync(0xffffffffu, i, src), m = __shfl_sync(0xffffffffu, cnt, src) - kTileDepth;
+                const uint32_t lane = threadIdx.x & 31u;
+                uint32_t at = 0;
+                if ((int)lane == src) {
+                    at = atomicAdd(a.plan.pool_used, m);
+                    if (at > a.plan.pool_size || m > a.plan.pool_size - at) at = 0xffffffffu;
+                    a.plan.tail[i] = at;
+                }
+                at = __shfl_sync(0xffffffffu, at, src);
+                if (at != 0xffffffffu)
+                    for (uint32_t k = lane; k < m; k += 32u)
+                        a.plan.pool[at + k] = a.idx[(size_t)(kTileDepth + k) * a.stride + li];
+            }
+        if (threadIdx.x == 0) {
+            a.plan.tile[tile] = make_uint4(over ? kHaloOver : halo, min(n - base, (uint32_t)T), s_rmax, 0u);
+        }
+        __syncthreads();
+        if (!over) {
+            uint2 *out = a.plan.rows + (size_t)tile * (T * kTileDepth / 4) + s_rank[o];
+            const auto offset = [&](uint32_t c) { return c & 0x8000u ? (uint32_t)s_val[c & 0x7fffu] : c; };
+#pragma unroll 1
+            for (uint32_t q = sub; q * 4u < depth; q += S) {
+                uint32_t c[4];
+                if (q < kKept) {
+                    const uint2 k = s_kept[q * T + o];
+                    c[0] = k.x & 0xffffu;
+                    c[1] = k.x >> 16;
+                    c[2] = k.y & 0xffffu;
+                    c[3] = k.y >> 16;
+                } else {
+                    load4(q, j);
+#pragma unroll
+                    for (uint32_t u = 0; u < 4; ++u) c[u] = 4u * q + u < depth ? enter(j[u]) : (T + o) * 16u;
+                }
+                out[q * T] =
+                    make_uint2(offset(c[0]) | offset(c[1]) << 16, offset(c[2]) | offset(c[3]) << 16);
+            }
+        }
+        __syncthreads();  // the shared arrays are the next tile's
+    }
+}
+
+// Two FP32 values in one 64-bit register pair: the packed operations round each half
+// like the scalar ones, at half the issue slots.  The assembler contracts a packed
+// product and a packed sum into one FMA whatever their rounding modifiers and -fmad say,
+// which the passes must not (dot3x): sums are written as fma(a, 1, b), which rounds
+// a + b once, with the 1 taken from the kernel's arguments so that it stays a value.
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 f2_pack(float lo, float hi) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 f2_unpack(F2 a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+    return r;
+}
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b, F2 one) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(one.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ F2 dot3_f2(F2 ax, F2 ay, F2 az, F2 bx, F2 by, F2 bz, F2 one) {
+    return f2_add(f2_add(ax * bx, ay * by, one), az * bz, one);
+}
+__device__ __forceinline__ float ex2_ftz(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// The Gauss height W and the gradient factor s (gradient = s D) of two offsets at
+// once, as gauss_terms_r2 computes them, for exponents of at least -126: below, exp2f
+// scales around the subnormal range, which the flushing form does not.  low collects the
+// smallest exponent; a row in which it fell below is summed again by gauss_terms_r2.
+__device__ __forceinline__ void gauss_two(F2 r2, F2 ivd36, F2 norm, F2 k2, float &low, F2 &W, F2 &s) {
+    const float2 x = f2_unpack(r2 * ivd36);
+    low = fminf(fminf(low, x.x), x.y);
+    W = f2_pack(ex2_ftz(x.x), ex2_ftz(x.y)) * norm;
+    const float2 t = f2_unpack(W * k2), q = f2_unpack(r2);
+    // no gradient below 0.0001 reference units
+    s = f2_pack(q.x < 1.0e-8f * 0x1p36f ? 0.0f : t.x, q.y < 1.0e-8f * 0x1p36f ? 0.0f : t.y);
+}
+constexpr float kLowExponent = -126.0f;
+
+__device__ __forceinline__ const int4 &tile_record(const int4 *s_rec, uint32_t offset) {
+    return *reinterpret_cast<const int4 *>(reinterpret_cast<const char *>(s_rec) + offset);
+}
+__device__ __forceinline__ uint32_t row_offset(uint2 e, uint32_t u) {
+    const uint32_t w = (u & 2u) ? e.y : e.x;
+    return (u & 1u) ? w >> 16 : w & 0xffffu;
+}
+
+// Exact sum over a warp of 32-bit values, as two 16-bit halves.
+__device__ __forceinline__ long long warp_sum32(int32_t v) {
+    const int32_t hi = __reduce_add_sync(0xffffffffu, v >> 16);
+    const uint32_t lo = __reduce_add_sync(0xffffffffu, (uint32_t)v & 0xffffu);
+    return ((long long)hi << 16) + (long long)lo;
+}
+
+// The entries from kTileDepth on of lane src's row, walked by its whole warp: lane l takes
+// entries l, l + 32, ... of them, four loads in flight.  A lane alone would wait two memory
+// latencies for every entry.
+struct WarpRow {
+    const uint32_t *entry;
+    size_t stride;
+    uint32_t m;
+    int4 p;
+    __device__ __forceinline__ WarpRow(const TilePlan &plan, const uint32_t *idx, uint32_t row_stride, uint32_t i_,
+                                       uint32_t cnt_, const int4 &p_, int src) {
+        const uint32_t i = __shfl_sync(0xffffffffu, i_, src);
+        m = __shfl_sync(0xffffffffu, cnt_, src) - kTileDepth;
+        p.x = __shfl_sync(0xffffffffu, p_.x, src);
+        p.y = __shfl_sync(0xffffffffu, p_.y, src);
+        p.z = __shfl_sync(0xffffffffu, p_.z, src);
+        p.w = 0;
+        const uint32_t at = plan.tail[i];
+        entry = at != 0xffffffffu ? plan.pool + at : idx + (size_t)kTileDepth * row_stride + i;
+        stride = at != 0xffffffffu ? 1u : row_stride;
+    }
+    template <typename G, typename F>
+    __device__ __forceinline__ void each(G load, F f) const {
+        for (uint32_t k0 = threadIdx.x & 31u; k0 < m; k0 += 128u) {
+            uint32_t j[4];
+            int4 q[4];
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) j[u] = k0 + 32u * u < m ? entry[(k0 + 32u * u) * stride] : 0u;
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) q[u] = k0 + 32u * u < m ? load(j[u]) : make_int4(0, 0, 0, 0);
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u)
+                if (k0 + 32u * u < m) f(j[u], q[u]);
+        }
+    }
+};
+
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// A tile's density pass: T particles, L threads each.  At a million particles in a
+// waterfall (13.4 M pairs) 62 us against 92 us for the direct kernel, 26 against 35 us at
+// 250 000 (4.45 M pairs).  Bound by the latency of a tile's own loads (three rounds: the
+// plan's words, the records, the barrier): half of a block's time, while the pair loop
+// issues at 55 % of the cycles; so the plan's words come in one round and before the
+// kernel in front has ended, and eight blocks (64 registers) share an SM.
+template <int T, int L>
+__global__ void __launch_bounds__(T *L, 1024 / (T * L)) k_density_tiles(PassA a, TilePlan plan) {
+    extern __shared__ int4 s_pos[];  // the tile's records, its null records, its halo's; w: mass x 2^18
+    constexpr uint32_t B = T * L;
+    const uint32_t n = a.d_len[kLenParticles];
+    const uint32_t sub = threadIdx.x % L, rank = threadIdx.x / L;
+    bool defer = false;
+    uint32_t slot = 0;
+    PassSums ps;
+    for (uint32_t tile = blockIdx.x; tile * T < n || tile == 0u; tile += gridDim.x) {
+        // what stays between the passes of a substep first, in one round of loads (those
+        // beyond the tile's row lengths and halo are not used): with a programmatic launch
+        // they run while the kernel before drains
+        const uint32_t base = tile * T;
+        const uint4 head = plan.tile[tile];
+        const uint32_t lane = plan.lane[base + rank];
+        const uint2 *row = plan.rows + (size_t)tile * (T * kTileDepth / 4) + rank;
+        const uint32_t *halo = plan.halo + (size_t)tile * kTileHalo;
+        const uint32_t h0 = halo[threadIdx.x], h1 = halo[threadIdx.x + B];
+        uint2 e = row[sub * T];
+        if (tile == blockIdx.x) grid_dependency_trigger();
+        const bool over = head.x == kHaloOver;
+        const uint32_t H = over || n == 0u ? 0u : head.x;
+        const bool valid = n != 0u && lane != kNoParticle;
+        const uint32_t o = valid ? lane & 255u : 0u, i = base + o;
+        const uint32_t cnt = valid ? lane >> 8 : 0u;
+        const float kw = a.kw[i], im = a.inv_mass[i], radius = a.radius[i];
+        ps.kw0 = __float_as_uint(a.kw[0]);
+        const uint32_t depth = over ? 0u : min(cnt, (uint32_t)kTileDepth);
+        if (tile == blockIdx.x) {
+            grid_dependency_wait();
+            const bool skip = (a.early_exit && *(volatile uint32_t *)&a.st->converged) ||
+                              (a.loop_offset >= 0 && a.st->pass_index + (uint32_t)a.loop_offset >= a.max_passes);
+            defer = a.filt && a.method == 2 && (a.st->range_min == a.st->range_max || a.st->union_rows != 0u);
+            slot = *(volatile uint32_t *)&a.sync->cur_density & 1u;
+            if (blockIdx.x == 0 && threadIdx.x == 0) {
+                a.st->filter_tag = (!skip && defer) ? 1u : 0u;
+                a.sync->cur_update = slot;
+                a.sync->pool_used[0] = a.sync->pool_used[1] = 0u;  // for the next substep's rows
+            }
+            if (skip || n == 0u) return;  // uniform over the grid
+        }
+        const auto stage = [&](uint32_t k, uint32_t g) {
+            int4 v = a.pos[g];
+            v.w = __float_as_int(__int_as_float(v.w) * APBF_FIX);
+            s_pos[k] = v;
+        };
+        const float b0 = a.bness[i];
+        for (uint32_t k = threadIdx.x; k < T; k += B)
+            if (k < head.y) {
+                const int4 v = a.pos[base + k];
+                s_pos[k] = make_int4(v.x, v.y, v.z, __float_as_int(__int_as_float(v.w) * APBF_FIX));
+                s_pos[T + k] = make_int4(v.x, v.y, v.z, 0);
+            }
+        if (threadIdx.x < H) stage(2 * T + threadIdx.x, h0);
+        if (threadIdx.x + B < H) stage(2 * T + B + threadIdx.x, h1);
+        for (uint32_t k = threadIdx.x + 2 * B; k < H; k += B) stage(2 * T + k, halo[k]);
+        __syncthreads();
+        const int4 p = s_pos[o];
+        const KConst c = gauss_consts(kw);
+        const GaussPair gp = gauss_pair(c);
+        RowSums rs;
+        float low = 0.0f;
+        {
+            const F2 one = f2_pack(a.one, a.one);
+            const F2 ivd = f2_pack(gp.ivd36, gp.ivd36), norm = f2_pack(gp.norm, gp.norm), kk = f2_pack(gp.k2, gp.k2);
+            const auto two = [&](uint32_t w) {
+                const int4 q0 = tile_record(s_pos, w & 0xffffu), q1 = tile_record(s_pos, w >> 16);
+                const F2 dx = f2_pack((float)wadd(q0.x, -p.x), (float)wadd(q1.x, -p.x));
+                const F2 dy = f2_pack((float)wadd(q0.y, -p.y), (float)wadd(q1.y, -p.y));
+                const F2 dz = f2_pack((float)wadd(q0.z, -p.z), (float)wadd(q1.z, -p.z));
+                const F2 m = f2_pack(__int_as_float(q0.w), __int_as_float(q1.w));
+                F2 W, s;
+                gauss_two(dot3_f2(dx, dy, dz, dx, dy, dz, one), ivd, norm, kk, low, W, s);
+                const F2 gx = s * dx, gy = s * dy, gz = s * dz;
+                const float2 tw = f2_unpack(W * m), tx = f2_unpack(gx * m), ty = f2_unpack(gy * m),
+                             tz = f2_unpack(gz * m), tq = f2_unpack(dot3_f2(gx, gy, gz, gx, gy, gz, one) * m);
+                rs.dens += f2u(tw.x) + f2u(tw.y);
+                rs.gx = wadd(rs.gx, wadd(f2i(tx.x), f2i(tx.y)));
+                rs.gy = wadd(rs.gy, wadd(f2i(ty.x), f2i(ty.y)));
+                rs.gz = wadd(rs.gz, wadd(f2i(tz.x), f2i(tz.y)));
+                rs.sq += f2u(tq.x) + f2u(tq.y);
+            };
+            for (uint32_t k = sub * 4u; k < depth; k += L * 4u) {
+                const uint2 cur = e;
+                if (k + L * 4u < depth) e = row[(k / 4u + L) * T];
+                two(cur.x);
+                if (k + 2u < depth) two(cur.y);
+            }
+        }
+        const auto add = [&](int4 q, float mjf) {
+            float W;
+            float3 g;
+            gauss_terms(udiff(p, q), gp, W, g);
+            rs.dens += f2u(W * mjf);
+            rs.gx = wadd(rs.gx, f2i(g.x * mjf));
+            rs.gy = wadd(rs.gy, f2i(g.y * mjf));
+            rs.gz = wadd(rs.gz, f2i(g.z * mjf));
+            rs.sq += f2u(dot3x(g, g) * mjf);
+        };
+        if (L > 1) low = group_min<L>(low);  // the group sums its row again as one
+        if (low < kLowExponent) {  // far out in a narrow kernel: exp2f's own range handling
+            rs = RowSums();
+#pragma unroll 1
+            for (uint32_t k = sub; k < depth; k += L) {
+                const int4 q = tile_record(s_pos, row_offset(row[(k / 4u) * T], k));
+                add(q, __int_as_float(q.w));
+            }
+        }
+        const uint32_t shallow = min(cnt, (uint32_t)kTileDepth);
+#pragma unroll 2
+        for (uint32_t k = depth + sub; k < shallow; k += L) {  // a tile whose halo did not fit
+            const int4 q = a.pos[a.idx[(size_t)k * a.stride + i]];
+            add(q, __int_as_float(q.w) * APBF_FIX);
+        }
+        // what is left of the long rows: one row after the other, by the whole warp
+        for (uint32_t left = __ballot_sync(0xffffffffu, sub == 0u && cnt > kTileDepth); left; left &= left - 1u) {
+            const int src = __ffs(left) - 1;
+            const WarpRow w(plan, a.idx, a.stride, i, cnt, p, src);
+            const GaussPair gw = gauss_pair(__shfl_sync(0xffffffffu, gp.ivd36, src), __shfl_sync(0xffffffffu, gp.norm, src));
+            RowSums t;
+            w.each([&](uint32_t j) { return a.pos[j]; }, [&](uint32_t, const int4 &q) {
+                const float mjf = __int_as_float(q.w) * APBF_FIX;
+                float W;
+                float3 g;
+                gauss_terms(udiff(w.p, q), gw, W, g);
+                t.dens += f2u(W * mjf);
+                t.gx = wadd(t.gx, f2i(g.x * mjf));
+                t.gy = wadd(t.gy, f2i(g.y * mjf));
+                t.gz = wadd(t.gz, f2i(g.z * mjf));
+                t.sq += f2u(dot3x(g, g) * mjf);
+            });
+            const uint32_t d = __reduce_add_sync(0xffffffffu, t.dens), s2 = __reduce_add_sync(0xffffffffu, t.sq);
+            const int32_t x = __reduce_add_sync(0xffffffffu, t.gx), y = __reduce_add_sync(0xffffffffu, t.gy),
+                          z = __reduce_add_sync(0xffffffffu, t.gz);
+            if ((int)(threadIdx.x & 31u) == src) {
+                rs.dens += d;
+                rs.sq += s2;
+                rs.gx = wadd(rs.gx, x);
+                rs.gy = wadd(rs.gy, y);
+                rs.gz = wadd(rs.gz, z);
+            }
+        }
+        if (L > 1) {
+            rs.dens = group_sum<L>(rs.dens);
+            rs.sq = group_sum<L>(rs.sq);
+            rs.gx = group_wsum<L>(rs.gx);
+            rs.gy = group_wsum<L>(rs.gy);
+            rs.gz = group_wsum<L>(rs.gz);
+        }
+        PassSums one;
+        one.kw0 = ps.kw0;
+        float3 ed = make_float3(0.f, 0.f, 0.f);
+        bool ask = false;
+        if (valid && sub == 0)
+            ask = density_finish<true, false>(a, a.pos, i, make_int4(p.x, p.y, p.z, 0), kw, c, gp, cnt, rs, im, radius, b0,
+                                              false, defer, false, one, ed);
+        if (__any_sync(0xffffffffu, ask)) {  // the boundariness filter of transposed rows
+            bool hit = false;
+            if (ask) {
+                uint2 r = depth ? row[0] : make_uint2(0u, 0u);
+#pragma unroll 1
+                for (uint32_t k = 0; k < depth && !hit; k += 4u) {  // (a null record never hits)
+                    const uint2 now = r;
+                    if (k + 4u < depth) r = row[(k / 4u + 1u) * T];
+#pragma unroll
+                    for (uint32_t u = 0; u < 4; ++u)
+                        hit = hit || gauss_filter_hit(ed, fdiff(p, tile_record(s_pos, row_offset(now, u))));
+                }
+#pragma unroll 2
+                for (uint32_t k = depth; k < shallow && !hit; ++k)
+                    hit = gauss_filter_hit(ed, fdiff(p, a.pos[a.idx[(size_t)k * a.stride + i]]));
+            }
+            for (uint32_t left = __ballot_sync(0xffffffffu, ask && !hit && cnt > kTileDepth); left; left &= left - 1u) {
+                const int src = __ffs(left) - 1;
+                const WarpRow w(plan, a.idx, a.stride, i, cnt, p, src);
+                const float3 ew = make_float3(__shfl_sync(0xffffffffu, ed.x, src), __shfl_sync(0xffffffffu, ed.y, src),
+                                              __shfl_sync(0xffffffffu, ed.z, src));
+                bool any = false;
+                w.each([&](uint32_t j) { return a.pos[j]; },
+                       [&](uint32_t, const int4 &q) { any = any || gauss_filter_hit(ew, fdiff(w.p, q)); });
+                any = __any_sync(0xffffffffu, any);
+                if ((int)(threadIdx.x & 31u) == src) hit = any;
+            }
+            if (hit) a.bness[i] = 0.0f;
+        }
+        ps.e1 += warp_sum32((int32_t)one.e1);  // one term each, in 32 bits (err_fix)
+        ps.e2 += warp_sum32((int32_t)one.e2);
+        ps.kw_diff = ps.kw_diff || one.kw_diff;
+        if (tile + gridDim.x < (n + T - 1) / T) __syncthreads();  // the shared records are the next tile's
+    }
+    __shared__ long long s_e[2][B / 32];
+    if ((threadIdx.x & 31u) == 0u) {
+        s_e[0][threadIdx.x / 32u] = ps.e1;
+        s_e[1][threadIdx.x / 32u] = ps.e2;
+    }
+    PassSums bs;
+    bs.kw_diff = __syncthreads_or(ps.kw_diff) != 0;
+    if (threadIdx.x == 0) {
+        for (uint32_t k = 0; k < B / 32u; ++k) {
+            bs.e1 += s_e[0][k];
+            bs.e2 += s_e[1][k];
+        }
+        add_pass_sums(a.sync, slot, bs);
+    }
+}
+
+// Boxes that can move no particle of a tile.  Thread k writes box k's outer faces for the
+// tile's largest |radius|: box_clear's own thresholds, which only move outwards as the
+// radius grows (rounding is monotone), so a position outside them is outside the
+// particle's.  Per box: the faces (w of the first word: 0 axis-aligned, 1 oriented, 2 beyond
+// box_clear's range, then the box itself is asked), the rotation's rows, the centre.
+constexpr uint32_t kTileBoxes = 8, kTileBoxWords = 6;
+__device__ __forceinline__ void tile_box(const PassB &a, uint32_t k, float rmax, float4 *s_box) {
+    const float c = 0.0500001f;
+    const float4 lo = a.bmin[k], hi = a.bmax[k], r0 = a.rot[3 * k];
+    const bool oriented = r0.w != 0.0f;
+    const float3 l = oriented ? make_float3(-hi.x, -hi.y, -hi.z) : make_float3(lo.x, lo.y, lo.z);
+    const float4 b0 = make_float4(__fsub_rn(__fsub_rn(l.x, rmax), c), __fsub_rn(__fsub_rn(l.y, rmax), c),
+                                  __fsub_rn(__fsub_rn(l.z, rmax), c), 0.0f);
+    const float4 b1 = make_float4(__fadd_rn(__fadd_rn(hi.x, rmax), c), __fadd_rn(__fadd_rn(hi.y, rmax), c),
+                                  __fadd_rn(__fadd_rn(hi.z, rmax), c), 0.0f);
+    const float m = fmaxf(fmaxf(fmaxf(fabsf(b0.x), fabsf(b0.y)), fmaxf(fabsf(b0.z), fabsf(b1.x))),
+                          fmaxf(fabsf(b1.y), fabsf(b1.z)));
+    float4 *w = s_box + kTileBoxWords * k;
+    w[0] = make_float4(b0.x, b0.y, b0.z, !(m < 1.0e30f) ? 2.0f : (oriented ? 1.0f : 0.0f));
+    w[1] = b1;
+    if (oriented) {
+        w[2] = r0;
+        w[3] = a.rot[3 * k + 1];
+        w[4] = a.rot[3 * k + 2];
+        w[5] = lo;
+    }
+}
+// The first box that may push v (nb: none).
+__device__ __forceinline__ uint32_t tile_boxes_clear(int4 v, const float4 *s_box, uint32_t nb) {
+    const float px = __fmul_rn((float)v.x, 0x1p-18f), py = __fmul_rn((float)v.y, 0x1p-18f),
+                pz = __fmul_rn((float)v.z, 0x1p-18f);
+    uint32_t first = nb;
+#pragma unroll 1
+    for (uint32_t k = nb; k-- > 0u;) {
+        const float4 *w = s_box + kTileBoxWords * k;
+        const float4 b0 = w[0], b1 = w[1];
+        float qx = px, qy = py, qz = pz;
+        if (b0.w != 0.0f) {  // as box_push takes the position into the box's frame
+            const float4 c = w[5];
+            const float dx = __fsub_rn(px, c.x), dy = __fsub_rn(py, c.y), dz = __fsub_rn(pz, c.z);
+            qx = dot3_rn(w[2], dx, dy, dz);
+            qy = dot3_rn(w[3], dx, dy, dz);
+            qz = dot3_rn(w[4], dx, dy, dz);
+        }
+        const bool clear = b0.w != 2.0f && (qx < b0.x || qy < b0.y || qz < b0.z || qx >= b1.x || qy >= b1.y || qz >= b1.z);
+        if (!clear) first = k;
+    }
+    return first;
+}
+// box_push from box `first` on, where the boxes before it are known to leave ip alone.
+__device__ __noinline__ int4 box_push_from(int4 ip, float r, uint32_t id, const float4 *__restrict__ bmin,
+                                           const float4 *__restrict__ bmax, const float4 *__restrict__ rot,
+                                           uint32_t first, uint32_t nb) {
+    return box_push(ip, r, id, bmin + first, bmax + first, rot + 3 * first, nb - first);
+}
+
+// A tile's position update.  fwd: the plan of the own rows, rev: that of the
+// transposed rows.  86 us at a million particles against 125 us for the direct kernel, 30
+// against 37 us at 250 000.  Of its instructions the deferred filter's row tests took a
+// quarter and the boxes a fifth; both now reject by cheap bounds first.
+template <int T, int L>
+__global__ void __launch_bounds__(T *L, 896 / (T * L)) k_delta_tiles(PassB a, TilePlan fwd, TilePlan rev) {
+    extern __shared__ int4 s_pk[];  // the tile's records, its null records, its halo's; w: lambda x 2^18
+    __shared__ float4 s_box[kTileBoxWords * kTileBoxes];
+    __shared__ UpdateHead s_head;
+    constexpr uint32_t B = T * L;
+    float2 *s_kc = reinterpret_cast<float2 *>(s_pk + 2 * T + kTileHalo);  // their Gauss constants when widths differ
+    const uint32_t n = a.d_len[kLenParticles];
+    // the rows' form is the search's: it stays between the passes too
+    const bool own = a.st->range_min == a.st->range_max || a.st->union_rows != 0u;
+    const TilePlan &plan = own ? fwd : rev;
+    const uint32_t *idx_arr = own ? a.idx : a.ridx;
+    const uint32_t sub = threadIdx.x % L, rank = threadIdx.x / L;
+    UpdateHead h;
+    for (uint32_t tile = blockIdx.x; tile * T < n || tile == 0u; tile += gridDim.x) {
+        const uint32_t base = tile * T;  // (as k_density_tiles starts)
+        const uint4 head = plan.tile[tile];
+        const uint32_t lane = plan.lane[base + rank];
+        const uint2 *row = plan.rows + (size_t)tile * (T * kTileDepth / 4) + rank;
+        const uint32_t *halo = plan.halo + (size_t)tile * kTileHalo;
+        const uint32_t h0 = halo[threadIdx.x], h1 = halo[threadIdx.x + B];
+        uint2 e = row[sub * T];
+        if (tile == blockIdx.x) grid_dependency_trigger();
+        const bool over = head.x == kHaloOver;
+        const uint32_t H = over || n == 0u ? 0u : head.x;
+        const bool valid = n != 0u && lane != kNoParticle;
+        const uint32_t o = valid ? lane & 255u : 0u, j = base + o;
+        const uint32_t cnt = valid ? lane >> 8 : 0u;
+        const uint32_t depth = over ? 0u : min(cnt, (uint32_t)kTileDepth);
+        if (threadIdx.x < min(a.nboxes, kTileBoxes)) tile_box(a, threadIdx.x, __uint_as_float(head.z), s_box);
+        if (tile == blockIdx.x) {
+            grid_dependency_wait();
+            if (threadIdx.x < 32u) {  // its latency runs beside the staging's
+                h = update_head<true>(a, n);
+                if (threadIdx.x == 0) s_head = h;
+            }
+        }
+        const int4 shj = valid ? a.shift[j] : make_int4(0, 0, 0, 0);
+        const float2 kcj = a.kc[j];
+        const int pw = a.pos[j].w;  // the mass rides along
+        const auto stage = [&](uint32_t k, uint32_t g) {
+            int4 v = a.pk[g];
+            v.w = __float_as_int(__int_as_float(v.w) * APBF_FIX);
+            s_pk[k] = v;
+            s_kc[k] = a.kc[g];
+        };
+        for (uint32_t k = threadIdx.x; k < T; k += B)
+            if (n != 0u && k < head.y) {
+                const int4 v = a.pk[base + k];
+                s_pk[k] = make_int4(v.x, v.y, v.z, __float_as_int(__int_as_float(v.w) * APBF_FIX));
+                s_pk[T + k] = make_int4(v.x, v.y, v.z, 0);
+                s_kc[k] = s_kc[T + k] = a.kc[base + k];
+            }
+        if (threadIdx.x < H) stage(2 * T + threadIdx.x, h0);
+        if (threadIdx.x + B < H) stage(2 * T + B + threadIdx.x, h1);
+        for (uint32_t k = threadIdx.x + 2 * B; k < H; k += B) stage(2 * T + k, halo[k]);
+        bool fil = false, hit = false, near = false;  // this particle's deferred filter, a neighbour cleared it or may have
+        float3 ed = make_float3(0.f, 0.f, 0.f);
+        if (shj.w != 0) {  // (only a deferred filter sets it)
+            const int4 fj = a.filt[j];
+            fil = filter_dir(fj.x, fj.y, fj.z, ed);
+        }
+        __syncthreads();
+        if (tile == blockIdx.x) {
+            h = s_head;
+            if (h.skip) {
+                update_skipped(a, h);
+                return;
+            }
+            if (n == 0u) return;
+            fil = fil && h.filter;
+        }
+        const int4 p = s_pk[o];
+        const GaussPair cj = gauss_pair(kcj.x, kcj.y);
+        const int3 start = sub == 0 ? make_int3(shj.x, shj.y, shj.z) : make_int3(0, 0, 0);
+        int3 acc = start;
+        float low = 0.0f;
+        {
+            const F2 one = f2_pack(a.one, a.one);
+            const F2 k36 = f2_pack(0.693147180559945309f * 0x1p19f, 0.693147180559945309f * 0x1p19f);
+            const F2 ivd0 = f2_pack(cj.ivd36, cj.ivd36), norm0 = f2_pack(cj.norm, cj.norm), kk0 = f2_pack(cj.k2, cj.k2);
+            const auto two = [&](uint32_t w, auto uniform, auto filter) {
+                const uint32_t o0 = w & 0xffffu, o1 = w >> 16;
+                const int4 q0 = tile_record(s_pk, o0), q1 = tile_record(s_pk, o1);
+                const F2 dx = f2_pack((float)wadd(p.x, -q0.x), (float)wadd(p.x, -q1.x));
+                const F2 dy = f2_pack((float)wadd(p.y, -q0.y), (float)wadd(p.y, -q1.y));
+                const F2 dz = f2_pack((float)wadd(p.z, -q0.z), (float)wadd(p.z, -q1.z));
+                const F2 r2 = dot3_f2(dx, dy, dz, dx, dy, dz, one);
+                if (decltype(filter)::value) {
+                    // gauss_filter_hit_fixed by squares, with margins a hundred times its
+                    // rounding: above the upper line it hits, up to the lower it does not (nor
+                    // below 0.0001 reference units, r2 < 688), between them the row is asked again
+                    const F2 ex = f2_pack(ed.x, ed.x), ey = f2_pack(ed.y, ed.y), ez = f2_pack(ed.z, ed.z);
+                    const float2 d = f2_unpack(dot3_f2(ex, ey, ez, dx, dy, dz, one));
+                    const float2 lo = f2_unpack(r2 * f2_pack(0.35999f, 0.35999f));
+                    const float2 hi = f2_unpack(f2_fma(r2, f2_pack(0.36001f, 0.36001f), f2_pack(700.0f, 700.0f)));
+                    const float t0 = d.x * fabsf(d.x), t1 = d.y * fabsf(d.y);
+                    near = near || t0 > lo.x || t1 > lo.y;
+                    hit = hit || t0 > hi.x || t1 > hi.y;
+                }
+                F2 ivd = ivd0, norm = norm0, kk = kk0;
+                if (!decltype(uniform)::value) {
+                    const float2 c0 = *reinterpret_cast<const float2 *>(reinterpret_cast<const char *>(s_kc) + o0 / 2u),
+                                 c1 = *reinterpret_cast<const float2 *>(reinterpret_cast<const char *>(s_kc) + o1 / 2u);
+                    ivd = f2_pack(c0.x, c1.x);
+                    norm = f2_pack(c0.y, c1.y);
+                    kk = ivd * k36;
+                }
+                F2 W, s;
+                gauss_two(r2, ivd, norm, kk, low, W, s);
+                const F2 sc = f2_pack(__int_as_float(q0.w), __int_as_float(q1.w));
+                const float2 tx = f2_unpack((s * dx) * sc), ty = f2_unpack((s * dy) * sc), tz = f2_unpack((s * dz) * sc);
+                acc.x = wadd(acc.x, wadd(f2i(tx.x), f2i(tx.y)));
+                acc.y = wadd(acc.y, wadd(f2i(ty.x), f2i(ty.y)));
+                acc.z = wadd(acc.z, wadd(f2i(tz.x), f2i(tz.y)));
+            };
+            const auto rows = [&](auto uniform, auto filter) {
+                for (uint32_t k = sub * 4u; k < depth; k += L * 4u) {
+                    const uint2 cur = e;
+                    if (k + L * 4u < depth) e = row[(k / 4u + L) * T];
+                    two(cur.x, uniform, filter);
+                    if (k + 2u < depth) two(cur.y, uniform, filter);
+                }
+            };
+            using Yes = std::true_type;
+            using No = std::false_type;
+            if (__any_sync(0xffffffffu, fil)) {  // one form per warp
+                if (h.packed) rows(Yes(), Yes());
+                else rows(No(), Yes());
+                hit = hit && fil;
+                if (fil && near && !hit) {
+#pragma unroll 1
+                    for (uint32_t k = 0; k < depth && !hit; ++k) {
+                        const float3 D = udiff(tile_record(s_pk, row_offset(row[(k / 4u) * T], k)), p);
+                        hit = gauss_filter_hit_fixed(ed, D, dot3x(D, D));
+                    }
+                }
+            } else {
+                if (h.packed) rows(Yes(), No());
+                else rows(No(), No());
+            }
+        }
+        const auto add = [&](int4 q, float sc, const GaussPair &gk, bool test) {
+            const float3 D = udiff(q, p);
+            const float r2 = dot3x(D, D);
+            if (test && fil && !hit) hit = gauss_filter_hit_fixed(ed, D, r2);
+            if (sc == 0.0f) return;
+            float W;
+            float3 g;
+            gauss_terms_r2(D, r2, gk, W, g);
+            acc.x = wadd(acc.x, f2i(g.x * sc));
+            acc.y = wadd(acc.y, f2i(g.y * sc));
+            acc.z = wadd(acc.z, f2i(g.z * sc));
+        };
+        if (L > 1) low = group_min<L>(low);  // the group sums its row again as one
+        if (low < kLowExponent) {  // far out in a narrow kernel: exp2f's own range handling
+            acc = start;
+#pragma unroll 1
+            for (uint32_t k = sub; k < depth; k += L) {
+                const uint32_t of = row_offset(row[(k / 4u) * T], k);
+                const int4 q = tile_record(s_pk, of);
+                const float2 kk = h.packed ? kcj : s_kc[of / 16u];
+                add(q, __int_as_float(q.w), gauss_pair(kk.x, kk.y), false);
+            }
+        }
+        const uint32_t shallow = min(cnt, (uint32_t)kTileDepth);
+#pragma unroll 2
+        for (uint32_t k = depth + sub; k < shallow; k += L) {  // a tile whose halo did not fit
+            const uint32_t g = idx_arr[(size_t)k * a.stride + j] & ~kNoDelta;
+            const float2 kk = h.packed ? kcj : a.kc[g];
+            const int4 q = a.pk[g];
+            add(q, __int_as_float(q.w) * APBF_FIX, gauss_pair(kk.x, kk.y), true);
+        }
+        // what is left of the long rows: one row after the other, by the whole warp
+        for (uint32_t left = __ballot_sync(0xffffffffu, sub == 0u && cnt > kTileDepth); left; left &= left - 1u) {
+            const int src = __ffs(left) - 1;
+            const WarpRow w(plan, idx_arr, a.stride, j, cnt, p, src);
+            const float2 kw = make_float2(__shfl_sync(0xffffffffu, kcj.x, src), __shfl_sync(0xffffffffu, kcj.y, src));
+            const bool test = __shfl_sync(0xffffffffu, fil && !hit ? 1 : 0, src) != 0;
+            const float3 ew = make_float3(__shfl_sync(0xffffffffu, ed.x, src), __shfl_sync(0xffffffffu, ed.y, src),
+                                          __shfl_sync(0xffffffffu, ed.z, src));
+            int3 t = make_int3(0, 0, 0);
+            bool any = false;
+            w.each([&](uint32_t g) { return a.pk[g & ~kNoDelta]; }, [&](uint32_t g, const int4 &q) {
+                const float3 D = udiff(q, w.p);
+                const float r2 = dot3x(D, D);
+                if (test && !any) any = gauss_filter_hit_fixed(ew, D, r2);
+                const float lam = __int_as_float(q.w);
+                if (lam == 0.0f) return;
+                const float2 kk = h.packed ? kw : a.kc[g & ~kNoDelta];
+                const int3 v = gauss_delta(D, r2, lam, gauss_pair(kk.x, kk.y));
+                t.x = wadd(t.x, v.x);
+                t.y = wadd(t.y, v.y);
+                t.z = wadd(t.z, v.z);
+            });
+            t.x = __reduce_add_sync(0xffffffffu, t.x);
+            t.y = __reduce_add_sync(0xffffffffu, t.y);
+            t.z = __reduce_add_sync(0xffffffffu, t.z);
+            any = __any_sync(0xffffffffu, any);
+            if ((int)(threadIdx.x & 31u) == src) {
+                acc.x = wadd(acc.x, t.x);
+                acc.y = wadd(acc.y, t.y);
+                acc.z = wadd(acc.z, t.z);
+                hit = hit || any;
+            }
+        }
+        if (h.corr) {  // the correction row (radii that differ): usually empty
+            const uint32_t m = valid ? a.rcount[j] : 0u;
+            if (m)
+                acc = h.packed ? delta_corrections<true, L, true>(a, a.pos, m, j, sub, p, cj, acc)
+                               : delta_corrections<true, L, false>(a, a.pos, m, j, sub, p, cj, acc);
+        }
+        if (L > 1) {
+            acc.x = group_wsum<L>(acc.x);
+            acc.y = group_wsum<L>(acc.y);
+            acc.z = group_wsum<L>(acc.z);
+            if (h.filter) {
+                int x = hit ? 1 : 0;
+#pragma unroll
+                for (int off = L / 2; off > 0; off >>= 1) x |= __shfl_xor_sync(0xffffffffu, x, off);
+                hit = x != 0;
+            }
+        }
+        if (valid && sub == 0) {
+            const float lj = (a.prev_mode | a.acc_mode) ? __int_as_float(a.pk[j].w) : 0.0f;
+            uint32_t nb = h.nboxes, first = 0;
+            int4 v = make_int4(wadd(p.x, acc.x), wadd(p.y, acc.y), wadd(p.z, acc.z), pw);
+            if (nb && nb <= kTileBoxes) {
+                first = tile_boxes_clear(v, s_box, nb);
+                if (first == nb) {  // no box: box_push's round trip through FP32 and 2^-18
+                    v.x = f2i((float)v.x);
+                    v.y = f2i((float)v.y);
+                    v.z = f2i((float)v.z);
+                    nb = 0u;
+                }
+            }
+            if (nb) v = box_push_from(v, a.radius[j], j, a.bmin, a.bmax, a.rot, first, nb);
+            delta_store(a, a.pos_out, j, v, hit, 0.0f, lj, 0u);
+        }
+        if (tile + gridDim.x < (n + T - 1) / T) __syncthreads();  // the shared records are the next tile's
+    }
 }
 
 // ---- the solve loop as one persistent cooperative kernel ----
@@ -896,7 +1749,8 @@ __device__ __forceinline__ bool grid_barrier(Status *st, uint32_t &gen, const Pa
                 const unsigned long long t2 = *(volatile unsigned long long *)&st->loop_e2;
                 st->loop_e1 = 0ull;
                 st->loop_e2 = 0ull;
-                finish_pass(*fin, n, (long long)t1, (long long)t2);
+                finish_pass(fin->red_out, fin->st, fin->target, n, (long long)t1, (long long)t2,
+                            error_meets_target(t1, n, fin->target, fin->target_m, fin->target_s));
             }
             st->bar_arrive = 0u;
             __threadfence();
@@ -1016,7 +1870,9 @@ __device__ __forceinline__ bool batch_barrier(BatchSync *sy, uint32_t &gen, cons
                 const unsigned long long t2 = *(volatile unsigned long long *)&acc[2 * sc + 1];
                 acc[2 * sc] = 0ull;
                 acc[2 * sc + 1] = 0ull;
-                finish_pass(tab[sc].a, s_n[sc], (long long)t1, (long long)t2);
+                const PassA &pa = tab[sc].a;
+                finish_pass(pa.red_out, pa.st, pa.target, s_n[sc], (long long)t1, (long long)t2,
+                            error_meets_target(t1, s_n[sc], pa.target, pa.target_m, pa.target_s));
             }
         __threadfence();
         __syncthreads();
@@ -1250,11 +2106,12 @@ static PassA make_pass_a(apbf_ctx *ctx, const SolveOpts &o) {
     a.dbg_dens = ctx->debug ? ctx->dbg_density : nullptr;
     a.dbg_grad = ctx->dbg_grad;
     a.dbg_sq = ctx->dbg_sq;
-    a.partials = reinterpret_cast<long long *>(ctx->red_partials);
+    a.sync = ctx->pass_sync;
     a.d_len = ctx->d_len;
     a.st = ctx->status;
     a.red_out = ctx->red_out;
     a.target = converge ? st.density_error_target : 0.0f;
+    split_target(a.target, a.target_m, a.target_s);
     a.early_exit = converge ? 1 : 0;
     a.features = feature_mode ? ctx->features : nullptr;
     a.selfdir = ctx->selfdir;
@@ -1266,6 +2123,7 @@ static PassA make_pass_a(apbf_ctx *ctx, const SolveOpts &o) {
     a.filt = ctx->tuning.filter_in_density ? nullptr : ctx->filt;
     const float rm2 = 2.0f * st.smallest_target_radius;
     a.rmin3 = rm2 * rm2 * rm2;
+    a.one = 1.0f;
     a.hk = st.height_kernel_id;
     a.gk = st.gradient_kernel_id;
     a.method = st.boundariness_calculation_method;
@@ -1300,6 +2158,11 @@ static PassB make_pass_b(apbf_ctx *ctx, const SolveOpts &o) {
     b.stride = ctx->row_stride;
     b.d_len = ctx->d_len;
     b.st = ctx->status;
+    b.sync = ctx->pass_sync;
+    b.red_out = ctx->red_out;
+    b.target = o.converge ? st.density_error_target : 0.0f;
+    split_target(b.target, b.target_m, b.target_s);
+    b.one = 1.0f;
     b.gk = st.gradient_kernel_id;
     b.early_exit = o.converge ? 1 : 0;
     b.lam_prev = f.lambda_prev;
@@ -1313,21 +2176,148 @@ static PassB make_pass_b(apbf_ctx *ctx, const SolveOpts &o) {
     return b;
 }
 
-apbf_status incompressibility(apbf_ctx *ctx, cudaStream_t s, const SolveOpts &o) {
-    const bool converge = o.converge, learned = o.learned;
+// Launch shape of the two passes: the caller's when one was set (apbf_set_tuning,
+// apbf_autotune), else lanes per particle by the list's capacity.
+struct PassShape {
+    int lanes, block, grid;
+};
+static PassShape pass_shape(const apbf_ctx *ctx, bool features) {
     const uint32_t cap = ctx->cfg.particle_capacity;
+    PassShape sh;
+    int per_sm = 32;  // a thread per particle (or lane) up to 1.2 million of them
+    if (ctx->shape_set) {
+        sh.lanes = (int)ctx->tuning.gather_lanes;
+        sh.block = ctx->tuning.pass_block == 128 ? 128 : 256;
+        per_sm = (int)std::min(8u, std::max(1u, ctx->tuning.pass_blocks_per_sm));
+    } else {
+        // Several threads share a row while the particles alone leave the chip's schedulers
+        // short of warps: a frame of 2 197 particles takes 325 / 299 / 279 us with 1 / 2 / 4
+        // threads, 32 768 particles 2107 / 1742 / 1756, 64 019 506 / 501 / 520, 119 771
+        // 2625 / 2751 / 3227.  The features' float sums keep the row's order: one thread.
+        sh.block = 256;
+        sh.lanes = features || cap > 98304u ? 1 : cap > 32768u ? 2 : 4;
+    }
+    sh.grid = grid_for(ctx, (uint32_t)std::min<uint64_t>((uint64_t)cap * sh.lanes, 0xffffffffu), sh.block, per_sm);
+    return sh;
+}
+
+// Calls f with the tile shape (particles, threads per particle) for the list: 128 x 1, or
+// 64 x 2 where 128 would leave SMs without a tile (2 197 particles: 294 us a frame with
+// 128 x 1, 285 with 64 x 2; from 30 000 particles on the larger tile is as fast or faster:
+// 1521 / 1509 us at 32 768, 2094 / 2570 at 119 771).
+template <typename F>
+static void with_tile_shape(const apbf_ctx *ctx, F &&f) {
+    if (ctx->cfg.particle_capacity <= 24576u)
+        f(std::integral_constant<int, 64>(), std::integral_constant<int, 2>());
+    else
+        f(std::integral_constant<int, 128>(), std::integral_constant<int, 1>());
+}
+
+// Rewriting the rows costs as much as about two passes gain by it, less where the passes
+// are short of warps anyway: at 250 000 particles 40 us against 23 us a pass, at 2 197
+// four passes are as fast with the direct kernels (273 against 285 us a frame).
+bool tiles_eligible(const apbf_ctx *ctx) {
+    const apbf_settings &st = ctx->settings;
+    return st.height_kernel_id == 1 && st.gradient_kernel_id == 1 && st.boundariness_calculation_method != 1 &&
+           st.solver_iterations >= (ctx->cfg.particle_capacity >= 65536u ? 4 : 6);
+}
+
+apbf_status tile_rows(apbf_ctx *ctx, cudaStream_t s, bool transposed) {
+    apbf_status r = APBF_OK;
+    with_tile_shape(ctx, [&](auto tc, auto) {
+        constexpr int T = decltype(tc)::value;
+        const uint32_t tiles = (ctx->cfg.particle_capacity + T - 1) / T;
+        const int grid = (int)std::min<uint32_t>(std::max(tiles, 1u), (uint32_t)ctx->num_sms * 32u);
+        for (int rev = 0; rev < (transposed ? 2 : 1) && r == APBF_OK; ++rev) {
+            TileRowsArgs a;
+            a.count = rev ? ctx->rev_count : ctx->nb_count;
+            a.idx = rev ? ctx->rev_idx : ctx->nb_idx;
+            a.stride = ctx->row_stride;
+            a.d_len = ctx->d_len;
+            a.st = ctx->status;
+            a.reverse = rev;
+            a.radius = ctx->fl[ctx->fcur].radius;
+            a.plan = ctx->tile_plan[rev];
+            r = [&]() -> apbf_status {
+                APBF_BEFORE_LAUNCH(ctx, s, "k_tile_rows");
+                k_tile_rows<T><<<grid, 256, 0, s>>>(a);
+                APBF_AFTER_LAUNCH(ctx, s, "k_tile_rows");
+                return APBF_OK;
+            }();
+        }
+    });
+    return r;
+}
+
+// Launches a kernel that waits itself (griddepcontrol.wait) for the one before it:
+// behind lets its blocks start as that one's last blocks run.
+template <typename... P, typename... V>
+static cudaError_t launch_behind(bool behind, void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s,
+                                 V... v) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = behind ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, v...);
+}
+
+// One Jacobi pass over the tiles of the substep's rows.
+static apbf_status launch_tiles(apbf_ctx *ctx, cudaStream_t s, const PassA &a, const PassB &b, const SolveOpts &o) {
+    const bool learned = o.learned;
+    apbf_status r = APBF_OK;
+    with_tile_shape(ctx, [&](auto tc, auto lc) {
+        constexpr int T = decltype(tc)::value, L = decltype(lc)::value;
+        const uint32_t tiles = (ctx->cfg.particle_capacity + T - 1) / T;
+        const int grid = (int)std::min<uint32_t>(std::max(tiles, 1u), (uint32_t)ctx->num_sms * 64u);
+        const size_t rec = (size_t)(2 * T + kTileHalo);
+        r = [&]() -> apbf_status {
+            APBF_BEFORE_LAUNCH(ctx, s, "k_density_tiles");
+            // a pass behind a position update starts while that drains (the kernels wait for it
+            // before they read what it wrote); the first kernel behind the rows does not, nor
+            // do those of a batch, whose waiting blocks would keep other scenes' off the SMs
+            // (16 scenes: 3113 against 3028 us)
+            APBF_CUDA(launch_behind(o.later_pass && o.behind && !ctx->in_batch, k_density_tiles<T, L>, grid, T * L, rec * sizeof(int4), s, a,
+                                    ctx->tile_plan[0]));
+            APBF_AFTER_LAUNCH(ctx, s, "k_density_tiles");
+            if (learned) {  // the network's lambda replaces the plain one in this update
+                apbf_status q = mlp_lambda(ctx, s, a.target, a.target_m, a.target_s);
+                if (q != APBF_OK) return q;
+            }
+            APBF_BEFORE_LAUNCH(ctx, s, "k_delta_tiles");
+            APBF_CUDA(launch_behind(!learned && !ctx->in_batch, k_delta_tiles<T, L>, grid, T * L, rec * (sizeof(int4) + sizeof(float2)), s, b,
+                                    ctx->tile_plan[0], ctx->tile_plan[1]));
+            APBF_AFTER_LAUNCH(ctx, s, "k_delta_tiles");
+            return APBF_OK;
+        }();
+    });
+    return r;
+}
+
+apbf_status incompressibility(apbf_ctx *ctx, cudaStream_t s, const SolveOpts &o) {
+    const bool learned = o.learned;
     FluidBufs &f = ctx->fl[ctx->fcur];
     FluidBufs &alt = ctx->fl[ctx->fcur ^ 1];
     const apbf_settings &st = ctx->settings;
     const bool gauss = st.height_kernel_id == 1 && st.gradient_kernel_id == 1;
     const PassA a = make_pass_a(ctx, o);
-    const int g = ctx->red_blocks;
-    const int lanes = ctx->tuning.gather_lanes;
-    const int pb = ctx->tuning.pass_block == 128 ? 128 : 256;
-    const int bps = (int)std::min(8u, std::max(1u, ctx->tuning.pass_blocks_per_sm));
-    // the error reduction has one partial per block: at most red_blocks blocks
-    const int ga = std::min(g, grid_for(ctx, (uint32_t)std::min<uint64_t>((uint64_t)cap * lanes, 0xffffffffu), pb, bps));
+    const PassShape sh = pass_shape(ctx, o.feature_mode != 0);
+    const int lanes = sh.lanes, pb = sh.block, ga = sh.grid, gd = sh.grid;
     const bool xtra = a.features != nullptr || a.method == 1;
+    if (o.tiles && gauss && !xtra) {
+        const PassB b = make_pass_b(ctx, o);
+        apbf_status r = launch_tiles(ctx, s, a, b, o);
+        if (r != APBF_OK) return r;
+        int4 *tmp = f.pos;
+        f.pos = alt.pos;
+        alt.pos = tmp;
+        return APBF_OK;
+    }
     APBF_BEFORE_LAUNCH(ctx, s, "k_density_lambda");
     launch_lanes(lanes, [&](auto lc) {
         constexpr int Lc = decltype(lc)::value;
@@ -1341,12 +2331,11 @@ apbf_status incompressibility(apbf_ctx *ctx, cudaStream_t s, const SolveOpts &o)
     APBF_AFTER_LAUNCH(ctx, s, "k_density_lambda");
 
     if (learned) {  // the network's lambda replaces the plain one in this update
-        apbf_status r = mlp_lambda(ctx, s, converge);
+        apbf_status r = mlp_lambda(ctx, s, a.target, a.target_m, a.target_s);
         if (r != APBF_OK) return r;
     }
     const PassB b = make_pass_b(ctx, o);
     APBF_BEFORE_LAUNCH(ctx, s, "k_delta");
-    const int gd = grid_for(ctx, (uint32_t)std::min<uint64_t>((uint64_t)cap * lanes, 0xffffffffu), pb, bps);
     launch_lanes(lanes, [&](auto lc) {
         constexpr int Lc = decltype(lc)::value;
         if (gauss)
@@ -1359,6 +2348,21 @@ apbf_status incompressibility(apbf_ctx *ctx, cudaStream_t s, const SolveOpts &o)
     int4 *tmp = f.pos;
     f.pos = alt.pos;
     alt.pos = tmp;
+    return APBF_OK;
+}
+
+// The tiled passes run behind one another with programmatic launches, so blocks of both
+// kernels share an SM: they ask for the same split of its L1 (at different ones each
+// launch waits for the SM to drain: 1760 against 1520 us for the 32 768-particle frame).
+// 75 % shared memory holds every block the registers allow (50 %: 2213, 100 %: 2151
+// against 2094 us at 119 771 particles).
+apbf_status tiles_prepare_device() {
+    constexpr int kShared = 75;
+    constexpr auto kAttr = cudaFuncAttributePreferredSharedMemoryCarveout;
+    APBF_CUDA(cudaFuncSetAttribute(k_density_tiles<64, 2>, kAttr, kShared));
+    APBF_CUDA(cudaFuncSetAttribute(k_delta_tiles<64, 2>, kAttr, kShared));
+    APBF_CUDA(cudaFuncSetAttribute(k_density_tiles<128, 1>, kAttr, kShared));
+    APBF_CUDA(cudaFuncSetAttribute(k_delta_tiles<128, 1>, kAttr, kShared));
     return APBF_OK;
 }
 

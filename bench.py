@@ -151,9 +151,9 @@ class ClockSampler:
 def algorithmic_bytes(kernel: str, n: int, pairs: int) -> float | None:
     """Compulsory HBM bytes of one launch (inputs read once, outputs written once,
     neighbour data counted once per particle, rows as 4 bytes per pair)."""
-    if kernel == "k_density_lambda":
+    if kernel in ("k_density_lambda", "k_density_tiles"):
         return 28.0 * n + 4.0 * pairs  # 4N + 4P + 12N pos + 8N (invMass, kw) + 4N lambda
-    if kernel == "k_delta":
+    if kernel in ("k_delta", "k_delta_tiles"):
         return 40.0 * n + 4.0 * pairs  # 4N + 4P + 12N + 4N lambda + 8N + 12N pos out
     if kernel == "k_build_rows":
         return 16.0 * n + 4.0 * n + 4.0 * pairs  # pos + range in, counts + rows out
