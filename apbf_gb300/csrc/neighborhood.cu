@@ -16,6 +16,7 @@
 //     scattering with atomics, and no transpose is needed.
 //  6. k_reverse_rows (binary-search rows and pruned rows): the transpose.
 #include <algorithm>
+#include <type_traits>
 
 #include "apbf_internal.cuh"
 
@@ -92,9 +93,13 @@ __global__ void k_reorder(FluidBufs src, FluidBufs dst, const uint32_t *__restri
         rmin = a2 < rmin ? a2 : rmin;
         rmax = c2 > rmax ? c2 : rmax;
     }
+    // a bound that already holds is left alone: every write of these two words passes
+    // between the SMs, a read does not
     if ((threadIdx.x & 31) == 0 && rmax >= 0) {
-        atomicMin(&st->range_min, (unsigned long long)rmin);
-        atomicMax(&st->range_max, (unsigned long long)rmax);
+        if ((unsigned long long)rmin < *(volatile unsigned long long *)&st->range_min)
+            atomicMin(&st->range_min, (unsigned long long)rmin);
+        if ((unsigned long long)rmax > *(volatile unsigned long long *)&st->range_max)
+            atomicMax(&st->range_max, (unsigned long long)rmax);
     }
 }
 
@@ -123,16 +128,6 @@ __global__ void k_cell_ranges(const uint32_t *__restrict__ skeys, const uint32_t
         if (id != 0 && cur != prev) end[prev] = id;
         if (id == n - 1) end[cur] = id + 1u;
     }
-}
-
-// Exact 32-bit form of `within` for particles that both lie inside the grid
-// (coordinates differ by less than 2^31): the same predicate, half the
-// instructions.  R2 = R * R.
-__device__ __forceinline__ bool within32(int4 a, int4 b, uint32_t R, unsigned long long R2) {
-    const uint32_t ax = (uint32_t)abs(b.x - a.x), ay = (uint32_t)abs(b.y - a.y), az = (uint32_t)abs(b.z - a.z);
-    if (max(ax, max(ay, az)) > R) return false;
-    const unsigned long long s = (unsigned long long)ax * ax + (unsigned long long)ay * ay + (unsigned long long)az * az;
-    return s <= R2;
 }
 
 struct BuildArgs {
@@ -194,65 +189,6 @@ __device__ __forceinline__ unsigned long long dist2_within(int4 a, int4 b, uint3
     return (unsigned long long)ax * ax + (unsigned long long)ay * ay + (unsigned long long)az * az;
 }
 
-// Walks the cells [x0, x1] x [y0, y1] x [z0, z1] and appends every neighbour of
-// particle i: j != i with |x_j - x_i| <= R_i (the neighbour predicate, C2).  The
-// walk is a chain of dependent loads (cell range -> candidates), so the ranges of
-// up to four cells of one (z, y) row are loaded together and candidates four at a
-// time.
-//
-// Correction rows (UNI, when the search radii differ): the position update of
-// particle i sums over the particles k whose rows hold i (|x_i - x_k| <= R_k),
-// and its deferred boundariness filter tests i's own row.  It sums over i's own
-// row and then over i's correction row: entries j of i's row whose radius does not
-// reach i (flagged kNoDelta, their terms subtracted), and particles k whose rows
-// hold i although i's radius does not reach them (added).  Both kinds are one-sided
-// pairs, found here (one_sided counts them) and appended after the walk.
-template <bool FAST>
-__device__ __forceinline__ uint32_t walk_cells(const BuildArgs &a, uint32_t i, int4 p, long long R, uint32_t x0,
-                                               uint32_t x1, uint32_t y0, uint32_t y1, uint32_t z0, uint32_t z1,
-                                               bool uni, uint32_t &one_sided) {
-    const uint32_t R32 = (uint32_t)R;
-    const unsigned long long R2 = (unsigned long long)R32 * R32;
-    uint32_t c = 0;
-    for (uint32_t cz = z0; cz <= z1; ++cz)
-        for (uint32_t cy = y0; cy <= y1; ++cy) {
-            const uint32_t yz = (spread3(cy) << 1) | (spread3(cz) << 2);
-            for (uint32_t cx0 = x0; cx0 <= x1; cx0 += 4) {
-                uint32_t cs[4], ce[4];
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const bool in = cx0 + v <= x1;
-                    const uint32_t key = yz | spread3(cx0 + v);
-                    cs[v] = in ? a.cstart[key] : 0u;
-                    ce[v] = in ? a.cend[key] : 0u;
-                }
-#pragma unroll 1  // one copy of the candidate loop: the kernel is bound by its instruction cache
-                for (int v = 0; v < 4; ++v) {
-                    const uint32_t s = cs[v], e = ce[v];
-                    for (uint32_t j0 = s; j0 < e; j0 += 4) {
-                        int4 q[4];
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) q[u] = j0 + u < e ? a.srec[j0 + u] : p;
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            const uint32_t j = j0 + u;
-                            if (j >= e || j == i) continue;
-                            const unsigned long long d2 = dist2_within<FAST>(p, q[u], R32);
-                            if (d2 > R2) continue;
-                            if (uni) {
-                                const unsigned long long Rj = (unsigned long long)(uint32_t)max(q[u].w, 0);
-                                one_sided += (q[u].w >= 0 && d2 <= Rj * Rj) ? 0u : 1u;
-                            }
-                            if (c < a.maxn) a.idx[(size_t)c * a.stride + i] = j;
-                            ++c;
-                        }
-                    }
-                }
-            }
-        }
-    return c;
-}
-
 // box_push as a call: the walk's kernel is bound by its instruction cache, and the
 // box pass runs once per particle.
 __device__ __noinline__ int4 box_push_call(int4 ip, float r, uint32_t id, const float4 *__restrict__ bmin,
@@ -282,46 +218,181 @@ __global__ void k_corrections(BuildArgs a) {
     }
 }
 
-// neighborhood_green.comp:49-87 with the canonical predicate (C2), one thread per
-// particle, candidates read from the search records.  A box that touches no edge
-// cell of the grid only meets particles inside the grid (edge cells also hold the
-// clamped outsiders), so it uses the 32-bit differences.
-__global__ void __launch_bounds__(256, 4) k_build_rows(BuildArgs a) {
+// The rows (neighborhood_green.comp:49-87 with the canonical predicate, C2): G threads
+// walk the cells around one particle and append every j != i with |x_j - x_i| <= R_i, cells
+// in z, y, x order and their particles in list order.
+//
+// A thread per particle (as this kernel once was) is a chain of dependent loads, 120 us
+// however few the particles (now 17 us at 2 197, 55 at 32 768), and idles at 12 of 32 lanes
+// where their cells differ in length (250 000: 260 against 206 us, a million: 800 against
+// 663; bound by instruction issue).  Here a group's threads each take a cell: they load the ranges of G cells at
+// once, add up the lengths by shuffles and then test G candidates of the joined ranges at a
+// time, whatever cells they come from; a ballot gives the kept ones their places, so the
+// rows keep their order.  The rows are collected in shared memory (kRowStage entries; the
+// rest goes out directly) and written a line at a time, as they are read later.
+//
+// Correction rows (uni, when the search radii differ): the position update of
+// particle i sums over the particles k whose rows hold i (|x_i - x_k| <= R_k),
+// and its deferred boundariness filter tests i's own row.  It sums over i's own
+// row and then over i's correction row: entries j of i's row whose radius does not
+// reach i (flagged kNoDelta, their terms subtracted), and particles k whose rows
+// hold i although i's radius does not reach them (added).  Both kinds are one-sided
+// pairs, counted here (one_sided) and appended by k_corrections.
+constexpr uint32_t kBuildThreads = 256, kRowStage = 64;
+
+// Sum over a group of G consecutive lanes.
+template <int G>
+__device__ __forceinline__ uint32_t group_total(uint32_t v) {
+#pragma unroll
+    for (int off = G / 2; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    return v;
+}
+
+// Squared distance as dist2_within, without its range test where the differences cannot
+// overflow the sum (FAST: below 2^31 each).
+template <bool FAST>
+__device__ __forceinline__ unsigned long long dist2_to(int4 a, int4 b, uint32_t R) {
+    if (!FAST) return dist2_within<false>(a, b, R);
+    const long long dx = b.x - a.x, dy = b.y - a.y, dz = b.z - a.z;
+    return (unsigned long long)(dx * dx) + (unsigned long long)(dy * dy) + (unsigned long long)(dz * dz);
+}
+
+template <int G>
+__global__ void __launch_bounds__(kBuildThreads, 6) k_build_rows(BuildArgs a) {
+    constexpr uint32_t P = kBuildThreads / G;  // particles per block
+    constexpr uint32_t kPad = P + 1;           // a group's consecutive places fall into different banks
+    __shared__ uint32_t s_row[kRowStage * kPad];
+    __shared__ uint32_t s_cnt[P];
     const uint32_t n = a.d_len[kLenParticles];
     const uint32_t last = (1u << a.L) - 1u;
     const bool uni = a.corrections && a.st->range_min != a.st->range_max;  // the radii differ: correction rows
     if (blockIdx.x == 0 && threadIdx.x == 0) a.st->union_rows = uni ? 1u : 0u;
+    const uint32_t gl = threadIdx.x % G, slot = threadIdx.x / G;
+    const uint32_t shift = threadIdx.x & 31u & ~(uint32_t)(G - 1);  // the group's first lane in its warp
+    const uint32_t below = (1u << gl) - 1u, mine = G == 32 ? 0xffffffffu : (1u << G) - 1u;
     unsigned long long local = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int4 p = a.srec[i];
+    for (uint32_t base = blockIdx.x * P; base < n; base += gridDim.x * P) {
+        const uint32_t i = base + slot;
+        const bool valid = i < n;
+        const int4 p = valid ? a.srec[i] : make_int4(0, 0, 0, -1);
         const long long R = p.w;
-        uint32_t c = 0;
-        if (R < 0) {
-            set_flag(a.st, APBF_FLAG_NONFINITE);  // NaN or negative kernel width: no neighbours
-        } else {
-            const Bounds &b = a.b;
-            const uint32_t x0 = cell_coord((long long)p.x - R, b.lo[0], b.hi[0], a.L);
-            const uint32_t x1 = cell_coord((long long)p.x + R, b.lo[0], b.hi[0], a.L);
-            const uint32_t y0 = cell_coord((long long)p.y - R, b.lo[1], b.hi[1], a.L);
-            const uint32_t y1 = cell_coord((long long)p.y + R, b.lo[1], b.hi[1], a.L);
-            const uint32_t z0 = cell_coord((long long)p.z - R, b.lo[2], b.hi[2], a.L);
-            const uint32_t z1 = cell_coord((long long)p.z + R, b.lo[2], b.hi[2], a.L);
-            const bool fast = a.fast_ok && x0 > 0 && y0 > 0 && z0 > 0 && x1 < last && y1 < last && z1 < last;
-            uint32_t one_sided = 0;
-            c = fast ? walk_cells<true>(a, i, p, R, x0, x1, y0, y1, z0, z1, uni, one_sided)
-                     : walk_cells<false>(a, i, p, R, x0, x1, y0, y1, z0, z1, uni, one_sided);
-            if (uni) a.one_sided[i] = one_sided;  // k_corrections appends them
+        // the six faces of the cell box, a thread each
+        uint32_t face = 0;
+        if (R >= 0 && gl < 6u) {
+            const uint32_t d = gl >> 1;
+            const long long x = d == 0u ? p.x : d == 1u ? p.y : p.z;
+            const long long lo = d == 0u ? a.b.lo[0] : d == 1u ? a.b.lo[1] : a.b.lo[2];
+            const long long hi = d == 0u ? a.b.hi[0] : d == 1u ? a.b.hi[1] : a.b.hi[2];
+            face = cell_coord((gl & 1u) ? x + R : x - R, lo, hi, a.L);
         }
-        if (c > a.maxn) {
-            set_flag(a.st, APBF_FLAG_NEIGHBOR_OVERFLOW);
-            atomicMax(&a.st->required_neighbors, c);
+        const uint32_t x0 = __shfl_sync(0xffffffffu, face, 0, G), x1 = __shfl_sync(0xffffffffu, face, 1, G),
+                       y0 = __shfl_sync(0xffffffffu, face, 2, G), y1 = __shfl_sync(0xffffffffu, face, 3, G),
+                       z0 = __shfl_sync(0xffffffffu, face, 4, G), z1 = __shfl_sync(0xffffffffu, face, 5, G);
+        if (valid && R < 0 && gl == 0u) set_flag(a.st, APBF_FLAG_NONFINITE);  // NaN or negative width: no neighbours
+        const uint32_t nx = x1 - x0 + 1u, ny = y1 - y0 + 1u, nz = z1 - z0 + 1u;
+        const uint32_t ncell = R < 0 ? 0u : nx * ny * nz;
+        // A box that touches no edge cell of the grid only meets particles inside the grid
+        // (edge cells also hold the clamped outsiders): 32-bit differences.
+        const bool fast = a.fast_ok && x0 > 0 && y0 > 0 && z0 > 0 && x1 < last && y1 < last && z1 < last;
+        const bool all_fast = __all_sync(0xffffffffu, fast || ncell == 0u);
+        const uint32_t R32 = (uint32_t)max(p.w, 0);
+        const unsigned long long R2 = (unsigned long long)R32 * R32;
+        const auto range = [&](uint32_t c, uint32_t &s, uint32_t &len) {  // of the c-th cell of the box
+            s = len = 0u;
+            if (c >= ncell) return;
+            const uint32_t t = c / nx, cx = x0 + (c - t * nx), cz = z0 + t / ny, cy = y0 + t % ny;
+            const uint32_t key = morton3(cx, cy, cz);
+            s = a.cstart[key];
+            len = a.cend[key] - s;
+        };
+        uint32_t c = 0, one_sided = 0;
+        const uint32_t most = __reduce_max_sync(0xffffffffu, ncell);  // the warp's groups go on together
+        uint32_t s, len;
+        range(gl, s, len);
+        for (uint32_t c0 = 0; c0 < most; c0 += G) {
+            uint32_t ns, nlen;
+            range(c0 + G + gl, ns, nlen);  // in flight while this round's candidates are tested
+            uint32_t incl = len;
+#pragma unroll
+            for (int off = 1; off < G; off <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off, G);
+                if ((int)gl >= off) incl += y;
+            }
+            const uint32_t total = __shfl_sync(0xffffffffu, incl, G - 1, G);
+            const uint32_t adj = s - (incl - len);  // candidate f of the joined ranges is particle adj + f
+            const uint32_t rounds = __reduce_max_sync(0xffffffffu, total);
+            const auto candidate = [&](uint32_t f) {  // of the cell whose run holds f
+                uint32_t k = 0;
+#pragma unroll
+                for (int off = G / 2; off > 0; off >>= 1)
+                    if (__shfl_sync(0xffffffffu, incl, k + off - 1, G) <= f) k += off;
+                return __shfl_sync(0xffffffffu, adj, k, G) + f;
+            };
+            const auto test = [&](bool in, uint32_t j, int4 q, auto fast_form) {
+                const unsigned long long d2 = dist2_to<decltype(fast_form)::value>(p, q, R32);
+                const bool keep = in && j != i && d2 <= R2;
+                const uint32_t bal = (__ballot_sync(0xffffffffu, keep) >> shift) & mine;
+                if (keep) {
+                    const uint32_t at = c + __popc(bal & below);
+                    if (at < kRowStage) s_row[at * kPad + slot] = j;
+                    else if (at < a.maxn) a.idx[(size_t)at * a.stride + i] = j;
+                    if (uni) {
+                        const unsigned long long Rj = (unsigned long long)(uint32_t)max(q.w, 0);
+                        one_sided += (q.w >= 0 && d2 <= Rj * Rj) ? 0u : 1u;
+                    }
+                }
+                c += __popc(bal);
+            };
+            const auto windows = [&](auto fast_form) {
+                for (uint32_t w = 0; w < rounds; w += 2 * G) {  // two candidates of each thread in flight
+                    const uint32_t f0 = w + gl, f1 = f0 + G;
+                    const uint32_t j0 = candidate(f0), j1 = candidate(f1);
+                    const bool in0 = f0 < total, in1 = f1 < total;
+                    const int4 q0 = in0 ? a.srec[j0] : p, q1 = in1 ? a.srec[j1] : p;
+                    test(in0, j0, q0, fast_form);
+                    test(in1, j1, q1, fast_form);
+                }
+            };
+            if (all_fast) windows(std::true_type());
+            else windows(std::false_type());
+            s = ns;
+            len = nlen;
         }
-        a.count[i] = c < a.maxn ? c : a.maxn;
-        local += c < a.maxn ? c : a.maxn;
-        if (a.pos_box) a.pos_box[i] = box_push_call(a.pos[i], a.radius[i], i, a.bmin, a.bmax, a.rot, a.nboxes);
+        if (uni) {
+            one_sided = group_total<G>(one_sided);
+            if (valid && gl == 0u) a.one_sided[i] = one_sided;  // k_corrections appends them
+        }
+        if (gl == 0u) {
+            const uint32_t kept = min(c, a.maxn);
+            s_cnt[slot] = kept;
+            if (valid) {
+                if (c > a.maxn) {
+                    set_flag(a.st, APBF_FLAG_NEIGHBOR_OVERFLOW);
+                    atomicMax(&a.st->required_neighbors, c);
+                }
+                a.count[i] = kept;
+                local += kept;
+            }
+        }
+        __syncthreads();
+        {
+            const uint32_t pl = threadIdx.x % P, m = min(s_cnt[pl], kRowStage);
+            for (uint32_t k = threadIdx.x / P; k < m; k += kBuildThreads / P)
+                a.idx[(size_t)k * a.stride + base + pl] = s_row[k * kPad + pl];
+            if (a.pos_box && threadIdx.x < P && base + pl < n)
+                a.pos_box[base + pl] =
+                    box_push_call(a.pos[base + pl], a.radius[base + pl], base + pl, a.bmin, a.bmax, a.rot, a.nboxes);
+        }
+        __syncthreads();  // the rows are the next particles'
     }
+    // one addition per block: a word that many SMs write costs about 25 ns a time
+    __shared__ unsigned long long s_local;
+    if (threadIdx.x == 0) s_local = 0ull;
+    __syncthreads();
     for (int off = 16; off > 0; off >>= 1) local += __shfl_down_sync(0xffffffffu, local, off);
-    if ((threadIdx.x & 31) == 0 && local) atomicAdd(a.total, local);
+    if ((threadIdx.x & 31) == 0 && local) atomicAdd(&s_local, local);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_local) atomicAdd(a.total, s_local);
 }
 
 __global__ void k_reverse_rows(const uint32_t *d_len, uint32_t stride, uint32_t maxn, const uint32_t *__restrict__ count,
@@ -476,7 +547,15 @@ apbf_status neighborhood_green(apbf_ctx *ctx, float range_scale, const float min
     ba.one_sided = ctx->flag_scan;  // scratch: not in use during the search
     ba.corrections = corrections ? 1 : 0;
     APBF_CUDA(cudaMemsetAsync(ctx->rev_count, 0, (size_t)cap * sizeof(uint32_t), s));  // correction rows
-    k_build_rows<<<grid_for(ctx, cap, kBlock, 8), kBlock, 0, s>>>(ba);
+    // threads per particle: as many as it takes to fill the chip, since a smaller group
+    // shares less of its steps' fixed cost.  8 / 16 / 32 threads: 28 / 21 / 17 us at 2 197
+    // particles, 60 / 55 / 60 at 32 768, 206 / 222 / 290 at 250 000, 663 / 794 / 1087 at a million
+    if (cap <= 12288u)
+        k_build_rows<32><<<grid_for(ctx, cap, kBuildThreads / 32, 64), kBuildThreads, 0, s>>>(ba);
+    else if (cap <= 98304u)
+        k_build_rows<16><<<grid_for(ctx, cap, kBuildThreads / 16, 64), kBuildThreads, 0, s>>>(ba);
+    else
+        k_build_rows<8><<<grid_for(ctx, cap, kBuildThreads / 8, 64), kBuildThreads, 0, s>>>(ba);
     APBF_AFTER_LAUNCH(ctx, s, "k_build_rows");
     APBF_BEFORE_LAUNCH(ctx, s, "k_corrections");
     k_corrections<<<grid_for(ctx, cap), kBlock, 0, s>>>(ba);
