@@ -137,9 +137,12 @@ struct KConst {
 struct Ctx;
 
 // Sort scratch sizes.
-constexpr int kSortItems = 16;
+constexpr int kSortItems = 8;
 constexpr int kSortWarps = 8;
-constexpr int kSortTile = kSortItems * 32 * kSortWarps;  // 4096 keys per tile
+constexpr int kSortThreads = 32 * kSortWarps;
+constexpr int kSortTile = kSortItems * kSortThreads;  // 2048 keys per tile
+constexpr int kSortGroup = 32;                        // tiles whose digit counts are also added up
+constexpr uint32_t kSortScratchHead = 8 + 4 * 256;    // tile counters, digit histograms
 
 }  // namespace apbf
 
@@ -208,9 +211,9 @@ struct apbf_ctx {
 
     uint32_t *keys[2] = {nullptr, nullptr};
     uint32_t *vals[2] = {nullptr, nullptr};
+    uint32_t *sort_counters = nullptr;     // tile counters per pass; behind them in one allocation:
     uint32_t *sort_hist = nullptr;         // 4 passes x 256
-    uint32_t *sort_status = nullptr;       // tiles x 256
-    uint32_t *sort_counters = nullptr;     // tile counters per pass
+    uint32_t *sort_status = nullptr;       // passes x tiles x 256
     uint32_t sort_tiles = 0;
     uint32_t *sorted_keys = nullptr;       // result of the last neighbourhood sort
     uint32_t *perm = nullptr;              // new id -> old id of the last reorder
@@ -432,6 +435,7 @@ apbf_status glue_remap(apbf_ctx *ctx, cudaStream_t s);      // constraints.cu: g
 apbf_status sort_pairs_device(apbf_ctx *ctx, const uint32_t *keys_in, const uint32_t *vals_in, const uint32_t *d_count,
                               uint32_t max_count, uint32_t key_bits, uint32_t *keys_out, uint32_t *vals_out,
                               cudaStream_t s);
+apbf_status sort_prepare_device();  // kernel attributes on the current device
 apbf_status prefix_sum_device(apbf_ctx *ctx, uint32_t *d_values, const uint32_t *d_count, uint32_t max_count,
                               cudaStream_t s);
 // corrections = false: no correction rows (the substep prunes and transposes the rows

@@ -254,9 +254,9 @@ apbf_status apbf_create(const apbf_config *cfg, apbf_ctx **out) {
         A(ctx->vals[k], cap);
     }
     ctx->sort_tiles = (cap + kSortTile - 1) / kSortTile;
-    A(ctx->sort_hist, 4 * 256);
-    A(ctx->sort_counters, 8);
-    A(ctx->sort_status, (size_t)4 * ctx->sort_tiles * 256);
+    A(ctx->sort_counters, kSortScratchHead + (size_t)4 * ctx->sort_tiles * 256);
+    ctx->sort_hist = ctx->sort_counters + 8;
+    ctx->sort_status = ctx->sort_hist + 4 * 256;
     A(ctx->sorted_keys, cap);
     A(ctx->perm, cap);
     A(ctx->inv_perm, cap);
@@ -317,7 +317,7 @@ apbf_status apbf_create(const apbf_config *cfg, apbf_ctx **out) {
     A(ctx->emit_state, 8);
     A(ctx->status, 1);
 #undef A
-    if (tiles_prepare_device() != APBF_OK) {
+    if (tiles_prepare_device() != APBF_OK || sort_prepare_device() != APBF_OK) {
         apbf_destroy(ctx);
         return APBF_ERR_CUDA;
     }
