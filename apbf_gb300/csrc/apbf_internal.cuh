@@ -218,8 +218,7 @@ struct apbf_ctx {
     uint32_t *sorted_keys = nullptr;       // result of the last neighbourhood sort
     uint32_t *perm = nullptr;              // new id -> old id of the last reorder
     uint32_t *inv_perm = nullptr;
-    uint32_t *cell_start = nullptr;
-    uint32_t *cell_end = nullptr;
+    uint32_t *cells = nullptr;             // per cell: first particle; then per cell: end
     ulonglong2 *pos_code = nullptr;        // per particle: 96-bit position code {bits 0-63, bits 64-95}
     int4 *srec = nullptr;                  // per particle: search record (position xyz, fixed-point radius)
     int search_method = APBF_NEIGHBORHOOD_GREEN;  // the substep's neighbour search
@@ -536,6 +535,32 @@ __device__ __forceinline__ uint32_t f2u(float x) { return __float2uint_rz(x); }
 __device__ __forceinline__ int32_t wadd(int32_t a, int32_t b) { return (int32_t)((uint32_t)a + (uint32_t)b); }
 
 __device__ __forceinline__ void set_flag(Status *st, uint32_t f) { atomicOr(&st->flags, f); }
+
+// The state a search starts from: the radii's range, the pair count, and the solve's
+// convergence flag and loop counter (cleared with or without a target: the solve loop
+// graph's condition reads the flag, and one left by an earlier substep would end the loop).
+__device__ __forceinline__ void reset_search(Status *st, unsigned long long *total) {
+    st->range_min = 0xffffffffffffffffull;
+    st->range_max = 0ull;
+    st->converged = 0u;
+    st->pass_index = 1u;
+    *total = 0ull;
+}
+
+// The transfer list behind a reorder (indexed_list.h:288-308); every thread of the grid.
+__device__ __forceinline__ void remap_transfers(const TransferBufs &t, const uint32_t *__restrict__ inv_perm,
+                                                const uint32_t *d_len, Status *st) {
+    const uint32_t nt = d_len[kLenTransfers], n = d_len[kLenParticles];
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nt; k += gridDim.x * blockDim.x) {
+        const uint32_t s = t.source[k], g = t.target[k];
+        if (s >= n || g >= n) {  // a transfer naming a particle that does not exist
+            set_flag(st, APBF_FLAG_NONFINITE);
+            continue;
+        }
+        t.source[k] = inv_perm[s];
+        t.target[k] = inv_perm[g];
+    }
+}
 
 // Spin bound of a bounded wait and whether the wait ignores its flag (set by
 // apbf_set_wait_limit to test the failure path without a fault or a hang).

@@ -51,10 +51,13 @@ struct CopyField {
 constexpr int kMaxCopyFields = 11;
 struct CopyList {
     CopyField f[kMaxCopyFields];
+    uint32_t *length;  // non-null: set to `count` by the first thread
+    uint32_t count;
 };
 
 __global__ void __launch_bounds__(256) k_copy_fields(CopyList list) {
     const CopyField fd = list.f[blockIdx.y];
+    if (list.length && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *list.length = list.count;
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
     const unsigned long long t = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long done = 0;
@@ -101,11 +104,13 @@ void *mapped_host(const void *p) {
 }
 
 // Copies `nf` fields of `n` particles (bytes per particle each) between host and
-// device: one k_copy_fields launch for the page-locked host arrays, cudaMemcpyAsync
-// for the others.  to_device: host -> device.
+// device: one k_copy_fields launch for the page-locked host arrays (which also sets the
+// list's length word, when given), cudaMemcpyAsync for the others.  to_device: host -> device.
 apbf_status copy_fluid_fields(apbf_ctx *ctx, void *const *dev, void *const *host, const size_t *bpp, int nf, size_t n,
-                              bool to_device, cudaStream_t s) {
+                              bool to_device, cudaStream_t s, uint32_t *length = nullptr) {
     CopyList list = {};
+    list.length = length;
+    list.count = (uint32_t)n;
     int nk = 0;
     size_t largest = 0;
     for (int k = 0; k < nf; ++k) {
@@ -131,6 +136,10 @@ apbf_status copy_fluid_fields(apbf_ctx *ctx, void *const *dev, void *const *host
         APBF_BEFORE_LAUNCH(ctx, s, "k_copy_fields");
         k_copy_fields<<<dim3(gx, (unsigned)nk), 256, 0, s>>>(list);
         APBF_AFTER_LAUNCH(ctx, s, "k_copy_fields");
+    } else if (length) {
+        APBF_BEFORE_LAUNCH(ctx, s, "k_set_length");
+        k_set_length<<<1, 1, 0, s>>>(length, 0u, (uint32_t)n);
+        APBF_AFTER_LAUNCH(ctx, s, "k_set_length");
     }
     return APBF_OK;
 }
@@ -264,8 +273,7 @@ apbf_status apbf_create(const apbf_config *cfg, apbf_ctx **out) {
     A(ctx->t_keep, tcap);
     A(ctx->t_scan, tcap);
     const size_t ncells = (size_t)1 << (3 * cfg->max_log2res);
-    A(ctx->cell_start, ncells);
-    A(ctx->cell_end, ncells);
+    A(ctx->cells, 2 * ncells);
     A(ctx->pos_code, cap);
     A(ctx->srec, cap);
     ctx->n_cells_log2_alloc = cfg->max_log2res;
@@ -556,12 +564,9 @@ apbf_status apbf_fluid_write(apbf_ctx *ctx, const apbf_host_fluid *in, uint32_t 
     void *const host[] = {in->position,      in->velocity,    in->inverse_mass,      in->radius,
                           in->pos_backup,    in->transferring, in->target_radius,    in->kernel_width,
                           in->boundariness,  in->boundary_distance, in->lambda_prev};
-    apbf_status r = apbf::copy_fluid_fields(ctx, dev, host, kFluidFieldBytes, 11, count, true, s);
-    if (r != APBF_OK) return r;
-    APBF_BEFORE_LAUNCH(ctx, s, "k_set_length");
-    apbf::k_set_length<<<1, 1, 0, s>>>(ctx->d_len, kLenParticles, count);
-    APBF_AFTER_LAUNCH(ctx, s, "k_set_length");
-    return APBF_OK;
+    apbf_status r = apbf::copy_fluid_fields(ctx, dev, host, kFluidFieldBytes, 11, count, true, s,
+                                            ctx->d_len + kLenParticles);
+    return r;
 }
 
 apbf_status apbf_fluid_read(apbf_ctx *ctx, apbf_host_fluid *out, uint32_t max_count, uint32_t *h_count, void *stream) {
@@ -687,9 +692,6 @@ apbf_status substep_body(apbf_ctx *ctx, float dt, cudaStream_t s, bool capture, 
         if (r != APBF_OK) return r;
     }
     const bool converge = st.density_error_target > 0.0f;
-    // cleared even without a target: the solve loop graph's condition reads it, and a
-    // flag left by an earlier substep that had a target would end the loop early
-    APBF_CUDA(cudaMemsetAsync(&ctx->status->converged, 0, sizeof(uint32_t), s));
     const bool recording = ctx->rec_iterations > 0;
     const bool learned = (ctx->warm_start & APBF_WARM_LEARNED) && ctx->mlp_loaded;
     const bool projected = (ctx->warm_start & APBF_WARM_PROJECTED) != 0;

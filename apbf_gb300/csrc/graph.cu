@@ -7,7 +7,8 @@
 // Here passes 1.. of a substep are one CUDA graph: a while-conditional node whose
 // body runs two passes (A -> B, B -> A, so the buffer roles are the same on every
 // run) and a one-thread kernel that advances the device pass counter and keeps the
-// loop going while no pass met the target and passes remain.  Passes past the
+// loop going while no pass met the target and passes remain (the search of the substep
+// set the counter to 1).  Passes past the
 // last one inside a body run copy the positions through, as a converged pass does.
 //
 // Kernel arguments are captured by value, so a graph is specific to the buffer
@@ -21,8 +22,6 @@
 namespace apbf {
 
 namespace {
-
-__global__ void k_loop_init(Status *st) { st->pass_index = 1u; }
 
 __global__ void k_loop_next(cudaGraphConditionalHandle h, Status *st, uint32_t max_passes) {
     const uint32_t next = st->pass_index + 2u;
@@ -140,9 +139,6 @@ apbf_status solve_loop(apbf_ctx *ctx, cudaStream_t s, const SolveOpts &o) {
         for (int k = 0; k < 4; ++k) slot.key[k] = key[k];
         hit = &slot;
     }
-    APBF_BEFORE_LAUNCH(ctx, s, "k_loop_init");
-    k_loop_init<<<1, 1, 0, s>>>(ctx->status);
-    APBF_AFTER_LAUNCH(ctx, s, "k_loop_init");
     APBF_CUDA(cudaGraphLaunch(hit->exec, s));
     return APBF_OK;
 }
@@ -150,8 +146,6 @@ apbf_status solve_loop(apbf_ctx *ctx, cudaStream_t s, const SolveOpts &o) {
 apbf_status solve_loop_captured(apbf_ctx *ctx, cudaStream_t s, const SolveOpts &o) {
     apbf_status r = ensure_streams(ctx);
     if (r != APBF_OK) return r;
-    k_loop_init<<<1, 1, 0, s>>>(ctx->status);
-    APBF_CUDA(cudaGetLastError());
     cudaStreamCaptureStatus cst;
     cudaGraph_t g = nullptr;
     const cudaGraphNode_t *deps = nullptr;

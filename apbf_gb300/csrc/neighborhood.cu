@@ -38,9 +38,12 @@ Bounds fixed_bounds(const float minp[3], const float maxp[3]) {
     return b;
 }
 
+// Its first thread also resets what the search and the solve behind it count from.
 __global__ void k_position_keys(const int4 *__restrict__ pos, const uint32_t *d_len, Bounds b, uint32_t L,
-                                uint32_t *__restrict__ keys, uint32_t *__restrict__ seq) {
+                                uint32_t *__restrict__ keys, uint32_t *__restrict__ seq, Status *st,
+                                unsigned long long *total) {
     uint32_t n = d_len[kLenParticles];
+    if (blockIdx.x == 0 && threadIdx.x == 0) reset_search(st, total);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         int4 p = pos[i];
         uint32_t cx = cell_coord(p.x, b.lo[0], b.hi[0], L);
@@ -103,24 +106,13 @@ __global__ void k_reorder(FluidBufs src, FluidBufs dst, const uint32_t *__restri
     }
 }
 
-__global__ void k_remap_transfers(TransferBufs t, const uint32_t *__restrict__ inv_perm, const uint32_t *d_len,
-                                  Status *st) {
-    const uint32_t nt = d_len[kLenTransfers], n = d_len[kLenParticles];
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nt; k += gridDim.x * blockDim.x) {
-        const uint32_t s = t.source[k], g = t.target[k];
-        if (s >= n || g >= n) {  // a transfer naming a particle that does not exist
-            set_flag(st, APBF_FLAG_NONFINITE);
-            continue;
-        }
-        t.source[k] = inv_perm[s];
-        t.target[k] = inv_perm[g];
-    }
-}
-
 // find_value_ranges.comp:15-31 (cell arrays zeroed beforehand).
+// The transfer list follows the reorder here as well.
 __global__ void k_cell_ranges(const uint32_t *__restrict__ skeys, const uint32_t *d_len, uint32_t *__restrict__ start,
-                              uint32_t *__restrict__ end) {
+                              uint32_t *__restrict__ end, TransferBufs tr, const uint32_t *__restrict__ inv_perm,
+                              Status *st) {
     uint32_t n = d_len[kLenParticles];
+    remap_transfers(tr, inv_perm, d_len, st);
     for (uint32_t id = blockIdx.x * blockDim.x + threadIdx.x; id < n; id += gridDim.x * blockDim.x) {
         uint32_t cur = skeys[id];
         uint32_t prev = id == 0 ? cur : skeys[id - 1];
@@ -154,7 +146,7 @@ struct BuildArgs {
 };
 
 // Appends an entry to a correction row (the reverse-row arrays; their counts were
-// zeroed before the walk, and any walk may append, so the slot is an atomic).
+// zeroed by the walk, and any row may append, so the slot is an atomic).
 __device__ __forceinline__ void push_correction(const BuildArgs &a, uint32_t row, uint32_t entry) {
     const uint32_t slot = atomicAdd(&a.ucount[row], 1u);
     if (slot < a.maxn) {
@@ -366,6 +358,7 @@ __global__ void __launch_bounds__(kBuildThreads, 6) k_build_rows(BuildArgs a) {
             const uint32_t kept = min(c, a.maxn);
             s_cnt[slot] = kept;
             if (valid) {
+                a.ucount[i] = 0u;  // no correction rows yet
                 if (c > a.maxn) {
                     set_flag(a.st, APBF_FLAG_NEIGHBOR_OVERFLOW);
                     atomicMax(&a.st->required_neighbors, c);
@@ -434,12 +427,6 @@ __global__ void k_clamp_rev(const uint32_t *d_len, uint32_t maxn, uint32_t *rcou
         if (rcount[i] > maxn) rcount[i] = maxn;
 }
 
-__global__ void k_reset_search(Status *st, unsigned long long *total) {
-    st->range_min = 0xffffffffffffffffull;
-    st->range_max = 0ull;
-    *total = 0ull;
-}
-
 // Pair export (the reference's uvec2 list): row-major order of the rows.
 __global__ void k_export_pairs(const uint32_t *d_len, uint32_t stride, const uint32_t *__restrict__ count,
                                const uint32_t *__restrict__ idx, const uint32_t *__restrict__ offsets, uint32_t cap,
@@ -463,7 +450,8 @@ void swap_all(apbf_ctx *ctx) { ctx->fcur ^= 1; }
 }  // namespace
 
 // Gathers every particle attribute in the order ctx->perm gives (new id -> old id),
-// remaps the transfer and glue lists, and makes the gathered set current.
+// remaps the glue list, and makes the gathered set current; the transfer list is left to
+// the caller's next kernel (remap_transfers with ctx->inv_perm).
 // With `search` the gather also writes the search records (srec) for range scale
 // `scale` and reduces the search radii's range into the status block.
 apbf_status reorder_particles(apbf_ctx *ctx, cudaStream_t s, bool search, float scale) {
@@ -474,10 +462,6 @@ apbf_status reorder_particles(apbf_ctx *ctx, cudaStream_t s, bool search, float 
     k_reorder<<<grid_for(ctx, cap), kBlock, 0, s>>>(cur, alt, ctx->perm, ctx->inv_perm, ctx->d_len,
                                                     search ? ctx->srec : nullptr, scale, ctx->status);
     APBF_AFTER_LAUNCH(ctx, s, "k_reorder");
-    APBF_BEFORE_LAUNCH(ctx, s, "k_remap_transfers");
-    k_remap_transfers<<<grid_for(ctx, ctx->cfg.transfer_capacity), kBlock, 0, s>>>(ctx->tr[ctx->tcur], ctx->inv_perm,
-                                                                                    ctx->d_len, ctx->status);
-    APBF_AFTER_LAUNCH(ctx, s, "k_remap_transfers");
     apbf_status r = glue_remap(ctx, s);
     if (r != APBF_OK) return r;
     swap_all(ctx);
@@ -496,24 +480,22 @@ apbf_status neighborhood_green(apbf_ctx *ctx, float range_scale, const float min
     const int g = grid_for(ctx, cap);
 
     APBF_BEFORE_LAUNCH(ctx, s, "k_position_keys");
-    k_position_keys<<<g, kBlock, 0, s>>>(cur.pos, ctx->d_len, b, L, ctx->keys[0], ctx->vals[0]);
+    k_position_keys<<<g, kBlock, 0, s>>>(cur.pos, ctx->d_len, b, L, ctx->keys[0], ctx->vals[0], ctx->status,
+                                         ctx->d_pairs);
     APBF_AFTER_LAUNCH(ctx, s, "k_position_keys");
     apbf_status r = sort_pairs_device(ctx, ctx->keys[0], ctx->vals[0], ctx->d_len + kLenParticles, cap, 3u * L,
                                       ctx->sorted_keys, ctx->perm, s);
     if (r != APBF_OK) return r;
-    // the reorder reduces the search radii's range: reset it first
-    APBF_BEFORE_LAUNCH(ctx, s, "k_reset_search");
-    k_reset_search<<<1, 1, 0, s>>>(ctx->status, ctx->d_pairs);
-    APBF_AFTER_LAUNCH(ctx, s, "k_reset_search");
     r = reorder_particles(ctx, s, true, range_scale);
     if (r != APBF_OK) return r;
     FluidBufs &f = ctx->fl[ctx->fcur];
 
     const size_t ncells = (size_t)1 << (3 * L);
-    APBF_CUDA(cudaMemsetAsync(ctx->cell_start, 0, ncells * sizeof(uint32_t), s));
-    APBF_CUDA(cudaMemsetAsync(ctx->cell_end, 0, ncells * sizeof(uint32_t), s));
+    uint32_t *cell_start = ctx->cells, *cell_end = ctx->cells + ncells;
+    APBF_CUDA(cudaMemsetAsync(ctx->cells, 0, 2 * ncells * sizeof(uint32_t), s));
     APBF_BEFORE_LAUNCH(ctx, s, "k_cell_ranges");
-    k_cell_ranges<<<g, kBlock, 0, s>>>(ctx->sorted_keys, ctx->d_len, ctx->cell_start, ctx->cell_end);
+    k_cell_ranges<<<g, kBlock, 0, s>>>(ctx->sorted_keys, ctx->d_len, cell_start, cell_end, ctx->tr[ctx->tcur],
+                                       ctx->inv_perm, ctx->status);
     APBF_AFTER_LAUNCH(ctx, s, "k_cell_ranges");
     APBF_BEFORE_LAUNCH(ctx, s, "k_build_rows");
     BuildArgs ba;
@@ -533,8 +515,8 @@ apbf_status neighborhood_green(apbf_ctx *ctx, float range_scale, const float min
     ba.fast_ok = 1;
     for (int d = 0; d < 3; ++d)
         if (b.hi[d] - b.lo[d] >= (1ll << 31)) ba.fast_ok = 0;
-    ba.cstart = ctx->cell_start;
-    ba.cend = ctx->cell_end;
+    ba.cstart = cell_start;
+    ba.cend = cell_end;
     ba.stride = ctx->row_stride;
     ba.maxn = ctx->cfg.max_neighbors;
     ba.count = ctx->nb_count;
@@ -546,7 +528,6 @@ apbf_status neighborhood_green(apbf_ctx *ctx, float range_scale, const float min
     ba.uidx = ctx->rev_idx;
     ba.one_sided = ctx->flag_scan;  // scratch: not in use during the search
     ba.corrections = corrections ? 1 : 0;
-    APBF_CUDA(cudaMemsetAsync(ctx->rev_count, 0, (size_t)cap * sizeof(uint32_t), s));  // correction rows
     // threads per particle: as many as it takes to fill the chip, since a smaller group
     // shares less of its steps' fixed cost.  8 / 16 / 32 threads: 28 / 21 / 17 us at 2 197
     // particles, 60 / 55 / 60 at 32 768, 206 / 222 / 290 at 250 000, 663 / 794 / 1087 at a million
@@ -557,17 +538,22 @@ apbf_status neighborhood_green(apbf_ctx *ctx, float range_scale, const float min
     else
         k_build_rows<8><<<grid_for(ctx, cap, kBuildThreads / 8, 64), kBuildThreads, 0, s>>>(ba);
     APBF_AFTER_LAUNCH(ctx, s, "k_build_rows");
-    APBF_BEFORE_LAUNCH(ctx, s, "k_corrections");
-    k_corrections<<<grid_for(ctx, cap), kBlock, 0, s>>>(ba);
-    APBF_AFTER_LAUNCH(ctx, s, "k_corrections");
+    if (corrections) {
+        APBF_BEFORE_LAUNCH(ctx, s, "k_corrections");
+        k_corrections<<<grid_for(ctx, cap), kBlock, 0, s>>>(ba);
+        APBF_AFTER_LAUNCH(ctx, s, "k_corrections");
+    }
     if (fuse_box) {  // the box-collided positions are the current ones now
         int4 *t = f.pos;
         f.pos = spare.pos;
         spare.pos = t;
     }
-    APBF_BEFORE_LAUNCH(ctx, s, "k_clamp_rev");
-    k_clamp_rev<<<grid_for(ctx, cap), kBlock, 0, s>>>(ctx->d_len, ctx->cfg.max_neighbors, ctx->rev_count, ctx->status);
-    APBF_AFTER_LAUNCH(ctx, s, "k_clamp_rev");
+    if (corrections) {
+        APBF_BEFORE_LAUNCH(ctx, s, "k_clamp_rev");
+        k_clamp_rev<<<grid_for(ctx, cap), kBlock, 0, s>>>(ctx->d_len, ctx->cfg.max_neighbors, ctx->rev_count,
+                                                          ctx->status);
+        APBF_AFTER_LAUNCH(ctx, s, "k_clamp_rev");
+    }
     return APBF_OK;
 }
 

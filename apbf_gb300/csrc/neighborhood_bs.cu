@@ -72,18 +72,18 @@ __global__ void k_code_word(const int4 *__restrict__ pos, const uint32_t *d_len,
     }
 }
 
-__global__ void k_sorted_codes(const int4 *__restrict__ pos, const uint32_t *d_len, ulonglong2 *__restrict__ code) {
+// Also: the transfer list follows the reorder, and the first thread resets what the search
+// and the solve behind it count from.
+__global__ void k_sorted_codes(const int4 *__restrict__ pos, const uint32_t *d_len, ulonglong2 *__restrict__ code,
+                               TransferBufs tr, const uint32_t *__restrict__ inv_perm, Status *st,
+                               unsigned long long *total) {
     const uint32_t n = d_len[kLenParticles];
+    if (blockIdx.x == 0 && threadIdx.x == 0) reset_search(st, total);
+    remap_transfers(tr, inv_perm, d_len, st);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int4 p = pos[i];
         code[i] = code96((uint32_t)p.x, (uint32_t)p.y, (uint32_t)p.z);
     }
-}
-
-__global__ void k_bs_reset(Status *st, unsigned long long *total) {
-    st->range_min = 0xffffffffffffffffull;
-    st->range_max = 0ull;
-    *total = 0ull;
 }
 
 // First index j in [0, n) with code[j] >= t (n when none), searched outward from
@@ -231,11 +231,9 @@ apbf_status neighborhood_binary_search(apbf_ctx *ctx, float range_scale, cudaStr
     if (r != APBF_OK) return r;
     FluidBufs &f = ctx->fl[ctx->fcur];
     APBF_BEFORE_LAUNCH(ctx, s, "k_sorted_codes");
-    k_sorted_codes<<<g, kBlock, 0, s>>>(f.pos, ctx->d_len, ctx->pos_code);
+    k_sorted_codes<<<g, kBlock, 0, s>>>(f.pos, ctx->d_len, ctx->pos_code, ctx->tr[ctx->tcur], ctx->inv_perm,
+                                        ctx->status, ctx->d_pairs);
     APBF_AFTER_LAUNCH(ctx, s, "k_sorted_codes");
-    APBF_BEFORE_LAUNCH(ctx, s, "k_bs_reset");
-    k_bs_reset<<<1, 1, 0, s>>>(ctx->status, ctx->d_pairs);
-    APBF_AFTER_LAUNCH(ctx, s, "k_bs_reset");
     FluidBufs &spare = ctx->fl[ctx->fcur ^ 1];
     BsArgs a;
     a.pos = f.pos;
