@@ -67,7 +67,8 @@ struct Status {
     uint32_t density_passes;       // density passes executed (not skipped after convergence)
     uint32_t converged;            // set by a density pass whose error met the target
     uint32_t converged_substeps;   // substeps in which a density pass met the target
-    uint32_t pass_index;           // solve loop graph: index of the first pass of the current body run
+    uint32_t pass_start;           // solve loop graph: number of the next body run's first pass
+    uint32_t pass_index;           // its copy for the kernels behind the body's first one
     uint32_t loop_iters;           // solve loop graph: body runs since the context was created
     uint32_t filter_tag;           // 1: this pass's density kernel left the boundariness filter to k_delta
     uint32_t union_rows;           // 1: the reverse-row arrays hold correction rows (see neighborhood.cu)
@@ -460,8 +461,10 @@ struct SolveOpts {
     bool later_pass = false;  // not the first pass of a substep (the widths' uniformity is known)
     bool behind = true;       // a pass behind another one's position update in the stream
     bool tiles = false;       // over the tiles of tile_rows (the substep's rows, unchanged since)
-    int loop_offset = -1;     // >= 0: a pass of the solve loop graph, number = pass_index + offset;
+    int loop_offset = -1;     // >= 0: a pass of the solve loop graph, number = pass_start + offset;
     uint32_t max_passes = 0;  //   skipped from max_passes on, box after it unless it is the last
+    bool loop_end = false;    // the body's last pass: its position update decides whether to go on
+    unsigned long long loop_handle = 0;  //   (the loop's conditional handle)
 };
 apbf_status incompressibility(apbf_ctx *ctx, cudaStream_t s, const SolveOpts &o = SolveOpts());
 // The tiled passes: whether the solve qualifies, and the rewriting of the rows the
@@ -543,7 +546,7 @@ __device__ __forceinline__ void reset_search(Status *st, unsigned long long *tot
     st->range_min = 0xffffffffffffffffull;
     st->range_max = 0ull;
     st->converged = 0u;
-    st->pass_index = 1u;
+    st->pass_start = 1u;
     *total = 0ull;
 }
 

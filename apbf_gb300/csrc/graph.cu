@@ -6,7 +6,7 @@
 // the maximum count from the host costs two kernel launches per skipped pass.
 // Here passes 1.. of a substep are one CUDA graph: a while-conditional node whose
 // body runs two passes (A -> B, B -> A, so the buffer roles are the same on every
-// run) and a one-thread kernel that advances the device pass counter and keeps the
+// run); the second one's position update advances the device pass counter and keeps the
 // loop going while no pass met the target and passes remain (the search of the substep
 // set the counter to 1).  Passes past the
 // last one inside a body run copy the positions through, as a converged pass does.
@@ -23,14 +23,6 @@ namespace apbf {
 
 namespace {
 
-__global__ void k_loop_next(cudaGraphConditionalHandle h, Status *st, uint32_t max_passes) {
-    const uint32_t next = st->pass_index + 2u;
-    st->pass_index = next;
-    st->loop_iters += 1u;
-    const uint32_t go = (*(volatile uint32_t *)&st->converged == 0u && next < max_passes) ? 1u : 0u;
-    cudaGraphSetConditional(h, go);
-}
-
 void release(SolveGraph &g) {
     if (g.exec) cudaGraphExecDestroy(g.exec);
     if (g.graph) cudaGraphDestroy(g.graph);
@@ -44,7 +36,7 @@ void destroy_solve_graphs(apbf_ctx *ctx) {
     ctx->solve_graph_next = 0;
 }
 
-// Records the loop body (two passes + the loop-condition kernel) into `body` on
+// Records the loop body (two passes, the second of which sets the loop's condition) into `body` on
 // stream cs (which must not be capturing anything else).
 static apbf_status capture_loop_body(apbf_ctx *ctx, cudaStream_t cs, cudaGraph_t body, cudaGraphConditionalHandle h,
                                      const SolveOpts &o) {
@@ -57,11 +49,9 @@ static apbf_status capture_loop_body(apbf_ctx *ctx, cudaStream_t cs, cudaGraph_t
         q.loop_offset = k;
         q.box_after = true;  // decided per pass on the device
         q.behind = k > 0;    // the body starts behind the loop's condition
+        q.loop_end = k == 1;
+        q.loop_handle = h;
         r = incompressibility(ctx, cs, q);
-    }
-    if (r == APBF_OK) {
-        k_loop_next<<<1, 1, 0, cs>>>(h, ctx->status, o.max_passes);
-        if (cudaGetLastError() != cudaSuccess) r = APBF_ERR_CUDA;
     }
     ctx->capturing = was;
     cudaGraph_t captured = nullptr;

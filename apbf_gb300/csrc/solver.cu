@@ -80,7 +80,7 @@ struct PassA {
     const float4 *vel;   // velocities, for the divergence feature
     const float *lam_prev;  // lambda_prev: the previous substep's sum at pass 0, this substep's after
     int projected;          // 1: pull-back allowed (passes after the first of a warm-started substep)
-    int loop_offset;        // >= 0: solve loop pass number = st->pass_index + loop_offset
+    int loop_offset;        // >= 0: solve loop pass number = st->pass_start + loop_offset
     uint32_t max_passes;    // loop passes from this number on are skipped
     int4 *filt;             // non-null: Gauss filter deferred to the position pass when rows are symmetric
     float target;        // > 0: set st->converged when the error is at most this
@@ -232,8 +232,8 @@ struct RowSums {
 template <bool GAUSS, bool XTRA>
 __device__ __forceinline__ bool density_finish(const PassA &a, const int4 *pos, uint32_t i, const int4 &p, float kw,
                                                const KConst &c, const GaussPair &gp, uint32_t cnt, const RowSums &rs,
-                                               float im, float radius, float b, bool feat, bool defer, bool write_rec,
-                                               PassSums &ps, float3 &ed) {
+                                               float im, float radius, float b, float pushed, bool feat, bool defer,
+                                               bool write_rec, PassSums &ps, float3 &ed) {
     bool ask = false;
     uint32_t dens = rs.dens;
     const uint32_t sq = rs.sq;
@@ -276,7 +276,7 @@ __device__ __forceinline__ bool density_finish(const PassA &a, const int4 *pos, 
     float applied = lam < 0.0f ? lam : 0.0f;
     float pull = 0.0f;
     if (a.projected && lam > 0.0f) {
-        applied = fminf(lam, -a.lam_prev[i]);  // lam_prev: the sum applied so far (<= 0)
+        applied = fminf(lam, -pushed);  // the sum applied so far (<= 0)
         if (applied > 0.0f) pull = under * (applied / lam);
         else applied = 0.0f;
     }
@@ -457,7 +457,8 @@ __device__ __forceinline__ void density_one(const PassA &a, const int4 *__restri
         rs.div = div;
         rs.nprev = nprev;
         float3 ed;
-        if (!density_finish<GAUSS, XTRA>(a, pos, i, p, kw, c, gp, cnt, rs, im, radius, b, feat, defer, write_rec, ps, ed))
+        if (!density_finish<GAUSS, XTRA>(a, pos, i, p, kw, c, gp, cnt, rs, im, radius, b,
+                                           a.projected ? a.lam_prev[i] : 0.0f, feat, defer, write_rec, ps, ed))
             return;
         // batches of kUnroll neighbours in row order, software-pipelined as the sums above
         // (the first hit ends the test, as in the plain loop)
@@ -534,10 +535,19 @@ __device__ __forceinline__ void finish_pass(double *red_out, Status *st, float t
     }
 }
 
+// Whether a pass of the solve loop graph lies past the limit.  The body's first kernel
+// reads pass_start, which its last one advances, and leaves a copy for the kernels between
+// them: so no kernel writes a word that its own blocks read.
+__device__ __forceinline__ bool loop_over(const PassA &a) {
+    if (a.loop_offset < 0) return false;
+    const uint32_t first = a.loop_offset == 0 ? a.st->pass_start : a.st->pass_index;
+    if (a.loop_offset == 0 && blockIdx.x == 0 && threadIdx.x == 0) a.st->pass_index = first;
+    return first + (uint32_t)a.loop_offset >= a.max_passes;
+}
+
 template <bool GAUSS, int L, bool XTRA>
 __global__ void __launch_bounds__(256, GAUSS ? 4 : 3) k_density_lambda(PassA a) {
-    const bool skip = (a.early_exit && *(volatile uint32_t *)&a.st->converged) ||
-                      (a.loop_offset >= 0 && a.st->pass_index + (uint32_t)a.loop_offset >= a.max_passes);
+    const bool skip = (a.early_exit && *(volatile uint32_t *)&a.st->converged) || loop_over(a);
     // With symmetric rows or union rows the Gauss filter runs in this pass's position
     // update, which gathers over the same neighbours anyway; filter_tag tells it whether to.
     const bool defer = GAUSS && a.filt && a.method == 2 &&
@@ -600,6 +610,8 @@ struct PassB {
     float *lam_acc;   // this pass applied (rec.x: the learned one in a learned pass)
     int prev_mode, acc_mode;
     int loop_offset;      // >= 0: solve loop pass number = st->pass_index + loop_offset
+    int loop_end;         // 1: the loop body's last pass, which sets the loop's condition
+    cudaGraphConditionalHandle loop_handle;
     uint32_t max_passes;  // loop passes from this number on copy through; box after all but the last
     const int4 *filt;     // the density pass's deferred Gauss filter (gradient sum, boundariness > 0)
     float *bness;
@@ -860,6 +872,24 @@ struct UpdateHead {
     uint32_t n, nboxes;
     bool skip, filter, sym, corr, packed;
 };
+// The books of a pass and the slot of the next (one warp); a call, so that its few
+// instructions in one block cost the others no registers.
+__device__ __noinline__ void update_books(const PassB &a, uint32_t n, uint32_t slot, PassTotals t, bool ran, bool met) {
+    if (threadIdx.x < (uint32_t)kSumStripes)
+        for (int k = 0; k < 3; ++k) a.sync->e[slot ^ 1u][threadIdx.x][k] = 0ull;
+    if (threadIdx.x != 0u) return;
+    if (ran) {
+        a.st->kw_uniform = t.kw_diff ? 0u : 1u;
+        finish_pass(a.red_out, a.st, a.target, n, (long long)t.e1, (long long)t.e2, met);
+    }
+    a.sync->cur_density = slot ^ 1u;
+    if (a.loop_end) {  // once more while no pass met the target and passes remain
+        const uint32_t next = a.st->pass_index + 2u;
+        a.st->pass_start = next;
+        a.st->loop_iters += 1u;
+        cudaGraphSetConditional(a.loop_handle, a.st->converged == 0u && next < a.max_passes ? 1u : 0u);
+    }
+}
 template <bool GAUSS>
 __device__ __forceinline__ UpdateHead update_head(const PassB &a, uint32_t n) {
     UpdateHead h;
@@ -877,17 +907,7 @@ __device__ __forceinline__ UpdateHead update_head(const PassB &a, uint32_t n) {
     // this pass, and reading it early or late gives the same answer
     const bool ran = !h.skip;
     if (ran && a.early_exit) h.skip = error_meets_target(t.e1, n, a.target, a.target_m, a.target_s);
-    if (blockIdx.x == 0 && threadIdx.x < 32u) {  // the books of this pass, and the slot of the next
-        if (threadIdx.x < (uint32_t)kSumStripes)
-            for (int k = 0; k < 3; ++k) a.sync->e[slot ^ 1u][threadIdx.x][k] = 0ull;
-        if (threadIdx.x == 0) {
-            if (ran) {
-                a.st->kw_uniform = t.kw_diff ? 0u : 1u;
-                finish_pass(a.red_out, a.st, a.target, n, (long long)t.e1, (long long)t.e2, h.skip);
-            }
-            a.sync->cur_density = slot ^ 1u;
-        }
-    }
+    if (blockIdx.x == 0 && threadIdx.x < 32u) update_books(a, n, slot, t, ran, h.skip);
     // the density pass of this pass deferred the Gauss filter to here (symmetric rows)
     h.filter = GAUSS && *(volatile const uint32_t *)&a.st->filter_tag != 0u;
     // Rows: symmetric (equal radii) or with correction rows (the green search with
@@ -1239,8 +1259,7 @@ __global__ void __launch_bounds__(T *L, 1024 / (T * L)) k_density_tiles(PassA a,
         const uint32_t depth = over ? 0u : min(cnt, (uint32_t)kTileDepth);
         if (tile == blockIdx.x) {
             grid_dependency_wait();
-            const bool skip = (a.early_exit && *(volatile uint32_t *)&a.st->converged) ||
-                              (a.loop_offset >= 0 && a.st->pass_index + (uint32_t)a.loop_offset >= a.max_passes);
+            const bool skip = (a.early_exit && *(volatile uint32_t *)&a.st->converged) || loop_over(a);
             defer = a.filt && a.method == 2 && (a.st->range_min == a.st->range_max || a.st->union_rows != 0u);
             slot = *(volatile uint32_t *)&a.sync->cur_density & 1u;
             if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1255,7 +1274,7 @@ __global__ void __launch_bounds__(T *L, 1024 / (T * L)) k_density_tiles(PassA a,
             v.w = __float_as_int(__int_as_float(v.w) * APBF_FIX);
             s_pos[k] = v;
         };
-        const float b0 = a.bness[i];
+        const float b0 = a.bness[i], pushed = a.projected ? a.lam_prev[i] : 0.0f;
         for (uint32_t k = threadIdx.x; k < T; k += B)
             if (k < head.y) {
                 const int4 v = a.pos[base + k];
@@ -1364,7 +1383,7 @@ __global__ void __launch_bounds__(T *L, 1024 / (T * L)) k_density_tiles(PassA a,
         bool ask = false;
         if (valid && sub == 0)
             ask = density_finish<true, false>(a, a.pos, i, make_int4(p.x, p.y, p.z, 0), kw, c, gp, cnt, rs, im, radius, b0,
-                                              false, defer, false, one, ed);
+                                              pushed, false, defer, false, one, ed);
         if (__any_sync(0xffffffffu, ask)) {  // the boundariness filter of transposed rows
             bool hit = false;
             if (ask) {
@@ -1504,6 +1523,7 @@ __global__ void __launch_bounds__(T *L, 896 / (T * L)) k_delta_tiles(PassB a, Ti
         const uint32_t o = valid ? lane & 255u : 0u, j = base + o;
         const uint32_t cnt = valid ? lane >> 8 : 0u;
         const uint32_t depth = over ? 0u : min(cnt, (uint32_t)kTileDepth);
+        const uint32_t corrections = own ? a.rcount[j] : 0u;
         if (threadIdx.x < min(a.nboxes, kTileBoxes)) tile_box(a, threadIdx.x, __uint_as_float(head.z), s_box);
         if (tile == blockIdx.x) {
             grid_dependency_wait();
@@ -1512,9 +1532,12 @@ __global__ void __launch_bounds__(T *L, 896 / (T * L)) k_delta_tiles(PassB a, Ti
                 if (threadIdx.x == 0) s_head = h;
             }
         }
-        const int4 shj = valid ? a.shift[j] : make_int4(0, 0, 0, 0);
+        // everything the particle needs to its end, so that no load waits behind the row
+        const int4 shj = valid ? a.shift[j] : make_int4(0, 0, 0, 0), fj = a.filt[j];
         const float2 kcj = a.kc[j];
+        const int4 p = a.pk[j];  // w: the applied (learned) lambda
         const int pw = a.pos[j].w;  // the mass rides along
+        const float pushed = a.prev_mode == 2 ? a.lam_prev[j] : 0.0f;
         const auto stage = [&](uint32_t k, uint32_t g) {
             int4 v = a.pk[g];
             v.w = __float_as_int(__int_as_float(v.w) * APBF_FIX);
@@ -1533,10 +1556,7 @@ __global__ void __launch_bounds__(T *L, 896 / (T * L)) k_delta_tiles(PassB a, Ti
         for (uint32_t k = threadIdx.x + 2 * B; k < H; k += B) stage(2 * T + k, halo[k]);
         bool fil = false, hit = false, near = false;  // this particle's deferred filter, a neighbour cleared it or may have
         float3 ed = make_float3(0.f, 0.f, 0.f);
-        if (shj.w != 0) {  // (only a deferred filter sets it)
-            const int4 fj = a.filt[j];
-            fil = filter_dir(fj.x, fj.y, fj.z, ed);
-        }
+        if (shj.w != 0) fil = filter_dir(fj.x, fj.y, fj.z, ed);  // (only a deferred filter sets it)
         __syncthreads();
         if (tile == blockIdx.x) {
             h = s_head;
@@ -1547,7 +1567,6 @@ __global__ void __launch_bounds__(T *L, 896 / (T * L)) k_delta_tiles(PassB a, Ti
             if (n == 0u) return;
             fil = fil && h.filter;
         }
-        const int4 p = s_pk[o];
         const GaussPair cj = gauss_pair(kcj.x, kcj.y);
         const int3 start = sub == 0 ? make_int3(shj.x, shj.y, shj.z) : make_int3(0, 0, 0);
         int3 acc = start;
@@ -1682,7 +1701,7 @@ __global__ void __launch_bounds__(T *L, 896 / (T * L)) k_delta_tiles(PassB a, Ti
             }
         }
         if (h.corr) {  // the correction row (radii that differ): usually empty
-            const uint32_t m = valid ? a.rcount[j] : 0u;
+            const uint32_t m = valid ? corrections : 0u;
             if (m)
                 acc = h.packed ? delta_corrections<true, L, true>(a, a.pos, m, j, sub, p, cj, acc)
                                : delta_corrections<true, L, false>(a, a.pos, m, j, sub, p, cj, acc);
@@ -1699,7 +1718,7 @@ __global__ void __launch_bounds__(T *L, 896 / (T * L)) k_delta_tiles(PassB a, Ti
             }
         }
         if (valid && sub == 0) {
-            const float lj = (a.prev_mode | a.acc_mode) ? __int_as_float(a.pk[j].w) : 0.0f;
+            const float lj = __int_as_float(p.w);
             uint32_t nb = h.nboxes, first = 0;
             int4 v = make_int4(wadd(p.x, acc.x), wadd(p.y, acc.y), wadd(p.z, acc.z), pw);
             if (nb && nb <= kTileBoxes) {
@@ -1712,7 +1731,10 @@ __global__ void __launch_bounds__(T *L, 896 / (T * L)) k_delta_tiles(PassB a, Ti
                 }
             }
             if (nb) v = box_push_from(v, a.radius[j], j, a.bmin, a.bmax, a.rot, first, nb);
-            delta_store(a, a.pos_out, j, v, hit, 0.0f, lj, 0u);
+            if (hit) a.bness[j] = 0.0f;
+            a.pos_out[j] = v;
+            if (a.prev_mode) a.lam_prev[j] = a.prev_mode == 1 ? lj : pushed + lj;
+            accumulate(a.lam_acc, a.acc_mode, j, lj);
         }
         if (tile + gridDim.x < (n + T - 1) / T) __syncthreads();  // the shared records are the next tile's
     }
@@ -2171,6 +2193,8 @@ static PassB make_pass_b(apbf_ctx *ctx, const SolveOpts &o) {
     b.acc_mode = o.acc_mode;
     b.loop_offset = o.loop_offset;
     b.max_passes = o.max_passes;
+    b.loop_end = o.loop_end ? 1 : 0;
+    b.loop_handle = o.loop_handle;
     b.filt = ctx->filt;
     b.bness = f.boundariness;
     return b;
