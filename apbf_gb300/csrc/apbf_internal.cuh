@@ -221,6 +221,8 @@ struct apbf_ctx {
     uint32_t *inv_perm = nullptr;
     uint32_t *cells = nullptr;             // per cell: first particle; then per cell: end
     ulonglong2 *pos_code = nullptr;        // per particle: 96-bit position code {bits 0-63, bits 64-95}
+    ulonglong2 *bs_table = nullptr;        // cells of the binary-search rows (neighborhood_bs.cu)
+    uint32_t bs_slots = 0;                 // its slots, a power of two above the capacity
     int4 *srec = nullptr;                  // per particle: search record (position xyz, fixed-point radius)
     int search_method = APBF_NEIGHBORHOOD_GREEN;  // the substep's neighbour search
 

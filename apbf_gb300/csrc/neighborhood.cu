@@ -16,9 +16,9 @@
 //     scattering with atomics, and no transpose is needed.
 //  6. k_reverse_rows (binary-search rows and pruned rows): the transpose.
 #include <algorithm>
-#include <type_traits>
 
 #include "apbf_internal.cuh"
+#include "rowwalk.cuh"
 
 namespace apbf {
 namespace {
@@ -133,7 +133,7 @@ struct BuildArgs {
     const uint32_t *d_len;
     Bounds b;
     uint32_t L;
-    int fast_ok;  // the grid spans less than 2^31 units on every axis
+    int fast_ok;  // the grid spans less than 2^31 units on every axis, within the range of 32 bits
     const uint32_t *cstart, *cend;
     uint32_t stride, maxn;
     uint32_t *count, *idx;
@@ -155,38 +155,6 @@ __device__ __forceinline__ void push_correction(const BuildArgs &a, uint32_t row
         set_flag(a.st, APBF_FLAG_NEIGHBOR_OVERFLOW);
         atomicMax(&a.st->required_neighbors, slot + 1u);
     }
-}
-
-// Squared distance of two fixed-point positions when no axis differs by more than R
-// (else ~0: the pair is beyond R whatever the other axes).  FAST: both lie inside
-// the grid, so the 32-bit differences cannot wrap.
-template <bool FAST>
-__device__ __forceinline__ unsigned long long dist2_within(int4 a, int4 b, uint32_t R) {
-    uint32_t ax, ay, az;
-    if (FAST) {
-        ax = (uint32_t)abs(b.x - a.x);
-        ay = (uint32_t)abs(b.y - a.y);
-        az = (uint32_t)abs(b.z - a.z);
-    } else {
-        long long dx = (long long)b.x - a.x, dy = (long long)b.y - a.y, dz = (long long)b.z - a.z;
-        dx = dx < 0 ? -dx : dx;
-        dy = dy < 0 ? -dy : dy;
-        dz = dz < 0 ? -dz : dz;
-        if (dx > (long long)R || dy > (long long)R || dz > (long long)R) return ~0ull;
-        ax = (uint32_t)dx;
-        ay = (uint32_t)dy;
-        az = (uint32_t)dz;
-    }
-    if (max(ax, max(ay, az)) > R) return ~0ull;
-    return (unsigned long long)ax * ax + (unsigned long long)ay * ay + (unsigned long long)az * az;
-}
-
-// box_push as a call: the walk's kernel is bound by its instruction cache, and the
-// box pass runs once per particle.
-__device__ __noinline__ int4 box_push_call(int4 ip, float r, uint32_t id, const float4 *__restrict__ bmin,
-                                           const float4 *__restrict__ bmax, const float4 *__restrict__ rot,
-                                           uint32_t nb) {
-    return box_push(ip, r, id, bmin, bmax, rot, nb);
 }
 
 // The one-sided pairs of the rows just built (radii that differ; particles whose
@@ -215,13 +183,10 @@ __global__ void k_corrections(BuildArgs a) {
 // in z, y, x order and their particles in list order.
 //
 // A thread per particle (as this kernel once was) is a chain of dependent loads, 120 us
-// however few the particles (now 17 us at 2 197, 55 at 32 768), and idles at 12 of 32 lanes
-// where their cells differ in length (250 000: 260 against 206 us, a million: 800 against
-// 663; bound by instruction issue).  Here a group's threads each take a cell: they load the ranges of G cells at
-// once, add up the lengths by shuffles and then test G candidates of the joined ranges at a
-// time, whatever cells they come from; a ballot gives the kept ones their places, so the
-// rows keep their order.  The rows are collected in shared memory (kRowStage entries; the
-// rest goes out directly) and written a line at a time, as they are read later.
+// however few the particles (now 10 us at 2 197, 39 at 32 768), and idles at 12 of 32 lanes
+// where their cells differ in length (250 000: 260 against 185 us, a million: 795 against
+// 606; bound by instruction issue).  Here a group's threads load the ranges of G pairs of
+// cells at once and then test the joined ranges together (RowWalk).
 //
 // Correction rows (uni, when the search radii differ): the position update of
 // particle i sums over the particles k whose rows hold i (|x_i - x_k| <= R_k),
@@ -230,41 +195,35 @@ __global__ void k_corrections(BuildArgs a) {
 // reach i (flagged kNoDelta, their terms subtracted), and particles k whose rows
 // hold i although i's radius does not reach them (added).  Both kinds are one-sided
 // pairs, counted here (one_sided) and appended by k_corrections.
-constexpr uint32_t kBuildThreads = 256, kRowStage = 64;
 
-// Sum over a group of G consecutive lanes.
-template <int G>
-__device__ __forceinline__ uint32_t group_total(uint32_t v) {
-#pragma unroll
-    for (int off = G / 2; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    return v;
-}
+// c / d of small numbers: d at most 512 and c below 2^22 by one product, exactly.
+struct SmallDiv {
+    uint32_t d, inv;
+    __device__ __forceinline__ explicit SmallDiv(uint32_t d_) : d(d_), inv(0xffffffffu / d_ + 1u) {}
+    __device__ __forceinline__ uint32_t operator()(uint32_t c, bool big) const {
+        if (big) return c / d;
+        return d == 1u ? c : __umulhi(c, inv);
+    }
+};
 
-// Squared distance as dist2_within, without its range test where the differences cannot
-// overflow the sum (FAST: below 2^31 each).
-template <bool FAST>
-__device__ __forceinline__ unsigned long long dist2_to(int4 a, int4 b, uint32_t R) {
-    if (!FAST) return dist2_within<false>(a, b, R);
-    const long long dx = b.x - a.x, dy = b.y - a.y, dz = b.z - a.z;
-    return (unsigned long long)(dx * dx) + (unsigned long long)(dy * dy) + (unsigned long long)(dz * dz);
-}
-
+// The cells are taken in pairs along x: cells 2k and 2k + 1 have neighbouring keys, so their
+// particles are one run, in the order the cells would give.  Pairs that lie beyond the
+// radius (a lower bound of the distance from the pair's box) bring nothing; a quarter of
+// the candidates are in such cells.
 template <int G>
 __global__ void __launch_bounds__(kBuildThreads, 6) k_build_rows(BuildArgs a) {
-    constexpr uint32_t P = kBuildThreads / G;  // particles per block
-    constexpr uint32_t kPad = P + 1;           // a group's consecutive places fall into different banks
-    __shared__ uint32_t s_row[kRowStage * kPad];
+    constexpr uint32_t P = RowWalk<G>::kParticles;
+    __shared__ uint32_t s_row[kRowStage * RowWalk<G>::kPad];
     __shared__ uint32_t s_cnt[P];
     const uint32_t n = a.d_len[kLenParticles];
     const uint32_t last = (1u << a.L) - 1u;
     const bool uni = a.corrections && a.st->range_min != a.st->range_max;  // the radii differ: correction rows
     if (blockIdx.x == 0 && threadIdx.x == 0) a.st->union_rows = uni ? 1u : 0u;
-    const uint32_t gl = threadIdx.x % G, slot = threadIdx.x / G;
-    const uint32_t shift = threadIdx.x & 31u & ~(uint32_t)(G - 1);  // the group's first lane in its warp
-    const uint32_t below = (1u << gl) - 1u, mine = G == 32 ? 0xffffffffu : (1u << G) - 1u;
+    RowWalk<G> w(a.srec, a.idx, a.stride, a.maxn, s_row, uni);
+    const uint32_t gl = w.gl;
     unsigned long long local = 0;
     for (uint32_t base = blockIdx.x * P; base < n; base += gridDim.x * P) {
-        const uint32_t i = base + slot;
+        const uint32_t i = base + w.slot;
         const bool valid = i < n;
         const int4 p = valid ? a.srec[i] : make_int4(0, 0, 0, -1);
         const long long R = p.w;
@@ -281,111 +240,75 @@ __global__ void __launch_bounds__(kBuildThreads, 6) k_build_rows(BuildArgs a) {
                        y0 = __shfl_sync(0xffffffffu, face, 2, G), y1 = __shfl_sync(0xffffffffu, face, 3, G),
                        z0 = __shfl_sync(0xffffffffu, face, 4, G), z1 = __shfl_sync(0xffffffffu, face, 5, G);
         if (valid && R < 0 && gl == 0u) set_flag(a.st, APBF_FLAG_NONFINITE);  // NaN or negative width: no neighbours
-        const uint32_t nx = x1 - x0 + 1u, ny = y1 - y0 + 1u, nz = z1 - z0 + 1u;
-        const uint32_t ncell = R < 0 ? 0u : nx * ny * nz;
+        const uint32_t nx = (x1 >> 1) - (x0 >> 1) + 1u, ny = y1 - y0 + 1u, nz = z1 - z0 + 1u;
+        const uint32_t npair = R < 0 ? 0u : nx * ny * nz;
         // A box that touches no edge cell of the grid only meets particles inside the grid
         // (edge cells also hold the clamped outsiders): 32-bit differences.
         const bool fast = a.fast_ok && x0 > 0 && y0 > 0 && z0 > 0 && x1 < last && y1 < last && z1 < last;
-        const bool all_fast = __all_sync(0xffffffffu, fast || ncell == 0u);
-        const uint32_t R32 = (uint32_t)max(p.w, 0);
-        const unsigned long long R2 = (unsigned long long)R32 * R32;
-        const auto range = [&](uint32_t c, uint32_t &s, uint32_t &len) {  // of the c-th cell of the box
-            s = len = 0u;
-            if (c >= ncell) return;
-            const uint32_t t = c / nx, cx = x0 + (c - t * nx), cz = z0 + t / ny, cy = y0 + t % ny;
-            const uint32_t key = morton3(cx, cy, cz);
-            s = a.cstart[key];
-            len = a.cend[key] - s;
+        const bool all_fast = __all_sync(0xffffffffu, fast || npair == 0u);
+        w.start(i, p, (uint32_t)max(p.w, 0));
+        const bool big = npair >= (1u << 22);
+        const SmallDiv by_x(nx), by_y(ny);
+        // gap of a coordinate to cells [c, e) of an axis (inside the grid)
+        const auto gap = [&](int x, int d, uint32_t c, uint32_t e) {
+            const uint32_t span = (uint32_t)(a.b.hi[d] - a.b.lo[d]);
+            const int lo = (int)a.b.lo[d];
+            const int first = lo + (int)(((unsigned long long)c * span) >> a.L),
+                      behind = lo + (int)(((unsigned long long)e * span) >> a.L);
+            return (uint32_t)max(max(first - x, x - behind), 0);
         };
-        uint32_t c = 0, one_sided = 0;
-        const uint32_t most = __reduce_max_sync(0xffffffffu, ncell);  // the warp's groups go on together
+        const auto range = [&](uint32_t c, uint32_t &s, uint32_t &len) {  // of the c-th pair of the box
+            s = len = 0u;
+            if (c >= npair) return;
+            const uint32_t t = by_x(c, big), u = by_y(t, big);
+            const uint32_t cx = 2u * ((x0 >> 1) + (c - t * nx)), cy = y0 + (t - u * ny), cz = z0 + u;
+            if (all_fast) {
+                const uint32_t gx = gap(p.x, 0, cx, cx + 2u), gy = gap(p.y, 1, cy, cy + 1u), gz = gap(p.z, 2, cz, cz + 1u);
+                if ((unsigned long long)gx * gx + (unsigned long long)gy * gy + (unsigned long long)gz * gz > w.R2) return;
+            }
+            const uint32_t key = morton3(cx, cy, cz);
+            const uint2 st = *reinterpret_cast<const uint2 *>(a.cstart + key), en = *reinterpret_cast<const uint2 *>(a.cend + key);
+            const uint32_t n0 = cx >= x0 ? en.x - st.x : 0u, n1 = cx + 1u <= x1 ? en.y - st.y : 0u;
+            s = n0 ? st.x : st.y;
+            len = n0 + n1;
+        };
+        const uint32_t most = __reduce_max_sync(0xffffffffu, npair);  // the warp's groups go on together
         uint32_t s, len;
         range(gl, s, len);
         for (uint32_t c0 = 0; c0 < most; c0 += G) {
             uint32_t ns, nlen;
             range(c0 + G + gl, ns, nlen);  // in flight while this round's candidates are tested
-            uint32_t incl = len;
-#pragma unroll
-            for (int off = 1; off < G; off <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off, G);
-                if ((int)gl >= off) incl += y;
-            }
-            const uint32_t total = __shfl_sync(0xffffffffu, incl, G - 1, G);
-            const uint32_t adj = s - (incl - len);  // candidate f of the joined ranges is particle adj + f
-            const uint32_t rounds = __reduce_max_sync(0xffffffffu, total);
-            const auto candidate = [&](uint32_t f) {  // of the cell whose run holds f
-                uint32_t k = 0;
-#pragma unroll
-                for (int off = G / 2; off > 0; off >>= 1)
-                    if (__shfl_sync(0xffffffffu, incl, k + off - 1, G) <= f) k += off;
-                return __shfl_sync(0xffffffffu, adj, k, G) + f;
-            };
-            const auto test = [&](bool in, uint32_t j, int4 q, auto fast_form) {
-                const unsigned long long d2 = dist2_to<decltype(fast_form)::value>(p, q, R32);
-                const bool keep = in && j != i && d2 <= R2;
-                const uint32_t bal = (__ballot_sync(0xffffffffu, keep) >> shift) & mine;
-                if (keep) {
-                    const uint32_t at = c + __popc(bal & below);
-                    if (at < kRowStage) s_row[at * kPad + slot] = j;
-                    else if (at < a.maxn) a.idx[(size_t)at * a.stride + i] = j;
-                    if (uni) {
-                        const unsigned long long Rj = (unsigned long long)(uint32_t)max(q.w, 0);
-                        one_sided += (q.w >= 0 && d2 <= Rj * Rj) ? 0u : 1u;
-                    }
-                }
-                c += __popc(bal);
-            };
-            const auto windows = [&](auto fast_form) {
-                for (uint32_t w = 0; w < rounds; w += 2 * G) {  // two candidates of each thread in flight
-                    const uint32_t f0 = w + gl, f1 = f0 + G;
-                    const uint32_t j0 = candidate(f0), j1 = candidate(f1);
-                    const bool in0 = f0 < total, in1 = f1 < total;
-                    const int4 q0 = in0 ? a.srec[j0] : p, q1 = in1 ? a.srec[j1] : p;
-                    test(in0, j0, q0, fast_form);
-                    test(in1, j1, q1, fast_form);
-                }
-            };
-            if (all_fast) windows(std::true_type());
-            else windows(std::false_type());
+            if (all_fast) w.template take<true>(s, len);
+            else w.template take<false>(s, len);
             s = ns;
             len = nlen;
         }
         if (uni) {
-            one_sided = group_total<G>(one_sided);
+            const uint32_t one_sided = group_total<G>(w.one_sided);
             if (valid && gl == 0u) a.one_sided[i] = one_sided;  // k_corrections appends them
         }
         if (gl == 0u) {
-            const uint32_t kept = min(c, a.maxn);
-            s_cnt[slot] = kept;
+            const uint32_t kept = min(w.count, a.maxn);
+            s_cnt[w.slot] = kept;
             if (valid) {
                 a.ucount[i] = 0u;  // no correction rows yet
-                if (c > a.maxn) {
+                if (w.count > a.maxn) {
                     set_flag(a.st, APBF_FLAG_NEIGHBOR_OVERFLOW);
-                    atomicMax(&a.st->required_neighbors, c);
+                    atomicMax(&a.st->required_neighbors, w.count);
                 }
                 a.count[i] = kept;
                 local += kept;
             }
         }
         __syncthreads();
-        {
-            const uint32_t pl = threadIdx.x % P, m = min(s_cnt[pl], kRowStage);
-            for (uint32_t k = threadIdx.x / P; k < m; k += kBuildThreads / P)
-                a.idx[(size_t)k * a.stride + base + pl] = s_row[k * kPad + pl];
-            if (a.pos_box && threadIdx.x < P && base + pl < n)
-                a.pos_box[base + pl] =
-                    box_push_call(a.pos[base + pl], a.radius[base + pl], base + pl, a.bmin, a.bmax, a.rot, a.nboxes);
+        w.write_rows(s_cnt, base);
+        if (a.pos_box && threadIdx.x < P && base + threadIdx.x < n) {
+            const uint32_t k = base + threadIdx.x;
+            a.pos_box[k] = box_push_call(a.pos[k], a.radius[k], k, a.bmin, a.bmax, a.rot, a.nboxes);
         }
         __syncthreads();  // the rows are the next particles'
     }
-    // one addition per block: a word that many SMs write costs about 25 ns a time
-    __shared__ unsigned long long s_local;
-    if (threadIdx.x == 0) s_local = 0ull;
-    __syncthreads();
-    for (int off = 16; off > 0; off >>= 1) local += __shfl_down_sync(0xffffffffu, local, off);
-    if ((threadIdx.x & 31) == 0 && local) atomicAdd(&s_local, local);
-    __syncthreads();
-    if (threadIdx.x == 0 && s_local) atomicAdd(a.total, s_local);
+    add_pairs(a.total, local);
 }
 
 __global__ void k_reverse_rows(const uint32_t *d_len, uint32_t stride, uint32_t maxn, const uint32_t *__restrict__ count,
@@ -514,7 +437,7 @@ apbf_status neighborhood_green(apbf_ctx *ctx, float range_scale, const float min
     ba.L = L;
     ba.fast_ok = 1;
     for (int d = 0; d < 3; ++d)
-        if (b.hi[d] - b.lo[d] >= (1ll << 31)) ba.fast_ok = 0;
+        if (b.hi[d] - b.lo[d] >= (1ll << 31) || b.lo[d] < -(1ll << 31) || b.hi[d] >= (1ll << 31)) ba.fast_ok = 0;
     ba.cstart = cell_start;
     ba.cend = cell_end;
     ba.stride = ctx->row_stride;
@@ -529,8 +452,9 @@ apbf_status neighborhood_green(apbf_ctx *ctx, float range_scale, const float min
     ba.one_sided = ctx->flag_scan;  // scratch: not in use during the search
     ba.corrections = corrections ? 1 : 0;
     // threads per particle: as many as it takes to fill the chip, since a smaller group
-    // shares less of its steps' fixed cost.  8 / 16 / 32 threads: 28 / 21 / 17 us at 2 197
-    // particles, 60 / 55 / 60 at 32 768, 206 / 222 / 290 at 250 000, 663 / 794 / 1087 at a million
+    // shares less of its steps' fixed cost.  8 / 16 / 32 threads (cells not yet in pairs):
+    // 28 / 21 / 17 us at 2 197 particles, 60 / 55 / 60 at 32 768, 206 / 222 / 290 at 250 000,
+    // 663 / 794 / 1087 at a million
     if (cap <= 12288u)
         k_build_rows<32><<<grid_for(ctx, cap, kBuildThreads / 32, 64), kBuildThreads, 0, s>>>(ba);
     else if (cap <= 98304u)

@@ -26,7 +26,7 @@
 //  * at k = 31 each axis has two cells, so the offsets -1 and +1 name the same cell;
 //    it is scanned once (the reference scans it twice and lists those neighbours
 //    twice).
-#include "apbf_internal.cuh"
+#include "rowwalk.cuh"
 
 namespace apbf {
 namespace {
@@ -72,28 +72,80 @@ __global__ void k_code_word(const int4 *__restrict__ pos, const uint32_t *d_len,
     }
 }
 
-// Also: the transfer list follows the reorder, and the first thread resets what the search
-// and the solve behind it count from.
-__global__ void k_sorted_codes(const int4 *__restrict__ pos, const uint32_t *d_len, ulonglong2 *__restrict__ code,
-                               TransferBufs tr, const uint32_t *__restrict__ inv_perm, Status *st,
-                               unsigned long long *total) {
+// The cells of one level as a hash table: 63-bit cell number + 1 (0: empty), first particle
+// and end of the cell's run of the sorted list.
+struct __align__(16) BsCell {
+    unsigned long long key;
+    uint32_t start, end;
+};
+__device__ __forceinline__ unsigned long long bs_key(uint32_t ux, uint32_t uy, uint32_t uz) {
+    return 1ull + ((unsigned long long)ux | (unsigned long long)uy << 21 | (unsigned long long)uz << 42);
+}
+__device__ __forceinline__ uint32_t bs_hash(unsigned long long key, uint32_t mask) {
+    return (uint32_t)((key * 0x9E3779B97F4A7C15ull) >> 32) & mask;
+}
+// The level of a search radius: the smallest k with 2^k >= R (R < 2^31, so k <= 31).
+__device__ __forceinline__ uint32_t bs_level(long long R) {
+    return R <= 1 ? 0u : 32u - (uint32_t)__clz((uint32_t)(R - 1));
+}
+constexpr uint32_t kTableLevel = 11;  // from this level on a cell number has at most 63 bits
+
+// Also: the transfer list follows the reorder, the first thread resets what the search
+// and the solve behind it count from, and the particles enter the cells of their radius's
+// level into the table (the first of a cell's run its start, the last its end).  The table
+// holds every cell when all radii have one level; the levels' range tells.  (table cleared,
+// levels {all ones, 0} beforehand.)
+__global__ void k_sorted_codes(const int4 *__restrict__ pos, const float *__restrict__ width, float scale,
+                               const uint32_t *d_len, ulonglong2 *__restrict__ code, BsCell *__restrict__ table,
+                               uint32_t mask, uint32_t *levels, TransferBufs tr, const uint32_t *__restrict__ inv_perm,
+                               Status *st, unsigned long long *total) {
     const uint32_t n = d_len[kLenParticles];
     if (blockIdx.x == 0 && threadIdx.x == 0) reset_search(st, total);
     remap_transfers(tr, inv_perm, d_len, st);
+    uint32_t kmin = 32u, kmax = 0u;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int4 p = pos[i];
         code[i] = code96((uint32_t)p.x, (uint32_t)p.y, (uint32_t)p.z);
+        const long long R = range_fixed(width[i], scale);
+        if (R < 0) {  // no cell of its own, but it may open or close another's run
+            kmin = 0u;
+            continue;
+        }
+        const uint32_t k = bs_level(R);
+        kmin = min(kmin, k);
+        kmax = max(kmax, k);
+        if (k < kTableLevel) continue;
+        const uint32_t ux = (uint32_t)p.x >> k, uy = (uint32_t)p.y >> k, uz = (uint32_t)p.z >> k;
+        const auto same = [&](int4 q) {
+            return (uint32_t)q.x >> k == ux && (uint32_t)q.y >> k == uy && (uint32_t)q.z >> k == uz;
+        };
+        const bool opens = i == 0u || !same(pos[i - 1u]), closes = i + 1u == n || !same(pos[i + 1u]);
+        if (!opens && !closes) continue;
+        const unsigned long long key = bs_key(ux, uy, uz);
+        for (uint32_t h = bs_hash(key, mask);; h = (h + 1u) & mask) {  // (never full: more slots than particles)
+            const unsigned long long was = atomicCAS(&table[h].key, 0ull, key);
+            if (was != 0ull && was != key) continue;
+            if (opens) table[h].start = i;
+            if (closes) table[h].end = i + 1u;
+            break;
+        }
+    }
+    kmin = __reduce_min_sync(0xffffffffu, kmin);
+    kmax = __reduce_max_sync(0xffffffffu, kmax);
+    if ((threadIdx.x & 31u) == 0u) {  // (a bound that already holds is left alone)
+        if (kmin < *(volatile uint32_t *)&levels[0]) atomicMin(&levels[0], kmin);
+        if (kmax > *(volatile uint32_t *)&levels[1]) atomicMax(&levels[1], kmax);
     }
 }
 
-// First index j in [0, n) with code[j] >= t (n when none), searched outward from
-// `hint` with doubling steps and then bisected: cells near a particle are mostly
-// near it in the sorted order.
-__device__ __forceinline__ uint32_t lower_bound96(const ulonglong2 *__restrict__ code, uint32_t n, uint32_t hint,
-                                                  ulonglong2 t) {
+// First index j in [0, n) with !before(code[j]) (n when none), for a predicate that holds
+// for a prefix of the list; searched outward from `hint` with doubling steps and then
+// bisected: cells near a particle are mostly near it in the sorted order.
+template <typename F>
+__device__ __forceinline__ uint32_t first_not(const ulonglong2 *__restrict__ code, uint32_t n, uint32_t hint, F before) {
     uint32_t lo, hi;  // the answer lies in [lo, hi]
-    if (less96(code[hint], t)) {
-        uint32_t a = hint, step = 1;  // code[a] < t
+    if (before(code[hint])) {
+        uint32_t a = hint, step = 1;  // before(code[a])
         for (;;) {
             const uint32_t b = step <= n - 1 - a ? a + step : n;  // index to probe, or n
             if (b >= n) {
@@ -101,7 +153,7 @@ __device__ __forceinline__ uint32_t lower_bound96(const ulonglong2 *__restrict__
                 hi = n;
                 break;
             }
-            if (!less96(code[b], t)) {
+            if (!before(code[b])) {
                 lo = a + 1;
                 hi = b;
                 break;
@@ -110,14 +162,14 @@ __device__ __forceinline__ uint32_t lower_bound96(const ulonglong2 *__restrict__
             step <<= 1;
         }
     } else {
-        uint32_t b = hint, step = 1;  // code[b] >= t
+        uint32_t b = hint, step = 1;  // !before(code[b])
         for (;;) {
             if (b == 0) {
                 lo = hi = 0;
                 break;
             }
             const uint32_t a = b > step ? b - step : 0;
-            if (less96(code[a], t)) {
+            if (before(code[a])) {
                 lo = a + 1;
                 hi = b;
                 break;
@@ -126,9 +178,9 @@ __device__ __forceinline__ uint32_t lower_bound96(const ulonglong2 *__restrict__
             step <<= 1;
         }
     }
-    while (lo < hi) {  // bisect: code[hi] >= t (or hi == n), code[lo - 1] < t
+    while (lo < hi) {  // bisect: hi == n or !before(code[hi]), before(code[lo - 1])
         const uint32_t mid = lo + (hi - lo) / 2;
-        if (less96(code[mid], t))
+        if (before(code[mid]))
             lo = mid + 1;
         else
             hi = mid;
@@ -150,64 +202,104 @@ struct BsArgs {
     uint32_t *count, *idx;
     unsigned long long *total;
     Status *st;
+    const BsCell *table;  // k_sorted_codes' cells, mask + 1 slots
+    uint32_t mask;
+    const uint32_t *levels;
 };
 
-// neighborhood_binary_search.comp:180-275, one thread per particle.
-__global__ void __launch_bounds__(256) k_bs_rows(BsArgs a) {
+// neighborhood_binary_search.comp:180-275 by groups of G threads (RowWalk): a thread per
+// cell finds its run, in the table of cells when all radii have one level, else by two
+// searches of the sorted codes.  The searches are about 40 dependent loads for each of 27
+// cells: 178 us at 64 019 particles, with the table 60.
+template <int G>
+__global__ void __launch_bounds__(kBuildThreads) k_bs_rows(BsArgs a) {
+    using Walk = RowWalk<G>;
+    __shared__ uint32_t s_row[kRowStage * Walk::kPad];
+    __shared__ uint32_t s_cnt[Walk::kParticles];
     const uint32_t n = a.d_len[kLenParticles];
+    const bool tabled = a.levels[0] == a.levels[1] && a.levels[0] >= kTableLevel;
+    Walk w(a.pos, a.idx, a.stride, a.maxn, s_row, false);
+    const uint32_t gl = w.gl;
     unsigned long long local = 0;
     long long rmin = 0x7fffffffffffffffll, rmax = -1;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int4 p = a.pos[i];
-        const long long R = range_fixed(a.range[i], a.scale);
-        uint32_t c = 0;
-        if (R < 0) {
-            set_flag(a.st, APBF_FLAG_NONFINITE);  // NaN or negative kernel width: no neighbours
-        } else {
+    for (uint32_t base = blockIdx.x * Walk::kParticles; base < n; base += gridDim.x * Walk::kParticles) {
+        const uint32_t i = base + w.slot;
+        const bool valid = i < n;
+        const int4 p = valid ? a.pos[i] : make_int4(0, 0, 0, 0);
+        const long long R = valid ? range_fixed(a.range[i], a.scale) : -1;
+        if (valid && R < 0 && gl == 0u) set_flag(a.st, APBF_FLAG_NONFINITE);  // NaN or negative width: no neighbours
+        if (R >= 0) {
             rmin = R < rmin ? R : rmin;
             rmax = R > rmax ? R : rmax;
-            // level: smallest k with 2^k >= R (R < 2^31, so k <= 31)
-            const uint32_t k = R <= 1 ? 0u : 32u - (uint32_t)__clz((uint32_t)(R - 1));
+        }
+        const uint32_t k = bs_level(R);
+        const uint32_t m = k == 31 ? 2u : 3u;  // at k = 31 the offset +1 is the offset -1
+        const uint32_t ncell = R < 0 ? 0u : m * m * m;
+        const uint32_t ux = (uint32_t)p.x >> k, uy = (uint32_t)p.y >> k, uz = (uint32_t)p.z >> k;
+        w.start(i, p, (uint32_t)(R < 0 ? 0 : R));
+        const auto range = [&](uint32_t c, uint32_t &s, uint32_t &len) {  // of the c-th cell
+            s = len = 0u;
+            if (c >= ncell) return;
+            const uint32_t t = c / m, dx = c - t * m, dz = t / m, dy = t - dz * m;
+            // the cell, wrapping modulo 2^32 like the code arithmetic
+            const uint32_t cx = (ux + dx - 1u) << k, cy = (uy + dy - 1u) << k, cz = (uz + dz - 1u) << k;
+            if (tabled) {
+                const unsigned long long key = bs_key(cx >> k, cy >> k, cz >> k);
+                for (uint32_t h = bs_hash(key, a.mask);; h = (h + 1u) & a.mask) {
+                    const uint4 e = *reinterpret_cast<const uint4 *>(&a.table[h]);
+                    const unsigned long long found = (unsigned long long)e.y << 32 | e.x;
+                    if (found == 0ull) return;
+                    if (found != key) continue;
+                    s = e.z;
+                    len = e.w - e.z;
+                    return;
+                }
+            }
             const uint32_t d3 = 3u * k;  // the code bits below the cell
             const ulonglong2 m96 = make_ulonglong2(d3 >= 64 ? ~0ull : (1ull << d3) - 1ull,
                                                    d3 > 64 ? (1ull << (d3 - 64)) - 1ull : 0ull);
-            const uint32_t top = k == 31 ? 1u : 2u;  // at k = 31 the offset +1 is the offset -1
-            const uint32_t ux = (uint32_t)p.x >> k, uy = (uint32_t)p.y >> k, uz = (uint32_t)p.z >> k;
-            for (uint32_t dz = 0; dz <= top; ++dz)
-                for (uint32_t dy = 0; dy <= top; ++dy)
-                    for (uint32_t dx = 0; dx <= top; ++dx) {
-                        // the corner of the cell, wrapping modulo 2^32 like the code arithmetic
-                        const ulonglong2 first = code96((ux + dx - 1u) << k, (uy + dy - 1u) << k, (uz + dz - 1u) << k);
-                        const ulonglong2 last = make_ulonglong2(first.x | m96.x, first.y | m96.y);
-                        for (uint32_t j = lower_bound96(a.code, n, i, first); j < n; ++j) {
-                            if (less96(last, a.code[j])) break;
-                            if (j == i || !within(p, a.pos[j], R)) continue;
-                            if (c < a.maxn) a.idx[(size_t)c * a.stride + i] = j;
-                            ++c;
-                        }
-                    }
+            const ulonglong2 first = code96(cx, cy, cz);
+            const ulonglong2 last = make_ulonglong2(first.x | m96.x, first.y | m96.y);
+            s = first_not(a.code, n, i, [&](ulonglong2 x) { return less96(x, first); });
+            if (s < n) len = first_not(a.code, n, s, [&](ulonglong2 x) { return !less96(last, x); }) - s;
+        };
+        uint32_t s, len;
+        range(gl, s, len);
+        for (uint32_t c0 = 0; c0 < 27u; c0 += G) {
+            uint32_t ns, nlen;
+            range(c0 + G + gl, ns, nlen);  // in flight while this round's candidates are tested
+            __syncwarp();
+            w.template take<false>(s, len);
+            s = ns;
+            len = nlen;
         }
-        if (c > a.maxn) {
-            set_flag(a.st, APBF_FLAG_NEIGHBOR_OVERFLOW);
-            atomicMax(&a.st->required_neighbors, c);
+        if (gl == 0u) {
+            const uint32_t kept = min(w.count, a.maxn);
+            s_cnt[w.slot] = kept;
+            if (valid) {
+                if (w.count > a.maxn) {
+                    set_flag(a.st, APBF_FLAG_NEIGHBOR_OVERFLOW);
+                    atomicMax(&a.st->required_neighbors, w.count);
+                }
+                a.count[i] = kept;
+                local += kept;
+            }
         }
-        a.count[i] = c < a.maxn ? c : a.maxn;
-        local += c < a.maxn ? c : a.maxn;
-        if (a.pos_box) a.pos_box[i] = box_push(p, a.radius[i], i, a.bmin, a.bmax, a.rot, a.nboxes);
+        __syncthreads();
+        w.write_rows(s_cnt, base);
+        if (a.pos_box && threadIdx.x < Walk::kParticles && base + threadIdx.x < n) {
+            const uint32_t j = base + threadIdx.x;
+            a.pos_box[j] = box_push_call(a.pos[j], a.radius[j], j, a.bmin, a.bmax, a.rot, a.nboxes);
+        }
+        __syncthreads();  // the rows are the next particles'
     }
-    for (int off = 16; off > 0; off >>= 1) {
-        local += __shfl_down_sync(0xffffffffu, local, off);
-        const long long a2 = __shfl_down_sync(0xffffffffu, rmin, off);
-        const long long c2 = __shfl_down_sync(0xffffffffu, rmax, off);
-        rmin = a2 < rmin ? a2 : rmin;
-        rmax = c2 > rmax ? c2 : rmax;
-    }
-    if ((threadIdx.x & 31) == 0) {
-        if (local) atomicAdd(a.total, local);
-        if (rmax >= 0) {
+    add_pairs(a.total, local);
+    // (a bound that already holds is left alone)
+    if (gl == 0u && rmax >= 0) {
+        if ((unsigned long long)rmin < *(volatile unsigned long long *)&a.st->range_min)
             atomicMin(&a.st->range_min, (unsigned long long)rmin);
+        if ((unsigned long long)rmax > *(volatile unsigned long long *)&a.st->range_max)
             atomicMax(&a.st->range_max, (unsigned long long)rmax);
-        }
     }
 }
 
@@ -230,9 +322,15 @@ apbf_status neighborhood_binary_search(apbf_ctx *ctx, float range_scale, cudaStr
     apbf_status r = reorder_particles(ctx, s);
     if (r != APBF_OK) return r;
     FluidBufs &f = ctx->fl[ctx->fcur];
+    // the table and behind it the levels' range {all ones, 0}
+    BsCell *table = reinterpret_cast<BsCell *>(ctx->bs_table);
+    uint32_t *levels = reinterpret_cast<uint32_t *>(table + ctx->bs_slots);
+    APBF_CUDA(cudaMemsetAsync(table, 0, (size_t)ctx->bs_slots * sizeof(BsCell) + 2 * sizeof(uint32_t), s));
+    APBF_CUDA(cudaMemsetAsync(levels, 0xff, sizeof(uint32_t), s));
     APBF_BEFORE_LAUNCH(ctx, s, "k_sorted_codes");
-    k_sorted_codes<<<g, kBlock, 0, s>>>(f.pos, ctx->d_len, ctx->pos_code, ctx->tr[ctx->tcur], ctx->inv_perm,
-                                        ctx->status, ctx->d_pairs);
+    k_sorted_codes<<<g, kBlock, 0, s>>>(f.pos, f.kernel_width, range_scale, ctx->d_len, ctx->pos_code, table,
+                                        ctx->bs_slots - 1u, levels, ctx->tr[ctx->tcur], ctx->inv_perm, ctx->status,
+                                        ctx->d_pairs);
     APBF_AFTER_LAUNCH(ctx, s, "k_sorted_codes");
     FluidBufs &spare = ctx->fl[ctx->fcur ^ 1];
     BsArgs a;
@@ -253,8 +351,17 @@ apbf_status neighborhood_binary_search(apbf_ctx *ctx, float range_scale, cudaStr
     a.idx = ctx->nb_idx;
     a.total = ctx->d_pairs;
     a.st = ctx->status;
+    a.table = table;
+    a.mask = ctx->bs_slots - 1u;
+    a.levels = levels;
     APBF_BEFORE_LAUNCH(ctx, s, "k_bs_rows");
-    k_bs_rows<<<grid_for(ctx, cap, kBlock, 8), kBlock, 0, s>>>(a);
+    // threads per particle as in the Green search: 8 / 16 / 32 take 50 / 60 / 88 us at 64 019
+    if (cap <= 12288u)
+        k_bs_rows<32><<<grid_for(ctx, cap, RowWalk<32>::kParticles, 64), kBuildThreads, 0, s>>>(a);
+    else if (cap <= 32768u)
+        k_bs_rows<16><<<grid_for(ctx, cap, RowWalk<16>::kParticles, 64), kBuildThreads, 0, s>>>(a);
+    else
+        k_bs_rows<8><<<grid_for(ctx, cap, RowWalk<8>::kParticles, 64), kBuildThreads, 0, s>>>(a);
     APBF_AFTER_LAUNCH(ctx, s, "k_bs_rows");
     if (fuse_box) {  // the box-collided positions are the current ones now
         int4 *t = f.pos;
