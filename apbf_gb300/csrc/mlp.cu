@@ -569,6 +569,7 @@ __global__ void __launch_bounds__(kRowsCta) k_mlp_grad(const float *__restrict__
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         tc_fence_before();
     }
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the step before may still write P, the caller X and T
     load_weights(w, P);
     __syncthreads();
     tc_fence_after();
@@ -731,19 +732,27 @@ __global__ void __launch_bounds__(kRowsCta) k_mlp_grad(const float *__restrict__
     const uint32_t lane_tmem = tmem + ((uint32_t)(warp * 32) << 16);
     if (ok) {
         tc_fence_after();
+        const bool wide = (reinterpret_cast<uintptr_t>(partials) & 15u) == 0u;  // every row of D starts at 16 bytes then
+        const auto store = [&](float *o, const float *v, int count) {
+            if (wide) {
+                for (int i = 0; i < count; i += 4)
+                    *reinterpret_cast<float4 *>(o + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+            } else {
+                for (int i = 0; i < count; ++i) o[i] = v[i];
+            }
+        };
+        static_assert(kP_N % 4 == 0 && kP_W2 % 4 == 0 && kP_W1 % 4 == 0, "16-byte rows");
         if (warp < 2) {  // rows 0..63: dW2[tr][0..63]
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 float v[16];
                 tmem_ld16(lane_tmem + 16u * c, v);
-#pragma unroll
-                for (int i = 0; i < 16; ++i) out[kP_W2 + tr * kH + 16 * c + i] = v[i];
+                store(out + kP_W2 + tr * kH + 16 * c, v, 16);
             }
         } else {  // rows 64..127, columns 64..71: dW1[tr - 64][0..7]
             float v[16];
             tmem_ld16(lane_tmem + 64u, v);
-#pragma unroll
-            for (int f = 0; f < kF; ++f) out[kP_W1 + (tr - kH) * kF + f] = v[f];
+            store(out + kP_W1 + (tr - kH) * kF, v, kF);
         }
     } else {
         // the MMA did not complete in time: wait (bounded) before the TMEM is freed, and
@@ -760,18 +769,36 @@ __global__ void __launch_bounds__(kRowsCta) k_mlp_grad(const float *__restrict__
     }
 }
 
-// Fixed-order sum of the CTA gradients, then Adam on the trained parameters.
-__global__ void k_mlp_adam(float *P, float *m, float *v, const float *__restrict__ partials, int ctas, float lr,
-                           float b1p, float b2p, float *grad_out, float *loss_out, uint32_t nrows) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= kP_N) return;
+// Fixed-order sum of the CTA gradients, then Adam on the trained parameters.  A block takes
+// 32 parameters, its 32 warps every 32nd CTA's gradients of them (whole lines), and the
+// first warp adds the 32 partial sums in order: a thread per parameter took 256 loads one
+// behind the other, 18 of a minibatch step's 33 us.  Parameters that are not trained are not
+// read: no kernel writes their partials.
+constexpr int kAdamParams = 32, kAdamSlices = 32;
+__global__ void __launch_bounds__(kAdamParams *kAdamSlices) k_mlp_adam(float *P, float *m, float *v,
+                                                                       const float *__restrict__ partials, int ctas,
+                                                                       float lr, float b1p, float b2p, float *grad_out,
+                                                                       float *loss_out, uint32_t nrows) {
+    __shared__ float s_sum[kAdamSlices][kAdamParams];
+    const int pl = threadIdx.x % kAdamParams, slice = threadIdx.x / kAdamParams;
+    const int t = blockIdx.x * kAdamParams + pl;
+    const bool trained = t >= kP_W1 && t <= kP_B3;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    float sum = 0.0f;
+    if (trained || t == kP_N - 1) {
+#pragma unroll 8
+        for (int c = slice; c < ctas; c += kAdamSlices) sum += partials[(size_t)c * kP_N + t];
+    }
+    s_sum[slice][pl] = sum;
+    __syncthreads();
+    if (slice != 0 || t >= kP_N) return;
     float gsum = 0.0f;
-    for (int c = 0; c < ctas; ++c) gsum += partials[(size_t)c * kP_N + t];
+#pragma unroll
+    for (int k = 0; k < kAdamSlices; ++k) gsum += s_sum[k][pl];
     if (t == kP_N - 1) {
         if (loss_out) *loss_out = gsum / (float)nrows;
         return;
     }
-    const bool trained = t >= kP_W1 && t <= kP_B3;
     if (grad_out) grad_out[t] = trained ? gsum : 0.0f;
     if (!trained || lr == 0.0f) return;
     const float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
@@ -800,18 +827,30 @@ apbf_status mlp_train_step(float *P, float *m, float *v, float *partials, const 
                            float *loss_out, cudaStream_t s) {
     if (nrows == 0) return APBF_OK;
     const uint32_t ctas = (nrows + kRowsCta - 1) / kRowsCta;
-    APBF_CUDA(cudaMemsetAsync(partials, 0, (size_t)ctas * kP_N * sizeof(float), s));
     static bool attr_set = false;
     if (!attr_set) {
         APBF_CUDA(cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGradSmem));
         attr_set = true;
     }
-    k_mlp_grad<<<ctas, kRowsCta, kGradSmem, s>>>(P, X, T, nrows, over_weight, partials);
-    APBF_CUDA(cudaGetLastError());
+    // each kernel waits itself for the one before it (griddepcontrol.wait), so its blocks
+    // may start while that one drains
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(kRowsCta);
+    cfg.dynamicSmemBytes = kGradSmem;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    APBF_CUDA(cudaLaunchKernelEx(&cfg, k_mlp_grad, (const float *)P, X, T, nrows, over_weight, partials));
     const float b1p = powf(0.9f, (float)(step + 1)), b2p = powf(0.999f, (float)(step + 1));
-    k_mlp_adam<<<(kP_N + 255) / 256, 256, 0, s>>>(P, m, v, partials, (int)ctas, lr, b1p, b2p, grad_out, loss_out,
-                                                   nrows);
-    APBF_CUDA(cudaGetLastError());
+    cfg.gridDim = dim3((kP_N + kAdamParams - 1) / kAdamParams);
+    cfg.blockDim = dim3(kAdamParams * kAdamSlices);
+    cfg.dynamicSmemBytes = 0;
+    APBF_CUDA(cudaLaunchKernelEx(&cfg, k_mlp_adam, P, m, v, (const float *)partials, (int)ctas, lr, b1p, b2p, grad_out,
+                                 loss_out, nrows));
     return APBF_OK;
 }
 
