@@ -28,10 +28,22 @@ namespace {
 // floor(sqrt(x)) exactly: FP32 estimate, then integer correction.
 __device__ __forceinline__ uint32_t isqrt_u64(unsigned long long x) {
     unsigned long long r = (unsigned long long)sqrtf((float)x);
-    while (r > 0 && r * r > x) --r;
-    while ((r + 1) * (r + 1) <= x) ++r;
+    long long e = (long long)(x - r * r);  // small: the estimate is within 2^-23 of the root
+    while (e < 0) {
+        --r;
+        e += (long long)(2 * r + 1);
+    }
+    while (e > (long long)(2 * r)) {
+        e -= (long long)(2 * r + 1);
+        ++r;
+    }
     return (uint32_t)r;
 }
+
+// Rows longer than this are left by their thread to its whole warp: a lane alone waits a
+// memory latency for every four entries of a row that can hold hundreds, and its warp and
+// the kernel's last block with it.
+constexpr uint32_t kLongRow = 64;
 
 __device__ __forceinline__ uint32_t fixed_dist(int4 a, int4 b) {
     long long dx = (long long)b.x - a.x, dy = (long long)b.y - a.y, dz = (long long)b.z - a.z;
@@ -44,22 +56,38 @@ __device__ __forceinline__ uint32_t fixed_dist(int4 a, int4 b) {
 constexpr uint32_t kPropNone = 0u, kPropMerge = 1u, kPropSplit = 2u;
 
 // find_split_and_merge_1 + _2: bd_i = min_j(bd_j + d_ij), d_min_i, nearest_i.
+struct FsmMin {
+    uint32_t bd = 0xffffffffu, md = 0xffffffffu, nn = 0xffffffffu;
+    __device__ __forceinline__ void take(int4 p, int4 q, uint32_t old_bd, uint32_t j) {
+        const uint32_t d = fixed_dist(p, q);
+        const uint32_t cand = old_bd + d;  // uint wrap as in the shader
+        bd = cand < bd ? cand : bd;
+        if (d < md || (d == md && j < nn)) {
+            md = d;
+            nn = j;
+        }
+    }
+};
 __global__ void k_fsm12(const int4 *__restrict__ pos, const uint32_t *__restrict__ old_bd,
                         uint32_t *__restrict__ new_bd, uint32_t *__restrict__ nearest, const uint32_t *count,
                         const uint32_t *idx, uint32_t stride, const uint32_t *d_len) {
     const uint32_t n = d_len[kLenParticles];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int4 p = pos[i];
-        uint32_t bd = 0xffffffffu, md = 0xffffffffu, nn = 0xffffffffu;
-        const uint32_t c = count[i];
+    const uint32_t lane = threadIdx.x & 31u;
+    // (whole warps: the long rows need every lane)
+    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+        const uint32_t i = base + threadIdx.x;
+        const int4 p = i < n ? pos[i] : make_int4(0, 0, 0, 0);
+        const uint32_t c = i < n ? count[i] : 0u;
+        const uint32_t mine = c > kLongRow ? 0u : c;
+        FsmMin m;
         const uint32_t *row = idx + i;
         // batches of four neighbours, software-pipelined: a batch's gathers go out with
         // the row entries of the next (the minima do not depend on the order)
         constexpr uint32_t U = 4;
         uint32_t jj[U];
 #pragma unroll
-        for (uint32_t u = 0; u < U; ++u) jj[u] = u < c ? row[(size_t)u * stride] : i;
-        for (uint32_t k0 = 0; k0 < c; k0 += U) {
+        for (uint32_t u = 0; u < U; ++u) jj[u] = u < mine ? row[(size_t)u * stride] : 0u;
+        for (uint32_t k0 = 0; k0 < mine; k0 += U) {
             int4 q[U];
             uint32_t ob[U], jn[U];
 #pragma unroll
@@ -70,25 +98,36 @@ __global__ void k_fsm12(const int4 *__restrict__ pos, const uint32_t *__restrict
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u) {
                 const uint32_t k = k0 + U + u;
-                jn[u] = k < c ? row[(size_t)k * stride] : i;
+                jn[u] = k < mine ? row[(size_t)k * stride] : 0u;
             }
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u) {
-                if (k0 + u >= c) break;
-                const uint32_t j = jj[u];
-                const uint32_t d = fixed_dist(p, q[u]);
-                const uint32_t cand = ob[u] + d;  // uint wrap as in the shader
-                bd = cand < bd ? cand : bd;
-                if (d < md || (d == md && j < nn)) {
-                    md = d;
-                    nn = j;
-                }
+                if (k0 + u >= mine) break;
+                m.take(p, q[u], ob[u], jj[u]);
             }
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u) jj[u] = jn[u];
         }
-        new_bd[i] = bd;
-        nearest[i] = nn;
+        for (uint32_t left = __ballot_sync(0xffffffffu, c > kLongRow); left; left &= left - 1u) {
+            const int src = __ffs(left) - 1;
+            const uint32_t li = __shfl_sync(0xffffffffu, i, src), lc = __shfl_sync(0xffffffffu, c, src);
+            const int4 lp = pos[li];
+            FsmMin w;
+            for (uint32_t k = lane; k < lc; k += 32u) {
+                const uint32_t j = idx[(size_t)k * stride + li];
+                w.take(lp, pos[j], old_bd[j], j);
+            }
+            const uint32_t bd = __reduce_min_sync(0xffffffffu, w.bd), md = __reduce_min_sync(0xffffffffu, w.md);
+            const uint32_t nn = __reduce_min_sync(0xffffffffu, w.md == md ? w.nn : 0xffffffffu);
+            if ((int)lane == src) {
+                m.bd = bd;
+                m.nn = nn;
+            }
+        }
+        if (i < n) {
+            new_bd[i] = m.bd;
+            nearest[i] = m.nn;
+        }
     }
 }
 
@@ -433,26 +472,42 @@ __global__ void k_kw_init(FluidBufs f, uint32_t *ukw, const uint32_t *d_len, int
     }
 }
 
+// One pair of kernel_width.comp:26-61: j's kernel width grows to what i's influence asks
+// (a maximum only grows, so an atomic whose value a plain read already meets or exceeds would
+// change nothing and is left out); whether the pair stays in i's row.
+__device__ __forceinline__ bool spread_pair(int4 p, int4 q, uint32_t j, uint32_t cur, float ok, float cut, uint32_t *ukw) {
+    const float dx = (float)wadd(q.x, -p.x) / 262144.0f, dy = (float)wadd(q.y, -p.y) / 262144.0f,
+                dz = (float)wadd(q.z, -p.z) / 262144.0f;
+    const float dist = sqrtf((dx * dx + dy * dy) + dz * dz);
+    const float infl = fmaxf(0.0f, 1.0f - fmaxf(0.0f, (dist - ok) / (ok * 0.5f)));
+    const uint32_t v = f2u((ok * infl) * 262144.0f);
+    if (v > cur) atomicMax(&ukw[j], v);
+    return dist <= cut;
+}
+
 // kernel_width.comp:26-61: spread (atomicMax) and prune row i in place, order kept.
 __global__ void k_kw_spread(FluidBufs f, uint32_t *ukw, uint32_t *count, uint32_t *idx, uint32_t stride,
                             const uint32_t *d_len, int use_target) {
     const uint32_t n = d_len[kLenParticles];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int4 p = f.pos[i];
-        const float tr = use_target ? f.target_radius[i] : 0.0f;
-        const float ok = fmaxf(f.radius[i], tr) * 4.0f;
-        const float cut = fmaxf(ok, f.kernel_width[i]);
-        const uint32_t c = count[i];
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {  // whole warps
+        const uint32_t i = base + threadIdx.x;
+        const bool valid = i < n;
+        const int4 p = valid ? f.pos[i] : make_int4(0, 0, 0, 0);
+        const float tr = valid && use_target ? f.target_radius[i] : 0.0f;
+        const float ok = valid ? fmaxf(f.radius[i], tr) * 4.0f : 0.0f;
+        const float cut = valid ? fmaxf(ok, f.kernel_width[i]) : 0.0f;
+        const uint32_t c = valid ? count[i] : 0u;
+        const uint32_t mine = c > kLongRow ? 0u : c;
         uint32_t w = 0;
         // batches of four neighbours, software-pipelined (the pruned row is written
-        // behind the entries read ahead); a maximum only grows, so an atomic whose value
-        // a plain read already meets or exceeds would change nothing and is left out
+        // behind the entries read ahead)
         constexpr uint32_t U = 4;
         uint32_t *row = idx + i;
         uint32_t jj[U];
 #pragma unroll
-        for (uint32_t u = 0; u < U; ++u) jj[u] = u < c ? row[(size_t)u * stride] : i;
-        for (uint32_t k0 = 0; k0 < c; k0 += U) {
+        for (uint32_t u = 0; u < U; ++u) jj[u] = u < mine ? row[(size_t)u * stride] : 0u;
+        for (uint32_t k0 = 0; k0 < mine; k0 += U) {
             int4 q[U];
             uint32_t cur[U], jn[U];
 #pragma unroll
@@ -463,24 +518,34 @@ __global__ void k_kw_spread(FluidBufs f, uint32_t *ukw, uint32_t *count, uint32_
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u) {
                 const uint32_t k = k0 + U + u;
-                jn[u] = k < c ? row[(size_t)k * stride] : i;
+                jn[u] = k < mine ? row[(size_t)k * stride] : 0u;
             }
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u) {
-                if (k0 + u >= c) break;
-                const uint32_t j = jj[u];
-                const float dx = (float)wadd(q[u].x, -p.x) / 262144.0f, dy = (float)wadd(q[u].y, -p.y) / 262144.0f,
-                            dz = (float)wadd(q[u].z, -p.z) / 262144.0f;
-                const float dist = sqrtf((dx * dx + dy * dy) + dz * dz);
-                const float infl = fmaxf(0.0f, 1.0f - fmaxf(0.0f, (dist - ok) / (ok * 0.5f)));
-                const uint32_t v = f2u((ok * infl) * 262144.0f);
-                if (v > cur[u]) atomicMax(&ukw[j], v);
-                if (dist <= cut) row[(size_t)(w++) * stride] = j;
+                if (k0 + u >= mine) break;
+                if (spread_pair(p, q[u], jj[u], cur[u], ok, cut, ukw)) row[(size_t)(w++) * stride] = jj[u];
             }
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u) jj[u] = jn[u];
         }
-        count[i] = w;
+        for (uint32_t left = __ballot_sync(0xffffffffu, c > kLongRow); left; left &= left - 1u) {
+            const int src = __ffs(left) - 1;
+            const uint32_t li = __shfl_sync(0xffffffffu, i, src), lc = __shfl_sync(0xffffffffu, c, src);
+            const float lok = __shfl_sync(0xffffffffu, ok, src), lcut = __shfl_sync(0xffffffffu, cut, src);
+            const int4 lp = f.pos[li];
+            uint32_t *lrow = idx + li;
+            uint32_t lw = 0, next = lane < lc ? lrow[(size_t)lane * stride] : 0u;
+            for (uint32_t k0 = 0; k0 < lc; k0 += 32u) {
+                const uint32_t j = next, k = k0 + lane;
+                next = k + 32u < lc ? lrow[(size_t)(k + 32u) * stride] : 0u;  // read before anything is written here
+                const bool stays = k < lc && spread_pair(lp, f.pos[j], j, *(volatile const uint32_t *)&ukw[j], lok, lcut, ukw);
+                const uint32_t bal = __ballot_sync(0xffffffffu, stays);
+                if (stays) lrow[(size_t)(lw + __popc(bal & ((1u << lane) - 1u))) * stride] = j;
+                lw += __popc(bal);
+            }
+            if ((int)lane == src) w = lw;
+        }
+        if (valid) count[i] = w;
     }
 }
 
