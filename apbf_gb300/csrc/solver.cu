@@ -963,7 +963,11 @@ __global__ void __launch_bounds__(256, 4) k_delta(PassB a) {
 // Entries from kTileDepth on and tiles whose halo exceeds kTileHalo are read from the list's
 // own rows.
 
-__device__ __forceinline__ uint32_t tile_hash(uint32_t j, uint32_t mask) { return (j * 2654435761u >> 16) & mask; }
+// Eight neighbouring particles, whose records share a line, keep together in the table and
+// so in the halo, which takes its order; the groups are spread.
+__device__ __forceinline__ uint32_t tile_hash(uint32_t j, uint32_t mask) {
+    return (((j >> 3) * 2654435761u >> 16) << 3 | (j & 7u)) & mask;
+}
 
 struct TileRowsArgs {
     const uint32_t *count, *idx;
@@ -979,6 +983,7 @@ template <int T>
 __global__ void __launch_bounds__(256) k_tile_rows(TileRowsArgs a) {
     constexpr uint32_t S = 256 / T;    // threads per particle
     constexpr uint32_t kSlots = 2048;  // hash table, at most 32 % full
+    constexpr uint32_t kProbes = 64;   // slots looked at before a tile counts as overflowing
     constexpr uint32_t kKept = 8;      // row quads whose table slots are kept from the first walk
     static_assert(kTileHalo * 2 <= kSlots, "the hash table holds the halo with room to probe");
     __shared__ uint32_t s_key[kSlots];
@@ -986,7 +991,8 @@ __global__ void __launch_bounds__(256) k_tile_rows(TileRowsArgs a) {
     __shared__ uint2 s_kept[kKept * T];  // four 16-bit codes: 0x8000 | table slot, or the offset of a tile record
     __shared__ uint32_t s_bin[64];
     __shared__ uint16_t s_rank[T];
-    __shared__ uint32_t s_halo, s_rmax;
+    __shared__ uint32_t s_scan[8];
+    __shared__ uint32_t s_full, s_rmax;
     if (a.reverse && (a.st->range_min == a.st->range_max || a.st->union_rows != 0u)) return;
     const uint32_t n = a.d_len[kLenParticles];
     const uint32_t o = threadIdx.x % T, sub = threadIdx.x / T;  // a warp reads consecutive particles' entries
@@ -996,7 +1002,7 @@ __global__ void __launch_bounds__(256) k_tile_rows(TileRowsArgs a) {
         const float r = i < n ? fabsf(a.radius[i]) : 0.0f;
         for (uint32_t k = threadIdx.x; k < kSlots; k += 256) s_key[k] = 0xffffffffu;
         if (threadIdx.x < 64) s_bin[threadIdx.x] = 0u;
-        if (threadIdx.x == 0) s_halo = s_rmax = 0u;
+        if (threadIdx.x == 0) s_full = s_rmax = 0u;
         __syncthreads();
         const uint32_t depth = min(cnt, (uint32_t)kTileDepth);
         // falling row length: a counting sort (the order among equal lengths is free)
@@ -1005,27 +1011,20 @@ __global__ void __launch_bounds__(256) k_tile_rows(TileRowsArgs a) {
         const uint32_t rm = __reduce_max_sync(0xffffffffu, __float_as_uint(r));
         if ((threadIdx.x & 31u) == 0u) atomicMax(&s_rmax, rm);
         // the code of entry j: the offset of its record when it lies in the tile, else
-        // its slot in the table of the halo, entered when it is not there yet
+        // its slot in the table of the halo, entered when it is not there yet.  Only the keys
+        // are entered here; numbering them here as well (a counter that every insert waits
+        // for) made this walk four fifths of the kernel.
         const auto enter = [&](uint32_t j) -> uint32_t {
             if (j - base < T) return (j - base) * 16u;
             uint32_t h = tile_hash(j, kSlots - 1);
-            for (;;) {
+            for (uint32_t probe = 0; probe < kProbes; ++probe) {
                 uint32_t was = *(volatile uint32_t *)&s_key[h];
-                if (was == 0xffffffffu) {
-                    if (*(volatile uint32_t *)&s_halo >= kTileHalo) return 0u;  // overflow: bounds the probing too
-                    was = atomicCAS(&s_key[h], 0xffffffffu, j);
-                    if (was == 0xffffffffu) {
-                        const uint32_t slot = atomicAdd(&s_halo, 1u);
-                        if (slot < kTileHalo) {
-                            s_val[h] = (uint16_t)((2 * T + slot) * 16u);
-                            a.plan.halo[(size_t)tile * kTileHalo + slot] = j;
-                        }
-                        return 0x8000u | h;
-                    }
-                }
-                if (was == j) return 0x8000u | h;
+                if (was == 0xffffffffu) was = atomicCAS(&s_key[h], 0xffffffffu, j);
+                if (was == j || was == 0xffffffffu) return 0x8000u | h;
                 h = (h + 1u) & (kSlots - 1);
             }
+            s_full = 1u;  // far more outside particles than the halo holds
+            return 0u;
         };
         const auto load4 = [&](uint32_t q, uint32_t (&j)[4]) {
 #pragma unroll
@@ -1056,10 +1055,40 @@ __global__ void __launch_bounds__(256) k_tile_rows(TileRowsArgs a) {
             s_bin[2 * threadIdx.x] = v - x0 - x1;
             s_bin[2 * threadIdx.x + 1] = v - x1;
         }
-        const uint32_t halo = s_halo;
+        // the halo in the table's order: a thread numbers the keys of eight slots
+        constexpr uint32_t kPer = kSlots / 256;
+        uint32_t key[kPer], used = 0;
+#pragma unroll
+        for (uint32_t u = 0; u < kPer; ++u) {
+            key[u] = s_key[threadIdx.x * kPer + u];
+            used += key[u] != 0xffffffffu ? 1u : 0u;
+        }
+        uint32_t first = used;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, first, off);
+            if ((int)(threadIdx.x & 31u) >= off) first += y;
+        }
+        if ((threadIdx.x & 31u) == 31u) s_scan[threadIdx.x / 32u] = first;
         __syncthreads();
-        // (a tile that fills its halo exactly counts as overflowing: the inserts stop there)
-        const bool over = halo >= kTileHalo;
+        uint32_t halo = 0;
+        first -= used;
+#pragma unroll
+        for (uint32_t w = 0; w < 8; ++w) {
+            const uint32_t c = s_scan[w];
+            if (w < threadIdx.x / 32u) first += c;
+            halo += c;
+        }
+        const bool over = halo > kTileHalo || s_full != 0u;
+        if (!over) {
+#pragma unroll
+            for (uint32_t u = 0; u < kPer; ++u) {
+                if (key[u] == 0xffffffffu) continue;
+                s_val[threadIdx.x * kPer + u] = (uint16_t)((2 * T + first) * 16u);
+                a.plan.halo[(size_t)tile * kTileHalo + first] = key[u];
+                ++first;
+            }
+        }
         if (sub == 0) {
             const uint32_t k = atomicAdd(&s_bin[bin], 1u);
             s_rank[o] = (uint16_t)k;
