@@ -104,6 +104,7 @@ struct PassSync {
 // The neighbour rows of a substep rewritten for the tiled passes (solver.cu).
 constexpr int kTileHalo = 640;  // halo entries of a tile; one that fills it reads the list's own rows
 constexpr int kTileDepth = 64;  // row entries rewritten as offsets; the rest of a longer row goes to the pool
+constexpr uint32_t kTileSmallest = 64;  // particles of the smaller tile shape
 constexpr uint32_t kHaloOver = 0xffffffffu, kNoParticle = 0xffffffffu;
 struct TilePlan {
     uint32_t *halo;        // [tile * kTileHalo + slot]: particles outside the tile

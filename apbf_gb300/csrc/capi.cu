@@ -312,8 +312,8 @@ apbf_status apbf_create(const apbf_config *cfg, apbf_ctx **out) {
     for (int k = 0; k < 2; ++k) {
         TilePlan &t = ctx->tile_plan[k];
         const size_t whole = ((size_t)cap + 255u) / 256u * 256u;  // whole tiles of every shape
-        A(t.halo, whole / 32u * kTileHalo);
-        A(t.tile, whole / 32u);
+        A(t.halo, whole / kTileSmallest * kTileHalo);
+        A(t.tile, whole / kTileSmallest);
         A(t.lane, whole);
         A(t.rows, whole * (kTileDepth / 4));
         t.pool_size = cfg->max_neighbors > (uint32_t)kTileDepth ? 2u * cap : 0u;
