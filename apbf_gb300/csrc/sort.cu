@@ -532,7 +532,7 @@ apbf_status sort_pairs_device(apbf_ctx *ctx, const uint32_t *keys_in, const uint
         APBF_CUDA(cudaMemcpyAsync(vals_out, vals_in, (size_t)max_count * 4, cudaMemcpyDeviceToDevice, s));
         return APBF_OK;
     }
-    if (ctx->tuning.sort_digit_bits == 0u && max_count <= SmallSort16k::kKeys) {
+    if (dbits == 8u && max_count <= SmallSort16k::kKeys) {
         APBF_BEFORE_LAUNCH(ctx, s, "k_sort_small");
         if (max_count <= SmallSort4k::kKeys)
             k_sort_small<256, 16><<<1, 256, sizeof(SmallSort4k), s>>>(keys_in, vals_in, keys_out, vals_out, d_count,
@@ -545,7 +545,7 @@ apbf_status sort_pairs_device(apbf_ctx *ctx, const uint32_t *keys_in, const uint
     }
     // scratch: hist passes x nb <= 4 x 256 words, status passes x tiles x nb <= 4 x tiles x 256
     // one block of memory: counters, histograms, status words or group counts (one clear)
-    const bool wait_free = ctx->tuning.sort_digit_bits == 0u && max_count > kWaitFree;
+    const bool wait_free = dbits == 8u && max_count > kWaitFree;
     const uint32_t groups = (tiles + kSortGroup - 1) / kSortGroup;
     APBF_CUDA(cudaMemsetAsync(ctx->sort_counters, 0,
                               (kSortScratchHead + (size_t)passes * (wait_free ? groups * 256u : tiles * nb)) *
