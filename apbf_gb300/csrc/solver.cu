@@ -8,7 +8,7 @@
 //    (lambda, boundariness, self shift) + the boundariness filter of
 //    incompressibility_3.comp:41-46,60.  Writes lambda, the self shift, the
 //    per-particle Gauss constants and the density-error partials (64-bit
-//    fixed-point integers, turned into the FP64 mean by the last block).
+//    fixed-point integers, turned into the FP64 mean by the position update).
 //  k_delta (particle j, over the particles whose rows contain j):
 //    incompressibility_3.comp:62-66 as a gather: x_j += sum_i int(gradW_ij * lambda_i * 2^18)
 //    plus the self shift, into the other position buffer.
@@ -1520,7 +1520,7 @@ __device__ __noinline__ int4 box_push_from(int4 ip, float r, uint32_t id, const 
 }
 
 // A tile's position update.  fwd: the plan of the own rows, rev: that of the
-// transposed rows.  86 us at a million particles against 125 us for the direct kernel, 30
+// transposed rows.  84 us at a million particles against 125 us for the direct kernel, 30
 // against 37 us at 250 000.  Of its instructions the deferred filter's row tests took a
 // quarter and the boxes a fifth; both now reject by cheap bounds first.
 template <int T, int L>
@@ -2530,7 +2530,7 @@ int solve_batch_blocks(int device, int num_sms) {
 apbf_status reduce_fp64(apbf_ctx *ctx, double out[4], cudaStream_t s) {
     FluidBufs &f = ctx->fl[ctx->fcur];
     const int g = ctx->red_blocks;
-    // red_out[2..3] hold the error of the last density pass (its last block wrote them)
+    // red_out[2..3] hold the error of the last density pass (the position update behind it wrote them)
     APBF_BEFORE_LAUNCH(ctx, s, "k_mass_volume");
     k_mass_volume<<<g, kBlock, 0, s>>>(f.inv_mass, f.radius, ctx->d_len, ctx->red_partials + 4 * g);
     APBF_AFTER_LAUNCH(ctx, s, "k_mass_volume");
