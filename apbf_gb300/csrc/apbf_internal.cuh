@@ -223,6 +223,7 @@ struct apbf_ctx {
     uint32_t *cells = nullptr;             // per cell: first particle; then per cell: end
     ulonglong2 *pos_code = nullptr;        // per particle: 96-bit position code {bits 0-63, bits 64-95}
     ulonglong2 *bs_table = nullptr;        // cells of the binary-search rows (neighborhood_bs.cu)
+    uint32_t *bs_counts = nullptr;         // 12 x 256: the particles' code digits
     uint32_t bs_slots = 0;                 // its slots, a power of two above the capacity
     int4 *srec = nullptr;                  // per particle: search record (position xyz, fixed-point radius)
     int search_method = APBF_NEIGHBORHOOD_GREEN;  // the substep's neighbour search
@@ -437,7 +438,8 @@ apbf_status reorder_particles(apbf_ctx *ctx, cudaStream_t s, bool search = false
 apbf_status glue_remap(apbf_ctx *ctx, cudaStream_t s);      // constraints.cu: glue ids follow a reorder
 apbf_status sort_pairs_device(apbf_ctx *ctx, const uint32_t *keys_in, const uint32_t *vals_in, const uint32_t *d_count,
                               uint32_t max_count, uint32_t key_bits, uint32_t *keys_out, uint32_t *vals_out,
-                              cudaStream_t s);
+                              cudaStream_t s, const uint32_t *counts = nullptr);
+bool sort_takes_counts(const apbf_ctx *ctx, uint32_t max_count);
 apbf_status sort_prepare_device();  // kernel attributes on the current device
 apbf_status prefix_sum_device(apbf_ctx *ctx, uint32_t *d_values, const uint32_t *d_count, uint32_t max_count,
                               cudaStream_t s);

@@ -277,6 +277,7 @@ apbf_status apbf_create(const apbf_config *cfg, apbf_ctx **out) {
     A(ctx->pos_code, cap);
     for (ctx->bs_slots = 256u; ctx->bs_slots < 2u * cap;) ctx->bs_slots *= 2u;
     A(ctx->bs_table, (size_t)ctx->bs_slots + 1u);
+    A(ctx->bs_counts, 12 * 256);
     A(ctx->srec, cap);
     ctx->n_cells_log2_alloc = cfg->max_log2res;
     A(ctx->lambda, cap);

@@ -72,6 +72,30 @@ __global__ void k_code_word(const int4 *__restrict__ pos, const uint32_t *d_len,
     }
 }
 
+// Word 0 of every particle's code, and the counts of all twelve 8-bit digits of the codes
+// (counts: 12 x 256, cleared): how often a digit occurs does not depend on the order, so the
+// three sorts need no pass over their keys for it (three launches of 4 us each).
+__global__ void __launch_bounds__(512) k_code_counts(const int4 *__restrict__ pos, const uint32_t *d_len,
+                                                     uint32_t *__restrict__ keys, uint32_t *__restrict__ vals,
+                                                     uint32_t *__restrict__ counts) {
+    __shared__ uint32_t sh[12 * 256];
+    for (uint32_t q = threadIdx.x; q < 12u * 256u; q += blockDim.x) sh[q] = 0u;
+    __syncthreads();
+    const uint32_t n = d_len[kLenParticles];
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const int4 p = pos[k];
+        const ulonglong2 c = code96((uint32_t)p.x, (uint32_t)p.y, (uint32_t)p.z);
+        keys[k] = code_word(c, 0);
+        vals[k] = k;
+#pragma unroll
+        for (int d = 0; d < 12; ++d)
+            atomicAdd(&sh[d * 256 + (int)((code_word(c, d / 4) >> (8 * (d % 4))) & 255u)], 1u);
+    }
+    __syncthreads();
+    for (uint32_t q = threadIdx.x; q < 12u * 256u; q += blockDim.x)
+        if (sh[q]) atomicAdd(&counts[q], sh[q]);
+}
+
 // The cells of one level as a hash table: 63-bit cell number + 1 (0: empty), first particle
 // and end of the cell's run of the sorted list.
 struct __align__(16) BsCell {
@@ -309,14 +333,24 @@ apbf_status neighborhood_binary_search(apbf_ctx *ctx, float range_scale, cudaStr
     const uint32_t cap = ctx->cfg.particle_capacity;
     const int g = grid_for(ctx, cap);
     // three stable passes, least significant word first
+    const bool counted = sort_takes_counts(ctx, cap);
+    if (counted) APBF_CUDA(cudaMemsetAsync(ctx->bs_counts, 0, 12 * 256 * sizeof(uint32_t), s));
     for (uint32_t w = 0; w < 3; ++w) {
         const FluidBufs &cur = ctx->fl[ctx->fcur];
-        APBF_BEFORE_LAUNCH(ctx, s, "k_code_word");
-        k_code_word<<<g, kBlock, 0, s>>>(cur.pos, ctx->d_len, w, w ? ctx->perm : nullptr, ctx->keys[0],
-                                         ctx->vals[0]);
-        APBF_AFTER_LAUNCH(ctx, s, "k_code_word");
+        if (counted && w == 0) {
+            APBF_BEFORE_LAUNCH(ctx, s, "k_code_counts");
+            k_code_counts<<<grid_for(ctx, cap, 512, 2), 512, 0, s>>>(cur.pos, ctx->d_len, ctx->keys[0], ctx->vals[0],
+                                                                     ctx->bs_counts);
+            APBF_AFTER_LAUNCH(ctx, s, "k_code_counts");
+        } else {
+            APBF_BEFORE_LAUNCH(ctx, s, "k_code_word");
+            k_code_word<<<g, kBlock, 0, s>>>(cur.pos, ctx->d_len, w, w ? ctx->perm : nullptr, ctx->keys[0],
+                                             ctx->vals[0]);
+            APBF_AFTER_LAUNCH(ctx, s, "k_code_word");
+        }
         apbf_status r = sort_pairs_device(ctx, ctx->keys[0], ctx->vals[0], ctx->d_len + kLenParticles, cap, 32u,
-                                          ctx->sorted_keys, ctx->perm, s);
+                                          ctx->sorted_keys, ctx->perm, s,
+                                          counted ? ctx->bs_counts + w * 4 * 256 : nullptr);
         if (r != APBF_OK) return r;
     }
     apbf_status r = reorder_particles(ctx, s);

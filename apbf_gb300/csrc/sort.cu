@@ -133,7 +133,8 @@ __device__ __forceinline__ void write_tile(const uint32_t (&keys)[kSortItems], c
 // the scatter, so the tiles are small (2 048 keys), the look-back reads eight earlier tiles
 // at a time (4 096 keys or 16 and 32 tiles at a time were slower), and the keys go through
 // shared memory so that a digit's run leaves as whole lines.  Nine to seven microseconds a
-// pass from 30 000 to 260 000 pairs.
+// pass from 30 000 to 260 000 pairs.  A digit that all keys share (the histogram has them in
+// one bin) moves none: the tile is copied, without ranks and look-back.
 constexpr int kLookBack = 8;
 template <int BITS>
 __global__ void __launch_bounds__(kSortThreads) k_onesweep(const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin,
@@ -156,7 +157,7 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const uint32_t *__res
     const uint32_t hist_t = owner ? hist[t] : 0u;
     const uint32_t n = min(*d_count, max_count);
     const uint32_t ntiles = (n + kSortTile - 1) / kSortTile;
-    __syncthreads();
+    const bool shared_digit = __syncthreads_or(owner && hist_t == n);
     const uint32_t tile = s_tile;
     if (tile >= ntiles) return;
     const uint32_t first = tile * kSortTile, here = min(n - first, (uint32_t)kSortTile);
@@ -168,8 +169,13 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const uint32_t *__res
         const bool valid = idx < here;
         keys[k] = valid ? kin[first + idx] : 0u;
         vals[k] = valid ? vin[first + idx] : 0u;
+        if (shared_digit && valid) {
+            kout[first + idx] = keys[k];
+            vout[first + idx] = vals[k];
+        }
         digit[k] = valid ? ((keys[k] & key_mask) >> shift) & (NB - 1u) : NB + (uint32_t)l;
     }
+    if (shared_digit) return;
     rank_digits<NB>(digit, rank, s_cnt[w]);
     __syncthreads();
     // thread t owns digit t: warp exclusive offsets and the tile total, published at once
@@ -509,11 +515,17 @@ static apbf_status launch_hist(apbf_ctx *ctx, const uint32_t *keys_in, const uin
     return APBF_OK;
 }
 
+bool sort_takes_counts(const apbf_ctx *ctx, uint32_t max_count) {
+    const uint32_t d = ctx->tuning.sort_digit_bits;
+    return d != 6u && d != 7u && max_count > SmallSort16k::kKeys && max_count <= kWaitFree;
+}
+
 // Stable sort by the low key_bits bits of the keys (rounded up to whole 4-bit
-// digits exactly as the reference's pass loop, algorithms.cpp:73).
+// digits exactly as the reference's pass loop, algorithms.cpp:73).  counts (may be null;
+// only where sort_takes_counts): the keys' 8-bit digits already counted, passes x 256.
 apbf_status sort_pairs_device(apbf_ctx *ctx, const uint32_t *keys_in, const uint32_t *vals_in, const uint32_t *d_count,
                               uint32_t max_count, uint32_t key_bits, uint32_t *keys_out, uint32_t *vals_out,
-                              cudaStream_t s) {
+                              cudaStream_t s, const uint32_t *counts) {
     if (max_count == 0) return APBF_OK;
     if (max_count >= (1u << 30)) return APBF_ERR_INVALID_ARG;
     uint32_t nib = (key_bits + 3u) / 4u;  // 4-bit subkeys the reference would sort
@@ -550,7 +562,7 @@ apbf_status sort_pairs_device(apbf_ctx *ctx, const uint32_t *keys_in, const uint
     APBF_CUDA(cudaMemsetAsync(ctx->sort_counters, 0,
                               (kSortScratchHead + (size_t)passes * (wait_free ? groups * 256u : tiles * nb)) *
                                   sizeof(uint32_t), s));
-    if (!wait_free) {
+    if (!wait_free && !counts) {
         const apbf_status r = launch_hist(ctx, keys_in, d_count, max_count, key_mask, passes, (int)dbits, s);
         if (r != APBF_OK) return r;
     }
@@ -584,7 +596,8 @@ apbf_status sort_pairs_device(apbf_ctx *ctx, const uint32_t *keys_in, const uint
             continue;
         }
         APBF_BEFORE_LAUNCH(ctx, s, "k_onesweep");
-        uint32_t *hp = ctx->sort_hist + p * nb, *tp = ctx->sort_status + (size_t)p * tiles * nb;
+        const uint32_t *hp = (counts ? counts : ctx->sort_hist) + p * nb;
+        uint32_t *tp = ctx->sort_status + (size_t)p * tiles * nb;
         if (dbits == 6u)
             k_onesweep<6><<<tiles, kSortThreads, 0, s>>>(src_k, src_v, dk, dv, d_count, max_count, key_mask, sh, hp,
                                                 ctx->sort_counters + p, tp, ctx->status);

@@ -32,3 +32,28 @@ def test_sort_forms(n, bits, in_place):
     assert np.array_equal(ok[:m].cpu().numpy().view(np.uint32), k[:m][order])
     assert torch.equal(ok[m:], tail[0]) and torch.equal(ov[m:], tail[1])  # nothing past the count
     ctx.close()
+
+
+@pytest.mark.parametrize("n", [1, 16_384, 16_385, 20_481, 1 << 18, (1 << 18) + 1])
+@pytest.mark.parametrize("spread", [0x00000000, 0x000000ff, 0x00ff0000, 0xff0000ff, 0x80000000, 0x00ffff00])
+def test_sort_of_shared_digits(n, spread):
+    """Keys that differ in some of their digits only; the others are the same in all keys."""
+    from apbf_gb300.api import Context, algorithms
+
+    rng = np.random.default_rng(n)
+    k = (rng.integers(0, 1 << 32, size=n, dtype=np.uint64).astype(np.uint32) & np.uint32(spread)) | np.uint32(
+        0x5a3c96e1 & ~spread)
+    ctx = Context(particle_capacity=n, max_neighbors=8, max_log2res=3)
+    keys = torch.from_numpy(k.view(np.int32)).cuda()
+    vals = torch.arange(n, dtype=torch.int32, device="cuda")
+    m = n - n // 9
+    cnt = torch.tensor([m], dtype=torch.int32, device="cuda")
+    ok, ov = torch.full_like(keys, -1), torch.full_like(vals, -1)
+    algorithms.sort(ctx, keys, vals, cnt, n, ok, ov, (1 << 32) - 1)
+    torch.cuda.synchronize()
+    ctx.check_status()
+    order = np.argsort(k[:m], kind="stable")
+    assert np.array_equal(ov[:m].cpu().numpy(), order)
+    assert np.array_equal(ok[:m].cpu().numpy().view(np.uint32), k[:m][order])
+    assert bool((ok[m:] == -1).all()) and bool((ov[m:] == -1).all())
+    ctx.close()
