@@ -547,9 +547,9 @@ static_assert(kRowsCta == 128, "the weight-gradient GEMM takes K = 128 rows per 
 // w = over_weight where e < 0 (a lambda more negative than the target: a larger
 // push than the plain solve made), 1 elsewhere -- an expectile regression that,
 // for over_weight > 1, keeps the prediction below the target where it is uncertain.
-__global__ void __launch_bounds__(kRowsCta) k_mlp_grad(const float *__restrict__ P, const float *__restrict__ X,
-                                                        const float *__restrict__ T, uint32_t nrows,
-                                                        float over_weight, float *__restrict__ partials) {
+// (No __restrict__: what the kernel before writes is read behind the wait.)
+__global__ void __launch_bounds__(kRowsCta) k_mlp_grad(const float *P, const float *X, const float *T, uint32_t nrows,
+                                                        float over_weight, float *partials) {
     extern __shared__ __align__(1024) unsigned char smem[];
     SmemW &w = *reinterpret_cast<SmemW *>(smem);
     unsigned char *ga = smem + kGradOffA;  // A of the weight-gradient GEMM (M 128 x K 128)
@@ -776,7 +776,7 @@ __global__ void __launch_bounds__(kRowsCta) k_mlp_grad(const float *__restrict__
 // read: no kernel writes their partials.
 constexpr int kAdamParams = 32, kAdamSlices = 32;
 __global__ void __launch_bounds__(kAdamParams *kAdamSlices) k_mlp_adam(float *P, float *m, float *v,
-                                                                       const float *__restrict__ partials, int ctas,
+                                                                       const float *partials, int ctas,
                                                                        float lr, float b1p, float b2p, float *grad_out,
                                                                        float *loss_out, uint32_t nrows) {
     __shared__ float s_sum[kAdamSlices][kAdamParams];
