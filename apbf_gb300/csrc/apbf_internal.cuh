@@ -404,6 +404,26 @@ inline int grid_for(const apbf_ctx *ctx, uint32_t n, int block = kBlock, int per
     return (int)(need < cap ? need : cap);
 }
 
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Launches a kernel that waits itself (griddepcontrol.wait) for the one before it:
+// behind lets its blocks start as that one's last blocks run.
+template <typename... P, typename... V>
+cudaError_t launch_behind(bool behind, void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s,
+                          V... v) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = behind ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, v...);
+}
+
 // target = m 2^-(s + 24) with m < 2^24, for error_meets_target.  s is clamped to 63
 // (then n m < 2^55 gives the limit 0) and to -8 (a target of 256 and more: every term
 // saturates at 128, so with the largest m any sum meets it).

@@ -1248,8 +1248,6 @@ struct WarpRow {
     }
 };
 
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_dependency_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // A tile's density pass: T particles, L threads each.  At a million particles in a
 // waterfall (13.4 M pairs) 62 us against 92 us for the direct kernel, 26 against 35 us at
@@ -2300,24 +2298,6 @@ apbf_status tile_rows(apbf_ctx *ctx, cudaStream_t s, bool transposed) {
         }
     });
     return r;
-}
-
-// Launches a kernel that waits itself (griddepcontrol.wait) for the one before it:
-// behind lets its blocks start as that one's last blocks run.
-template <typename... P, typename... V>
-static cudaError_t launch_behind(bool behind, void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s,
-                                 V... v) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = behind ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, v...);
 }
 
 // One Jacobi pass over the tiles of the substep's rows.
