@@ -454,7 +454,8 @@ inline int32_t f2i_host(float x) {
 // ---- host-side stage launchers (defined in the .cu files) ----
 apbf_status emit(apbf_ctx *ctx, float dt, cudaStream_t s);  // glue.cu
 // neighborhood.cu: gather by ctx->perm; with `search` also the search records for range scale `scale`
-apbf_status reorder_particles(apbf_ctx *ctx, cudaStream_t s, bool search = false, float scale = 0.0f);
+apbf_status reorder_particles(apbf_ctx *ctx, cudaStream_t s, bool search = false, float scale = 0.0f,
+                              bool behind = false);
 apbf_status glue_remap(apbf_ctx *ctx, cudaStream_t s);      // constraints.cu: glue ids follow a reorder
 apbf_status sort_pairs_device(apbf_ctx *ctx, const uint32_t *keys_in, const uint32_t *vals_in, const uint32_t *d_count,
                               uint32_t max_count, uint32_t key_bits, uint32_t *keys_out, uint32_t *vals_out,

@@ -59,9 +59,10 @@ __global__ void k_position_keys(const int4 *__restrict__ pos, const uint32_t *d_
 // fixed-point search radius R = range_fixed(kw, scale) in w, -1 for a NaN or
 // negative width) and reduces the radii's range into the status block, so that the
 // row build knows before it starts whether every radius is equal.
-__global__ void k_reorder(FluidBufs src, FluidBufs dst, const uint32_t *__restrict__ perm,
-                          uint32_t *__restrict__ inv_perm, const uint32_t *d_len, int4 *__restrict__ srec,
-                          float scale, Status *st) {
+__global__ void k_reorder(FluidBufs src, FluidBufs dst, const uint32_t *perm, uint32_t *inv_perm,
+                          const uint32_t *d_len, int4 *srec, float scale, Status *st) {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     uint32_t n = d_len[kLenParticles];
     long long rmin = 0x7fffffffffffffffll, rmax = -1;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
@@ -108,9 +109,10 @@ __global__ void k_reorder(FluidBufs src, FluidBufs dst, const uint32_t *__restri
 
 // find_value_ranges.comp:15-31 (cell arrays zeroed beforehand).
 // The transfer list follows the reorder here as well.
-__global__ void k_cell_ranges(const uint32_t *__restrict__ skeys, const uint32_t *d_len, uint32_t *__restrict__ start,
-                              uint32_t *__restrict__ end, TransferBufs tr, const uint32_t *__restrict__ inv_perm,
-                              Status *st) {
+__global__ void k_cell_ranges(const uint32_t *skeys, const uint32_t *d_len, uint32_t *start, uint32_t *end,
+                              TransferBufs tr, const uint32_t *inv_perm, Status *st) {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     uint32_t n = d_len[kLenParticles];
     remap_transfers(tr, inv_perm, d_len, st);
     for (uint32_t id = blockIdx.x * blockDim.x + threadIdx.x; id < n; id += gridDim.x * blockDim.x) {
@@ -215,6 +217,8 @@ __global__ void __launch_bounds__(kBuildThreads, 6) k_build_rows(BuildArgs a) {
     constexpr uint32_t P = RowWalk<G>::kParticles;
     __shared__ uint32_t s_row[kRowStage * RowWalk<G>::kPad];
     __shared__ uint32_t s_cnt[P];
+    grid_dependency_wait();
+    grid_dependency_trigger();
     const uint32_t n = a.d_len[kLenParticles];
     const uint32_t last = (1u << a.L) - 1u;
     const bool uni = a.corrections && a.st->range_min != a.st->range_max;  // the radii differ: correction rows
@@ -377,13 +381,13 @@ void swap_all(apbf_ctx *ctx) { ctx->fcur ^= 1; }
 // the caller's next kernel (remap_transfers with ctx->inv_perm).
 // With `search` the gather also writes the search records (srec) for range scale
 // `scale` and reduces the search radii's range into the status block.
-apbf_status reorder_particles(apbf_ctx *ctx, cudaStream_t s, bool search, float scale) {
+apbf_status reorder_particles(apbf_ctx *ctx, cudaStream_t s, bool search, float scale, bool behind) {
     const uint32_t cap = ctx->cfg.particle_capacity;
     FluidBufs &cur = ctx->fl[ctx->fcur];
     FluidBufs &alt = ctx->fl[ctx->fcur ^ 1];
     APBF_BEFORE_LAUNCH(ctx, s, "k_reorder");
-    k_reorder<<<grid_for(ctx, cap), kBlock, 0, s>>>(cur, alt, ctx->perm, ctx->inv_perm, ctx->d_len,
-                                                    search ? ctx->srec : nullptr, scale, ctx->status);
+    APBF_CUDA(launch_behind(behind, k_reorder, grid_for(ctx, cap), kBlock, 0, s, cur, alt, ctx->perm, ctx->inv_perm,
+                            ctx->d_len, search ? ctx->srec : nullptr, scale, ctx->status));
     APBF_AFTER_LAUNCH(ctx, s, "k_reorder");
     apbf_status r = glue_remap(ctx, s);
     if (r != APBF_OK) return r;
@@ -401,7 +405,14 @@ apbf_status neighborhood_green(apbf_ctx *ctx, float range_scale, const float min
     Bounds b = fixed_bounds(minp, maxp);
     FluidBufs &cur = ctx->fl[ctx->fcur];
     const int g = grid_for(ctx, cap);
-
+    const size_t ncells = (size_t)1 << (3 * L);
+    uint32_t *cell_start = ctx->cells, *cell_end = ctx->cells + ncells;
+    // cleared ahead, so that from the sort on kernel follows kernel and each starts as the one
+    // before it ends (19 683 particles stage by stage 202 -> 194 us, 2 197 143 -> 136 a frame,
+    // 250 000 1357 -> 1344; not in a batch, whose waiting blocks would keep
+    // other scenes' off the SMs)
+    const bool behind = !ctx->in_batch;
+    APBF_CUDA(cudaMemsetAsync(ctx->cells, 0, 2 * ncells * sizeof(uint32_t), s));
     APBF_BEFORE_LAUNCH(ctx, s, "k_position_keys");
     k_position_keys<<<g, kBlock, 0, s>>>(cur.pos, ctx->d_len, b, L, ctx->keys[0], ctx->vals[0], ctx->status,
                                          ctx->d_pairs);
@@ -409,16 +420,13 @@ apbf_status neighborhood_green(apbf_ctx *ctx, float range_scale, const float min
     apbf_status r = sort_pairs_device(ctx, ctx->keys[0], ctx->vals[0], ctx->d_len + kLenParticles, cap, 3u * L,
                                       ctx->sorted_keys, ctx->perm, s);
     if (r != APBF_OK) return r;
-    r = reorder_particles(ctx, s, true, range_scale);
+    r = reorder_particles(ctx, s, true, range_scale, behind);
     if (r != APBF_OK) return r;
     FluidBufs &f = ctx->fl[ctx->fcur];
 
-    const size_t ncells = (size_t)1 << (3 * L);
-    uint32_t *cell_start = ctx->cells, *cell_end = ctx->cells + ncells;
-    APBF_CUDA(cudaMemsetAsync(ctx->cells, 0, 2 * ncells * sizeof(uint32_t), s));
     APBF_BEFORE_LAUNCH(ctx, s, "k_cell_ranges");
-    k_cell_ranges<<<g, kBlock, 0, s>>>(ctx->sorted_keys, ctx->d_len, cell_start, cell_end, ctx->tr[ctx->tcur],
-                                       ctx->inv_perm, ctx->status);
+    APBF_CUDA(launch_behind(behind, k_cell_ranges, g, kBlock, 0, s, ctx->sorted_keys, ctx->d_len, cell_start, cell_end,
+                            ctx->tr[ctx->tcur], ctx->inv_perm, ctx->status));
     APBF_AFTER_LAUNCH(ctx, s, "k_cell_ranges");
     APBF_BEFORE_LAUNCH(ctx, s, "k_build_rows");
     BuildArgs ba;
@@ -456,11 +464,11 @@ apbf_status neighborhood_green(apbf_ctx *ctx, float range_scale, const float min
     // 28 / 21 / 17 us at 2 197 particles, 60 / 55 / 60 at 32 768, 206 / 222 / 290 at 250 000,
     // 663 / 794 / 1087 at a million
     if (cap <= 12288u)
-        k_build_rows<32><<<grid_for(ctx, cap, kBuildThreads / 32, 64), kBuildThreads, 0, s>>>(ba);
+        APBF_CUDA(launch_behind(behind, k_build_rows<32>, grid_for(ctx, cap, kBuildThreads / 32, 64), kBuildThreads, 0, s, ba));
     else if (cap <= 98304u)
-        k_build_rows<16><<<grid_for(ctx, cap, kBuildThreads / 16, 64), kBuildThreads, 0, s>>>(ba);
+        APBF_CUDA(launch_behind(behind, k_build_rows<16>, grid_for(ctx, cap, kBuildThreads / 16, 64), kBuildThreads, 0, s, ba));
     else
-        k_build_rows<8><<<grid_for(ctx, cap, kBuildThreads / 8, 64), kBuildThreads, 0, s>>>(ba);
+        APBF_CUDA(launch_behind(behind, k_build_rows<8>, grid_for(ctx, cap, kBuildThreads / 8, 64), kBuildThreads, 0, s, ba));
     APBF_AFTER_LAUNCH(ctx, s, "k_build_rows");
     if (corrections) {
         APBF_BEFORE_LAUNCH(ctx, s, "k_corrections");

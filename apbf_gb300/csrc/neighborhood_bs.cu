@@ -119,10 +119,11 @@ constexpr uint32_t kTableLevel = 11;  // from this level on a cell number has at
 // level into the table (the first of a cell's run its start, the last its end).  The table
 // holds every cell when all radii have one level; the levels' range tells.  (table cleared,
 // levels {all ones, 0} beforehand.)
-__global__ void k_sorted_codes(const int4 *__restrict__ pos, const float *__restrict__ width, float scale,
-                               const uint32_t *d_len, ulonglong2 *__restrict__ code, BsCell *__restrict__ table,
-                               uint32_t mask, uint32_t *levels, TransferBufs tr, const uint32_t *__restrict__ inv_perm,
-                               Status *st, unsigned long long *total) {
+__global__ void k_sorted_codes(const int4 *pos, const float *width, float scale, const uint32_t *d_len,
+                               ulonglong2 *code, BsCell *table, uint32_t mask, uint32_t *levels, TransferBufs tr,
+                               const uint32_t *inv_perm, Status *st, unsigned long long *total) {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     const uint32_t n = d_len[kLenParticles];
     if (blockIdx.x == 0 && threadIdx.x == 0) reset_search(st, total);
     remap_transfers(tr, inv_perm, d_len, st);
@@ -240,6 +241,8 @@ __global__ void __launch_bounds__(kBuildThreads) k_bs_rows(BsArgs a) {
     using Walk = RowWalk<G>;
     __shared__ uint32_t s_row[kRowStage * Walk::kPad];
     __shared__ uint32_t s_cnt[Walk::kParticles];
+    grid_dependency_wait();
+    grid_dependency_trigger();
     const uint32_t n = a.d_len[kLenParticles];
     const bool tabled = a.levels[0] == a.levels[1] && a.levels[0] >= kTableLevel;
     Walk w(a.pos, a.idx, a.stride, a.maxn, s_row, false);
@@ -333,6 +336,13 @@ apbf_status neighborhood_binary_search(apbf_ctx *ctx, float range_scale, cudaStr
     const uint32_t cap = ctx->cfg.particle_capacity;
     const int g = grid_for(ctx, cap);
     // three stable passes, least significant word first
+    // the table and behind it the levels' range {all ones, 0}: cleared ahead, so that from the
+    // sort on kernel follows kernel and each starts as the one before it ends
+    BsCell *table = reinterpret_cast<BsCell *>(ctx->bs_table);
+    uint32_t *levels = reinterpret_cast<uint32_t *>(table + ctx->bs_slots);
+    const bool behind = !ctx->in_batch;
+    APBF_CUDA(cudaMemsetAsync(table, 0, (size_t)ctx->bs_slots * sizeof(BsCell) + 2 * sizeof(uint32_t), s));
+    APBF_CUDA(cudaMemsetAsync(levels, 0xff, sizeof(uint32_t), s));
     const bool counted = sort_takes_counts(ctx, cap);
     if (counted) APBF_CUDA(cudaMemsetAsync(ctx->bs_counts, 0, 12 * 256 * sizeof(uint32_t), s));
     for (uint32_t w = 0; w < 3; ++w) {
@@ -353,18 +363,13 @@ apbf_status neighborhood_binary_search(apbf_ctx *ctx, float range_scale, cudaStr
                                           counted ? ctx->bs_counts + w * 4 * 256 : nullptr);
         if (r != APBF_OK) return r;
     }
-    apbf_status r = reorder_particles(ctx, s);
+    apbf_status r = reorder_particles(ctx, s, false, 0.0f, behind);
     if (r != APBF_OK) return r;
     FluidBufs &f = ctx->fl[ctx->fcur];
-    // the table and behind it the levels' range {all ones, 0}
-    BsCell *table = reinterpret_cast<BsCell *>(ctx->bs_table);
-    uint32_t *levels = reinterpret_cast<uint32_t *>(table + ctx->bs_slots);
-    APBF_CUDA(cudaMemsetAsync(table, 0, (size_t)ctx->bs_slots * sizeof(BsCell) + 2 * sizeof(uint32_t), s));
-    APBF_CUDA(cudaMemsetAsync(levels, 0xff, sizeof(uint32_t), s));
     APBF_BEFORE_LAUNCH(ctx, s, "k_sorted_codes");
-    k_sorted_codes<<<g, kBlock, 0, s>>>(f.pos, f.kernel_width, range_scale, ctx->d_len, ctx->pos_code, table,
-                                        ctx->bs_slots - 1u, levels, ctx->tr[ctx->tcur], ctx->inv_perm, ctx->status,
-                                        ctx->d_pairs);
+    APBF_CUDA(launch_behind(behind, k_sorted_codes, g, kBlock, 0, s, f.pos, f.kernel_width, range_scale, ctx->d_len,
+                            ctx->pos_code, table, ctx->bs_slots - 1u, levels, ctx->tr[ctx->tcur], ctx->inv_perm,
+                            ctx->status, ctx->d_pairs));
     APBF_AFTER_LAUNCH(ctx, s, "k_sorted_codes");
     FluidBufs &spare = ctx->fl[ctx->fcur ^ 1];
     BsArgs a;
@@ -391,11 +396,11 @@ apbf_status neighborhood_binary_search(apbf_ctx *ctx, float range_scale, cudaStr
     APBF_BEFORE_LAUNCH(ctx, s, "k_bs_rows");
     // threads per particle as in the Green search: 8 / 16 / 32 take 50 / 60 / 88 us at 64 019
     if (cap <= 12288u)
-        k_bs_rows<32><<<grid_for(ctx, cap, RowWalk<32>::kParticles, 64), kBuildThreads, 0, s>>>(a);
+        APBF_CUDA(launch_behind(behind, k_bs_rows<32>, grid_for(ctx, cap, RowWalk<32>::kParticles, 64), kBuildThreads, 0, s, a));
     else if (cap <= 32768u)
-        k_bs_rows<16><<<grid_for(ctx, cap, RowWalk<16>::kParticles, 64), kBuildThreads, 0, s>>>(a);
+        APBF_CUDA(launch_behind(behind, k_bs_rows<16>, grid_for(ctx, cap, RowWalk<16>::kParticles, 64), kBuildThreads, 0, s, a));
     else
-        k_bs_rows<8><<<grid_for(ctx, cap, RowWalk<8>::kParticles, 64), kBuildThreads, 0, s>>>(a);
+        APBF_CUDA(launch_behind(behind, k_bs_rows<8>, grid_for(ctx, cap, RowWalk<8>::kParticles, 64), kBuildThreads, 0, s, a));
     APBF_AFTER_LAUNCH(ctx, s, "k_bs_rows");
     if (fuse_box) {  // the box-collided positions are the current ones now
         int4 *t = f.pos;
