@@ -163,6 +163,8 @@ __device__ __forceinline__ void push_correction(const BuildArgs &a, uint32_t row
 // walk counted some): found again on the particle's row, i's correction row
 // subtracts j, j's adds i.  A kernel of its own, so that the walk holds no atomics.
 __global__ void k_corrections(BuildArgs a) {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     if (!a.corrections || a.st->range_min == a.st->range_max) return;  // none wanted, or nothing one-sided
     const uint32_t n = a.d_len[kLenParticles];
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -348,6 +350,8 @@ __global__ void k_reverse_rows(const uint32_t *d_len, uint32_t stride, uint32_t 
 }
 
 __global__ void k_clamp_rev(const uint32_t *d_len, uint32_t maxn, uint32_t *rcount, Status *st) {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     if (st->range_min == st->range_max) return;
     uint32_t n = d_len[kLenParticles];
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
@@ -472,7 +476,7 @@ apbf_status neighborhood_green(apbf_ctx *ctx, float range_scale, const float min
     APBF_AFTER_LAUNCH(ctx, s, "k_build_rows");
     if (corrections) {
         APBF_BEFORE_LAUNCH(ctx, s, "k_corrections");
-        k_corrections<<<grid_for(ctx, cap), kBlock, 0, s>>>(ba);
+        APBF_CUDA(launch_behind(behind, k_corrections, grid_for(ctx, cap), kBlock, 0, s, ba));
         APBF_AFTER_LAUNCH(ctx, s, "k_corrections");
     }
     if (fuse_box) {  // the box-collided positions are the current ones now
@@ -482,8 +486,8 @@ apbf_status neighborhood_green(apbf_ctx *ctx, float range_scale, const float min
     }
     if (corrections) {
         APBF_BEFORE_LAUNCH(ctx, s, "k_clamp_rev");
-        k_clamp_rev<<<grid_for(ctx, cap), kBlock, 0, s>>>(ctx->d_len, ctx->cfg.max_neighbors, ctx->rev_count,
-                                                          ctx->status);
+        APBF_CUDA(launch_behind(behind, k_clamp_rev, grid_for(ctx, cap), kBlock, 0, s, ctx->d_len,
+                                ctx->cfg.max_neighbors, ctx->rev_count, ctx->status));
         APBF_AFTER_LAUNCH(ctx, s, "k_clamp_rev");
     }
     return APBF_OK;

@@ -366,6 +366,8 @@ __global__ void __launch_bounds__(THREADS) k_sort_small(const uint32_t *kin, con
                                                         uint32_t key_mask, int passes) {
     extern __shared__ unsigned char s_raw[];
     SmallSort<THREADS, ITEMS> &s = *reinterpret_cast<SmallSort<THREADS, ITEMS> *>(s_raw);
+    grid_dependency_wait();
+    grid_dependency_trigger();
     const uint32_t t = threadIdx.x, w = t >> 5, l = t & 31u;
     const uint32_t n = min(*d_count, max_count);
     uint32_t keys[ITEMS], vals[ITEMS], digit[ITEMS], rank[ITEMS];
@@ -567,11 +569,11 @@ apbf_status sort_pairs_device(apbf_ctx *ctx, const uint32_t *keys_in, const uint
     if (dbits == 8u && max_count <= SmallSort16k::kKeys) {
         APBF_BEFORE_LAUNCH(ctx, s, "k_sort_small");
         if (max_count <= SmallSort4k::kKeys)
-            k_sort_small<256, 16><<<1, 256, sizeof(SmallSort4k), s>>>(keys_in, vals_in, keys_out, vals_out, d_count,
-                                                                      max_count, key_mask, passes);
+            APBF_CUDA(launch_behind(!ctx->in_batch, k_sort_small<256, 16>, 1, 256, sizeof(SmallSort4k), s, keys_in,
+                                    vals_in, keys_out, vals_out, d_count, max_count, key_mask, passes));
         else
-            k_sort_small<1024, 16><<<1, 1024, sizeof(SmallSort16k), s>>>(keys_in, vals_in, keys_out, vals_out, d_count,
-                                                                         max_count, key_mask, passes);
+            APBF_CUDA(launch_behind(!ctx->in_batch, k_sort_small<1024, 16>, 1, 1024, sizeof(SmallSort16k), s, keys_in,
+                                    vals_in, keys_out, vals_out, d_count, max_count, key_mask, passes));
         APBF_AFTER_LAUNCH(ctx, s, "k_sort_small");
         return APBF_OK;
     }
