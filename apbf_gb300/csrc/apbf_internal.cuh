@@ -459,7 +459,7 @@ apbf_status reorder_particles(apbf_ctx *ctx, cudaStream_t s, bool search = false
 apbf_status glue_remap(apbf_ctx *ctx, cudaStream_t s);      // constraints.cu: glue ids follow a reorder
 apbf_status sort_pairs_device(apbf_ctx *ctx, const uint32_t *keys_in, const uint32_t *vals_in, const uint32_t *d_count,
                               uint32_t max_count, uint32_t key_bits, uint32_t *keys_out, uint32_t *vals_out,
-                              cudaStream_t s, const uint32_t *counts = nullptr);
+                              cudaStream_t s, const uint32_t *counts = nullptr, bool behind_kernel = false);
 bool sort_takes_counts(const apbf_ctx *ctx, uint32_t max_count);
 apbf_status sort_prepare_device();  // kernel attributes on the current device
 apbf_status prefix_sum_device(apbf_ctx *ctx, uint32_t *d_values, const uint32_t *d_count, uint32_t max_count,

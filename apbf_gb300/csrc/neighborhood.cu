@@ -422,7 +422,7 @@ apbf_status neighborhood_green(apbf_ctx *ctx, float range_scale, const float min
                                          ctx->d_pairs);
     APBF_AFTER_LAUNCH(ctx, s, "k_position_keys");
     apbf_status r = sort_pairs_device(ctx, ctx->keys[0], ctx->vals[0], ctx->d_len + kLenParticles, cap, 3u * L,
-                                      ctx->sorted_keys, ctx->perm, s);
+                                      ctx->sorted_keys, ctx->perm, s, nullptr, true);
     if (r != APBF_OK) return r;
     r = reorder_particles(ctx, s, true, range_scale, behind);
     if (r != APBF_OK) return r;

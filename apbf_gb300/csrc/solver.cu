@@ -547,6 +547,8 @@ __device__ __forceinline__ bool loop_over(const PassA &a) {
 
 template <bool GAUSS, int L, bool XTRA>
 __global__ void __launch_bounds__(256, GAUSS ? 4 : 3) k_density_lambda(PassA a) {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     const bool skip = (a.early_exit && *(volatile uint32_t *)&a.st->converged) || loop_over(a);
     // With symmetric rows or union rows the Gauss filter runs in this pass's position
     // update, which gathers over the same neighbours anyway; filter_tag tells it whether to.
@@ -931,6 +933,8 @@ __device__ __forceinline__ void update_skipped(const PassB &a, const UpdateHead 
 
 template <bool GAUSS, int L>
 __global__ void __launch_bounds__(256, 4) k_delta(PassB a) {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     const UpdateHead h = update_head<GAUSS>(a, a.d_len[kLenParticles]);
     if (h.skip) {
         update_skipped(a, h);
@@ -2351,16 +2355,21 @@ apbf_status incompressibility(apbf_ctx *ctx, cudaStream_t s, const SolveOpts &o)
         alt.pos = tmp;
         return APBF_OK;
     }
+    // a pass starts behind a position update, the update behind its density pass: four passes
+    // stage by stage over 19 683 particles 190 -> 180 us
+    const bool first_behind = o.later_pass && o.behind && !ctx->in_batch;
     APBF_BEFORE_LAUNCH(ctx, s, "k_density_lambda");
+    cudaError_t e = cudaSuccess;
     launch_lanes(lanes, [&](auto lc) {
         constexpr int Lc = decltype(lc)::value;
         if (gauss && xtra)
-            k_density_lambda<true, Lc, true><<<ga, pb, 0, s>>>(a);
+            e = launch_behind(first_behind, k_density_lambda<true, Lc, true>, ga, pb, 0, s, a);
         else if (gauss)
-            k_density_lambda<true, Lc, false><<<ga, pb, 0, s>>>(a);
+            e = launch_behind(first_behind, k_density_lambda<true, Lc, false>, ga, pb, 0, s, a);
         else
-            k_density_lambda<false, Lc, true><<<ga, pb, 0, s>>>(a);
+            e = launch_behind(first_behind, k_density_lambda<false, Lc, true>, ga, pb, 0, s, a);
     });
+    APBF_CUDA(e);
     APBF_AFTER_LAUNCH(ctx, s, "k_density_lambda");
 
     if (learned) {  // the network's lambda replaces the plain one in this update
@@ -2372,10 +2381,11 @@ apbf_status incompressibility(apbf_ctx *ctx, cudaStream_t s, const SolveOpts &o)
     launch_lanes(lanes, [&](auto lc) {
         constexpr int Lc = decltype(lc)::value;
         if (gauss)
-            k_delta<true, Lc><<<gd, pb, 0, s>>>(b);
+            e = launch_behind(!learned && !ctx->in_batch, k_delta<true, Lc>, gd, pb, 0, s, b);
         else
-            k_delta<false, Lc><<<gd, pb, 0, s>>>(b);
+            e = launch_behind(!learned && !ctx->in_batch, k_delta<false, Lc>, gd, pb, 0, s, b);
     });
+    APBF_CUDA(e);
     APBF_AFTER_LAUNCH(ctx, s, "k_delta");
     // the updated positions now live in the alternate buffer: swap position buffers
     int4 *tmp = f.pos;

@@ -545,9 +545,10 @@ bool sort_takes_counts(const apbf_ctx *ctx, uint32_t max_count) {
 // Stable sort by the low key_bits bits of the keys (rounded up to whole 4-bit
 // digits exactly as the reference's pass loop, algorithms.cpp:73).  counts (may be null;
 // only where sort_takes_counts): the keys' 8-bit digits already counted, passes x 256.
+// behind_kernel: the keys come from a kernel just launched on s.
 apbf_status sort_pairs_device(apbf_ctx *ctx, const uint32_t *keys_in, const uint32_t *vals_in, const uint32_t *d_count,
                               uint32_t max_count, uint32_t key_bits, uint32_t *keys_out, uint32_t *vals_out,
-                              cudaStream_t s, const uint32_t *counts) {
+                              cudaStream_t s, const uint32_t *counts, bool behind_kernel) {
     if (max_count == 0) return APBF_OK;
     if (max_count >= (1u << 30)) return APBF_ERR_INVALID_ARG;
     uint32_t nib = (key_bits + 3u) / 4u;  // 4-bit subkeys the reference would sort
@@ -569,10 +570,10 @@ apbf_status sort_pairs_device(apbf_ctx *ctx, const uint32_t *keys_in, const uint
     if (dbits == 8u && max_count <= SmallSort16k::kKeys) {
         APBF_BEFORE_LAUNCH(ctx, s, "k_sort_small");
         if (max_count <= SmallSort4k::kKeys)
-            APBF_CUDA(launch_behind(!ctx->in_batch, k_sort_small<256, 16>, 1, 256, sizeof(SmallSort4k), s, keys_in,
+            APBF_CUDA(launch_behind(behind_kernel && !ctx->in_batch, k_sort_small<256, 16>, 1, 256, sizeof(SmallSort4k), s, keys_in,
                                     vals_in, keys_out, vals_out, d_count, max_count, key_mask, passes));
         else
-            APBF_CUDA(launch_behind(!ctx->in_batch, k_sort_small<1024, 16>, 1, 1024, sizeof(SmallSort16k), s, keys_in,
+            APBF_CUDA(launch_behind(behind_kernel && !ctx->in_batch, k_sort_small<1024, 16>, 1, 1024, sizeof(SmallSort16k), s, keys_in,
                                     vals_in, keys_out, vals_out, d_count, max_count, key_mask, passes));
         APBF_AFTER_LAUNCH(ctx, s, "k_sort_small");
         return APBF_OK;
