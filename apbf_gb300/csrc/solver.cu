@@ -2232,7 +2232,9 @@ static PassB make_pass_b(apbf_ctx *ctx, const SolveOpts &o) {
 }
 
 // Launch shape of the two passes: the caller's when one was set (apbf_set_tuning,
-// apbf_autotune), else lanes per particle by the list's capacity.
+// apbf_autotune), else lanes per particle by the list's capacity.  The features' float sums
+// keep the row's order: one thread per particle under any shape, or the applied lambda of a
+// learned pass would depend on the tuning.
 struct PassShape {
     int lanes, block, grid;
 };
@@ -2241,14 +2243,14 @@ static PassShape pass_shape(const apbf_ctx *ctx, bool features) {
     PassShape sh;
     int per_sm = 32;  // a thread per particle (or lane) up to 1.2 million of them
     if (ctx->shape_set) {
-        sh.lanes = (int)ctx->tuning.gather_lanes;
+        sh.lanes = features ? 1 : (int)ctx->tuning.gather_lanes;
         sh.block = ctx->tuning.pass_block == 128 ? 128 : 256;
         per_sm = (int)std::min(8u, std::max(1u, ctx->tuning.pass_blocks_per_sm));
     } else {
         // Several threads share a row while the particles alone leave the chip's schedulers
         // short of warps: a frame of 2 197 particles takes 325 / 299 / 279 us with 1 / 2 / 4
         // threads, 32 768 particles 2107 / 1742 / 1756, 64 019 506 / 501 / 520, 119 771
-        // 2625 / 2751 / 3227.  The features' float sums keep the row's order: one thread.
+        // 2625 / 2751 / 3227.
         sh.block = 256;
         sh.lanes = features || cap > 98304u ? 1 : cap > 32768u ? 2 : 4;
     }

@@ -158,3 +158,44 @@ def test_tuners_on_spread_kernel_width_scene():
     g, _ = ctx.download()
     assert np.all(np.isfinite(g["velocity"]))
     ctx.close()
+
+
+def test_learned_substeps_identical_for_every_shape():
+    """The features of the learned warm start hold float sums over a row (the velocity
+    divergence, the neighbours' lambdas): a launch shape leaves the order of their terms, and
+    with it the applied lambda, as it is."""
+    import torch
+    from oracle import mlp_oracle as M
+
+    from apbf_gb300 import _native as N
+    from apbf_gb300.warmstart import SampleBuffer
+
+    rng = np.random.default_rng(4)
+    p = np.zeros(M.P_N, np.float32)
+    p[M.P_IS:M.P_IS + 7] = (0.05, 2.0, 0.5, 1.0, 0.05, 0.2, 0.2)
+    p[M.P_W1:M.P_B1] = rng.normal(size=M.H * M.F) * 0.4
+    p[M.P_W1:M.P_B1].reshape(M.H, M.F)[:, 7:] = 0.0
+    p[M.P_W2:M.P_B2] = rng.normal(size=M.H * M.H) * 0.2
+    p[M.P_W3:M.P_B3] = rng.normal(size=M.H) * 0.2
+    p[M.P_B3] = -1.0
+    p[M.P_YS] = 1.0
+    p[M.P_OMEGA] = 3.0
+    spec = scenes.dam_break(n_side=14)
+    results = []
+    for lanes, block, per_sm in ((1, 256, 8), (1, 128, 4), (2, 256, 8), (4, 128, 2), (8, 256, 4)):
+        ctx = _ctx(spec, 5, maxn=160)
+        ctx.mlp_load(torch.from_numpy(p).cuda())
+        ctx.set_warm_start(N.WARM_LEARNED | N.WARM_PROJECTED)
+        ctx.set_tuning(gather_lanes=lanes, pass_block=block, pass_blocks_per_sm=per_sm)
+        for _ in range(12):
+            ctx.substep(spec.dt)
+        buf = SampleBuffer.allocate(spec.n)
+        ctx.record_samples(3, buf.features, buf.targets, buf.count)
+        ctx.substep(spec.dt)
+        ctx.check_status()
+        results.append({**ctx.download()[0], "features": buf.features[: spec.n].cpu().numpy()})
+        ctx.close()
+    assert np.any(results[0]["features"][:, 4] != 0) and np.any(results[0]["features"][:, 6] != 0)
+    for r in results[1:]:
+        for k in r:
+            assert np.array_equal(r[k], results[0][k]), k
