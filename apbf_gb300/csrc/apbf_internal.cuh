@@ -301,7 +301,6 @@ struct apbf_ctx {
     apbf::ProfSlot *prof_open = nullptr;
     bool capturing = false;        // launches go into a graph being built: not counted
 
-    bool shape_set = false;  // launch shapes given by apbf_set_tuning / apbf_autotune: pass_shape() leaves them alone
     apbf_tuning tuning = {1u, 256u, 8u, 0u, 0u, 0u, 0u, 0u};  // launch shapes (apbf_set_tuning / apbf_autotune)
 
     // solve loop graphs (graph.cu)

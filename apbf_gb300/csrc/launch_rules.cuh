@@ -1,0 +1,36 @@
+// launch_rules.cuh -- rules that pick launch shapes from sizes and settings.  Plain C++, so
+// that a host test can go through them without a device.
+#pragma once
+
+#include <stdint.h>
+
+namespace apbf {
+
+// Threads per particle, threads per block and blocks per SM (at most) of the direct Jacobi passes.
+struct PassShape {
+    uint32_t lanes, block, per_sm;
+};
+// The shape fields of a context's apbf_tuning at creation.  They stand for the automatic
+// shape, so a tuning that changes other fields only, or writes back what apbf_get_tuning
+// returned, leaves the choice where it was.
+constexpr PassShape kAutomaticShape = {1u, 256u, 8u};
+
+inline PassShape pass_shape_rule(PassShape tuned, uint32_t capacity, bool features) {
+    PassShape sh = tuned;
+    const bool automatic = tuned.lanes == kAutomaticShape.lanes && tuned.block == kAutomaticShape.block &&
+                           tuned.per_sm == kAutomaticShape.per_sm;
+    if (automatic) {
+        // Several threads share a row while the particles alone leave the chip's schedulers
+        // short of warps: a frame of 2 197 particles takes 325 / 299 / 279 us with 1 / 2 / 4
+        // threads, 32 768 particles 2107 / 1742 / 1756, 64 019 506 / 501 / 520, 119 771
+        // 2625 / 2751 / 3227.
+        sh.lanes = capacity > 98304u ? 1u : capacity > 32768u ? 2u : 4u;
+        sh.per_sm = 32u;  // a thread per particle (or lane) up to 1.2 million of them
+    }
+    // The features' float sums keep the row's order: one thread per particle under any shape,
+    // or the applied lambda of a learned pass would depend on the tuning.
+    if (features) sh.lanes = 1u;
+    return sh;
+}
+
+}  // namespace apbf

@@ -26,6 +26,7 @@
 #include <type_traits>
 
 #include "apbf_internal.cuh"
+#include "launch_rules.cuh"
 
 namespace apbf {
 namespace {
@@ -2231,30 +2232,13 @@ static PassB make_pass_b(apbf_ctx *ctx, const SolveOpts &o) {
     return b;
 }
 
-// Launch shape of the two passes: the caller's when one was set (apbf_set_tuning,
-// apbf_autotune), else lanes per particle by the list's capacity.  The features' float sums
-// keep the row's order: one thread per particle under any shape, or the applied lambda of a
-// learned pass would depend on the tuning.
-struct PassShape {
-    int lanes, block, grid;
-};
-static PassShape pass_shape(const apbf_ctx *ctx, bool features) {
+// Launch shape of the two direct passes (launch_rules.cuh) and its grid.
+static PassShape pass_shape(const apbf_ctx *ctx, bool features, int *grid) {
     const uint32_t cap = ctx->cfg.particle_capacity;
-    PassShape sh;
-    int per_sm = 32;  // a thread per particle (or lane) up to 1.2 million of them
-    if (ctx->shape_set) {
-        sh.lanes = features ? 1 : (int)ctx->tuning.gather_lanes;
-        sh.block = ctx->tuning.pass_block == 128 ? 128 : 256;
-        per_sm = (int)std::min(8u, std::max(1u, ctx->tuning.pass_blocks_per_sm));
-    } else {
-        // Several threads share a row while the particles alone leave the chip's schedulers
-        // short of warps: a frame of 2 197 particles takes 325 / 299 / 279 us with 1 / 2 / 4
-        // threads, 32 768 particles 2107 / 1742 / 1756, 64 019 506 / 501 / 520, 119 771
-        // 2625 / 2751 / 3227.
-        sh.block = 256;
-        sh.lanes = features || cap > 98304u ? 1 : cap > 32768u ? 2 : 4;
-    }
-    sh.grid = grid_for(ctx, (uint32_t)std::min<uint64_t>((uint64_t)cap * sh.lanes, 0xffffffffu), sh.block, per_sm);
+    const apbf_tuning &t = ctx->tuning;
+    const PassShape sh = pass_shape_rule({t.gather_lanes, t.pass_block, t.pass_blocks_per_sm}, cap, features);
+    *grid = grid_for(ctx, (uint32_t)std::min<uint64_t>((uint64_t)cap * sh.lanes, 0xffffffffu), (int)sh.block,
+                     (int)sh.per_sm);
     return sh;
 }
 
@@ -2345,8 +2329,9 @@ apbf_status incompressibility(apbf_ctx *ctx, cudaStream_t s, const SolveOpts &o)
     const apbf_settings &st = ctx->settings;
     const bool gauss = st.height_kernel_id == 1 && st.gradient_kernel_id == 1;
     const PassA a = make_pass_a(ctx, o);
-    const PassShape sh = pass_shape(ctx, o.feature_mode != 0);
-    const int lanes = sh.lanes, pb = sh.block, ga = sh.grid, gd = sh.grid;
+    int grid = 0;
+    const PassShape sh = pass_shape(ctx, o.feature_mode != 0, &grid);
+    const int lanes = (int)sh.lanes, pb = (int)sh.block;
     const bool xtra = a.features != nullptr || a.method == 1;
     if (o.tiles && gauss && !xtra) {
         const PassB b = make_pass_b(ctx, o);
@@ -2365,11 +2350,11 @@ apbf_status incompressibility(apbf_ctx *ctx, cudaStream_t s, const SolveOpts &o)
     launch_lanes(lanes, [&](auto lc) {
         constexpr int Lc = decltype(lc)::value;
         if (gauss && xtra)
-            e = launch_behind(first_behind, k_density_lambda<true, Lc, true>, ga, pb, 0, s, a);
+            e = launch_behind(first_behind, k_density_lambda<true, Lc, true>, grid, pb, 0, s, a);
         else if (gauss)
-            e = launch_behind(first_behind, k_density_lambda<true, Lc, false>, ga, pb, 0, s, a);
+            e = launch_behind(first_behind, k_density_lambda<true, Lc, false>, grid, pb, 0, s, a);
         else
-            e = launch_behind(first_behind, k_density_lambda<false, Lc, true>, ga, pb, 0, s, a);
+            e = launch_behind(first_behind, k_density_lambda<false, Lc, true>, grid, pb, 0, s, a);
     });
     APBF_CUDA(e);
     APBF_AFTER_LAUNCH(ctx, s, "k_density_lambda");
@@ -2383,9 +2368,9 @@ apbf_status incompressibility(apbf_ctx *ctx, cudaStream_t s, const SolveOpts &o)
     launch_lanes(lanes, [&](auto lc) {
         constexpr int Lc = decltype(lc)::value;
         if (gauss)
-            e = launch_behind(!learned && !ctx->in_batch, k_delta<true, Lc>, gd, pb, 0, s, b);
+            e = launch_behind(!learned && !ctx->in_batch, k_delta<true, Lc>, grid, pb, 0, s, b);
         else
-            e = launch_behind(!learned && !ctx->in_batch, k_delta<false, Lc>, gd, pb, 0, s, b);
+            e = launch_behind(!learned && !ctx->in_batch, k_delta<false, Lc>, grid, pb, 0, s, b);
     });
     APBF_CUDA(e);
     APBF_AFTER_LAUNCH(ctx, s, "k_delta");

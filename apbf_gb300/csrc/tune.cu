@@ -51,7 +51,6 @@ extern "C" apbf_status apbf_set_tuning(apbf_ctx *ctx, const apbf_tuning *t) {
         return APBF_ERR_INVALID_ARG;
     }
     ctx->tuning = *t;
-    ctx->shape_set = true;
     ctx->graph_version++;
     return APBF_OK;
 }
@@ -88,8 +87,6 @@ extern "C" apbf_status apbf_autotune(apbf_ctx *ctx, void *stream, apbf_tuning *c
     const bool prof = ctx->prof_on;
     ctx->prof_on = false;
     const apbf_tuning before = ctx->tuning;
-    const bool set_before = ctx->shape_set;
-    ctx->shape_set = true;  // the candidates' shapes are the ones timed
     const int lanes[4] = {1, 2, 4, 8}, blocks[2] = {128, 256}, per_sm[3] = {2, 4, 8};
     constexpr int kCands = 24;
     float best_ms = 0.0f, times[kCands] = {};
@@ -119,7 +116,6 @@ extern "C" apbf_status apbf_autotune(apbf_ctx *ctx, void *stream, apbf_tuning *c
     ctx->prof_on = prof;
     if (r != APBF_OK) {
         ctx->tuning = before;
-        ctx->shape_set = set_before;
         return r;
     }
     ctx->tuning = best_t;

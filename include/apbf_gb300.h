@@ -183,9 +183,15 @@ typedef struct apbf_status_info {
 
 /* Launch shapes of the context's kernels (no reference counterpart: the
  * reference's workgroup sizes are fixed in its shaders).  Results do not depend
- * on them. */
+ * on them.  The first three fields shape the direct density and position passes:
+ * those of apbf_incompressibility_apply, of substeps whose solve is short or uses
+ * other kernels than Gauss, and of the learned warm start's first pass.  The
+ * passes of a longer Gauss solve of apbf_substep have a shape of their own.  The
+ * values of a new context, 1, 256 and 8, stand for the shape the context picks by
+ * its capacity; apbf_get_tuning returns them as long as that one is in use. */
 typedef struct apbf_tuning {
-    uint32_t gather_lanes;        /* threads per particle in the density and position passes: 1, 2, 4 or 8 */
+    uint32_t gather_lanes;        /* threads per particle in the direct passes: 1, 2, 4 or 8 (one in the
+                                     learned warm start's first pass, whose sums keep the row's order) */
     uint32_t pass_block;          /* threads per block of those passes: 128 or 256 */
     uint32_t pass_blocks_per_sm;  /* their grid: up to this many blocks per SM (1..8) */
     uint32_t reserved0;           /* must be 0 */
@@ -410,11 +416,12 @@ apbf_status apbf_batch_destroy(apbf_batch *batch);
 apbf_status apbf_batch_set_persistent_solve(apbf_batch *batch, int enable);
 
 /* Launch shapes (no counterpart in the reference).  apbf_autotune times every
- * candidate shape of the Jacobi passes on the context's current particle state and
- * neighbour rows (call it after a substep or a neighbourhood search), keeps the
+ * candidate shape of the direct Jacobi passes on the context's current particle state
+ * and neighbour rows (call it after a substep or a neighbourhood search), keeps the
  * fastest and restores the state it ran on; pass_ms (may be NULL) receives the
  * time of one pass for each of the 24 candidates, in the order gather_lanes
- * (1, 2, 4, 8) x pass_block (128, 256) x pass_blocks_per_sm (2, 4, 8). */
+ * (1, 2, 4, 8) x pass_block (128, 256) x pass_blocks_per_sm (2, 4, 8).  The
+ * candidate 1, 256, 8 is the automatic shape (see apbf_tuning). */
 apbf_status apbf_set_tuning(apbf_ctx *ctx, const apbf_tuning *t);
 apbf_status apbf_get_tuning(apbf_ctx *ctx, apbf_tuning *t);
 apbf_status apbf_autotune(apbf_ctx *ctx, void *stream, apbf_tuning *chosen, float *pass_ms);
