@@ -40,10 +40,26 @@ __device__ __forceinline__ uint32_t isqrt_u64(unsigned long long x) {
     return (uint32_t)r;
 }
 
-// Rows longer than this are left by their thread to its whole warp: a lane alone waits a
-// memory latency for every four entries of a row that can hold hundreds, and its warp and
-// the kernel's last block with it.
+// The lanes whose rows (c entries each) their warp walks together, one row after the other;
+// the others walk their own.  A lane waits a memory latency for every four entries, so a
+// single row of hundreds holds up its warp and the kernel's last block; the whole warp takes
+// half that time for every 32 entries and once more to begin with, but row by row.  Rows above
+// the cut with the least time go to the warp: a few long rows among short ones, none where
+// most are long (262 144 particles with rows of 126 entries, k_kw_spread: 588 us when the warp
+// takes every row above 64, 125 so).
 constexpr uint32_t kLongRow = 64;
+__device__ __forceinline__ uint32_t rows_for_warp(uint32_t c) {
+    const uint32_t longest = __reduce_max_sync(0xffffffffu, c);
+    uint32_t cut = longest, least = longest / 2u;  // in steps of a warp
+    for (uint32_t t = kLongRow; t < longest; t *= 2u) {
+        const uint32_t time = t / 2u + __reduce_add_sync(0xffffffffu, c > t ? c / 32u + 1u : 0u);
+        if (time < least) {
+            least = time;
+            cut = t;
+        }
+    }
+    return __ballot_sync(0xffffffffu, c > cut);
+}
 
 __device__ __forceinline__ uint32_t fixed_dist(int4 a, int4 b) {
     long long dx = (long long)b.x - a.x, dy = (long long)b.y - a.y, dz = (long long)b.z - a.z;
@@ -68,7 +84,7 @@ struct FsmMin {
         }
     }
 };
-__global__ void k_fsm12(const int4 *__restrict__ pos, const uint32_t *__restrict__ old_bd,
+__global__ void __launch_bounds__(256, 4) k_fsm12(const int4 *__restrict__ pos, const uint32_t *__restrict__ old_bd,
                         uint32_t *__restrict__ new_bd, uint32_t *__restrict__ nearest, const uint32_t *count,
                         const uint32_t *idx, uint32_t stride, const uint32_t *d_len) {
     const uint32_t n = d_len[kLenParticles];
@@ -78,7 +94,8 @@ __global__ void k_fsm12(const int4 *__restrict__ pos, const uint32_t *__restrict
         const uint32_t i = base + threadIdx.x;
         const int4 p = i < n ? pos[i] : make_int4(0, 0, 0, 0);
         const uint32_t c = i < n ? count[i] : 0u;
-        const uint32_t mine = c > kLongRow ? 0u : c;
+        const uint32_t shared = rows_for_warp(c);
+        const uint32_t mine = shared >> lane & 1u ? 0u : c;
         FsmMin m;
         const uint32_t *row = idx + i;
         // batches of four neighbours, software-pipelined: a batch's gathers go out with
@@ -86,7 +103,7 @@ __global__ void k_fsm12(const int4 *__restrict__ pos, const uint32_t *__restrict
         constexpr uint32_t U = 4;
         uint32_t jj[U];
 #pragma unroll
-        for (uint32_t u = 0; u < U; ++u) jj[u] = u < mine ? row[(size_t)u * stride] : 0u;
+        for (uint32_t u = 0; u < U; ++u) jj[u] = u < mine ? row[(size_t)u * stride] : i;
         for (uint32_t k0 = 0; k0 < mine; k0 += U) {
             int4 q[U];
             uint32_t ob[U], jn[U];
@@ -98,7 +115,7 @@ __global__ void k_fsm12(const int4 *__restrict__ pos, const uint32_t *__restrict
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u) {
                 const uint32_t k = k0 + U + u;
-                jn[u] = k < mine ? row[(size_t)k * stride] : 0u;
+                jn[u] = k < mine ? row[(size_t)k * stride] : i;
             }
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u) {
@@ -108,7 +125,7 @@ __global__ void k_fsm12(const int4 *__restrict__ pos, const uint32_t *__restrict
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u) jj[u] = jn[u];
         }
-        for (uint32_t left = __ballot_sync(0xffffffffu, c > kLongRow); left; left &= left - 1u) {
+        for (uint32_t left = shared; left; left &= left - 1u) {
             const int src = __ffs(left) - 1;
             const uint32_t li = __shfl_sync(0xffffffffu, i, src), lc = __shfl_sync(0xffffffffu, c, src);
             const int4 lp = pos[li];
@@ -486,7 +503,7 @@ __device__ __forceinline__ bool spread_pair(int4 p, int4 q, uint32_t j, uint32_t
 }
 
 // kernel_width.comp:26-61: spread (atomicMax) and prune row i in place, order kept.
-__global__ void k_kw_spread(FluidBufs f, uint32_t *ukw, uint32_t *count, uint32_t *idx, uint32_t stride,
+__global__ void __launch_bounds__(256, 4) k_kw_spread(FluidBufs f, uint32_t *ukw, uint32_t *count, uint32_t *idx, uint32_t stride,
                             const uint32_t *d_len, int use_target) {
     const uint32_t n = d_len[kLenParticles];
     const uint32_t lane = threadIdx.x & 31u;
@@ -498,7 +515,8 @@ __global__ void k_kw_spread(FluidBufs f, uint32_t *ukw, uint32_t *count, uint32_
         const float ok = valid ? fmaxf(f.radius[i], tr) * 4.0f : 0.0f;
         const float cut = valid ? fmaxf(ok, f.kernel_width[i]) : 0.0f;
         const uint32_t c = valid ? count[i] : 0u;
-        const uint32_t mine = c > kLongRow ? 0u : c;
+        const uint32_t shared = rows_for_warp(c);
+        const uint32_t mine = shared >> lane & 1u ? 0u : c;
         uint32_t w = 0;
         // batches of four neighbours, software-pipelined (the pruned row is written
         // behind the entries read ahead)
@@ -506,7 +524,7 @@ __global__ void k_kw_spread(FluidBufs f, uint32_t *ukw, uint32_t *count, uint32_
         uint32_t *row = idx + i;
         uint32_t jj[U];
 #pragma unroll
-        for (uint32_t u = 0; u < U; ++u) jj[u] = u < mine ? row[(size_t)u * stride] : 0u;
+        for (uint32_t u = 0; u < U; ++u) jj[u] = u < mine ? row[(size_t)u * stride] : i;
         for (uint32_t k0 = 0; k0 < mine; k0 += U) {
             int4 q[U];
             uint32_t cur[U], jn[U];
@@ -518,7 +536,7 @@ __global__ void k_kw_spread(FluidBufs f, uint32_t *ukw, uint32_t *count, uint32_
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u) {
                 const uint32_t k = k0 + U + u;
-                jn[u] = k < mine ? row[(size_t)k * stride] : 0u;
+                jn[u] = k < mine ? row[(size_t)k * stride] : i;
             }
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u) {
@@ -528,7 +546,7 @@ __global__ void k_kw_spread(FluidBufs f, uint32_t *ukw, uint32_t *count, uint32_
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u) jj[u] = jn[u];
         }
-        for (uint32_t left = __ballot_sync(0xffffffffu, c > kLongRow); left; left &= left - 1u) {
+        for (uint32_t left = shared; left; left &= left - 1u) {
             const int src = __ffs(left) - 1;
             const uint32_t li = __shfl_sync(0xffffffffu, i, src), lc = __shfl_sync(0xffffffffu, c, src);
             const float lok = __shfl_sync(0xffffffffu, ok, src), lcut = __shfl_sync(0xffffffffu, cut, src);
