@@ -108,7 +108,8 @@ constexpr uint32_t kTileSmallest = 64;  // particles of the smaller tile shape
 constexpr uint32_t kHaloOver = 0xffffffffu, kNoParticle = 0xffffffffu;
 struct TilePlan {
     uint32_t *halo;        // [tile * kTileHalo + slot]: particles outside the tile
-    uint4 *tile;           // per tile: halo entries (kHaloOver: they did not fit), particles, largest |radius|, 0
+    uint4 *tile;           // per tile: halo entries (kHaloOver: they did not fit), particles, largest |radius|,
+                           // 1: long rows are walked by their threads (rests_by_lane)
     uint32_t *lane;        // [tile * T + rank]: the tile's particles by falling row length, place in the tile
                            // | row length << 8; kNoParticle past the list's end
     uint2 *rows;           // [(tile * kTileDepth / 4 + q) * T + rank]: entries 4q..4q+3 as 16-bit record offsets

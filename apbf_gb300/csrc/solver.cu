@@ -966,12 +966,23 @@ __global__ void __launch_bounds__(256, 4) k_delta(PassB a) {
 // the direct passes' own, so the results are bit-identical.
 //
 // Entries from kTileDepth on and tiles whose halo exceeds kTileHalo are read from the list's
-// own rows.
+// own rows, or from the pool (rests_by_lane).
 
 // Eight neighbouring particles, whose records share a line, keep together in the table and
 // so in the halo, which takes its order; the groups are spread.
 __device__ __forceinline__ uint32_t tile_hash(uint32_t j, uint32_t mask) {
     return (((j >> 3) * 2654435761u >> 16) << 3 | (j & 7u)) & mask;
+}
+
+// Who walks the entries from kTileDepth on of a tile's `rows` long rows, `longest` entries
+// the longest: their own threads (true), a memory latency for every four entries but all
+// rows at once, or each row a whole warp, two latencies for every 128 entries and the sums
+// across it, one row after the other.  Rows are dealt by falling length, so a tile's long
+// ones share warps.  Whole warps alone took 2.1 times the direct passes' time where all rows
+// are long (512 000 particles with rows of 181 entries, eight passes: 13.9 against 6.5 ms).
+__device__ __forceinline__ bool rests_by_lane(uint32_t rows, uint32_t longest) {
+    const uint32_t rest = longest - (uint32_t)kTileDepth;
+    return rows >= 32u || (rows != 0u && rows * (2u * (rest / 128u) + 3u) > rest);
 }
 
 struct TileRowsArgs {
@@ -997,7 +1008,7 @@ __global__ void __launch_bounds__(256) k_tile_rows(TileRowsArgs a) {
     __shared__ uint32_t s_bin[64];
     __shared__ uint16_t s_rank[T];
     __shared__ uint32_t s_scan[8];
-    __shared__ uint32_t s_full, s_rmax;
+    __shared__ uint32_t s_full, s_rmax, s_long, s_longest;
     if (a.reverse && (a.st->range_min == a.st->range_max || a.st->union_rows != 0u)) return;
     const uint32_t n = a.d_len[kLenParticles];
     const uint32_t o = threadIdx.x % T, sub = threadIdx.x / T;  // a warp reads consecutive particles' entries
@@ -1007,7 +1018,7 @@ __global__ void __launch_bounds__(256) k_tile_rows(TileRowsArgs a) {
         const float r = i < n ? fabsf(a.radius[i]) : 0.0f;
         for (uint32_t k = threadIdx.x; k < kSlots; k += 256) s_key[k] = 0xffffffffu;
         if (threadIdx.x < 64) s_bin[threadIdx.x] = 0u;
-        if (threadIdx.x == 0) s_full = s_rmax = 0u;
+        if (threadIdx.x == 0) s_full = s_rmax = s_long = s_longest = 0u;
         __syncthreads();
         const uint32_t depth = min(cnt, (uint32_t)kTileDepth);
         // falling row length: a counting sort (the order among equal lengths is free)
@@ -1015,6 +1026,13 @@ __global__ void __launch_bounds__(256) k_tile_rows(TileRowsArgs a) {
         if (sub == 0) atomicAdd(&s_bin[bin], 1u);
         const uint32_t rm = __reduce_max_sync(0xffffffffu, __float_as_uint(r));
         if ((threadIdx.x & 31u) == 0u) atomicMax(&s_rmax, rm);
+        if (sub == 0) {
+            const uint32_t lm = __ballot_sync(0xffffffffu, cnt > kTileDepth), most = __reduce_max_sync(0xffffffffu, cnt);
+            if (lm && (threadIdx.x & 31u) == 0u) {
+                atomicAdd(&s_long, (uint32_t)__popc(lm));
+                atomicMax(&s_longest, most);
+            }
+        }
         // the code of entry j: the offset of its record when it lies in the tile, else
         // its slot in the table of the halo, entered when it is not there yet.  Only the keys
         // are entered here; numbering them here as well (a counter that every insert waits
@@ -1100,8 +1118,9 @@ __global__ void __launch_bounds__(256) k_tile_rows(TileRowsArgs a) {
             a.plan.lane[base + k] = i < n ? o | cnt << 8 : kNoParticle;
         }
         // the rest of the long rows, each in one run of the pool: read through the list's
-        // own rows, every entry would touch another page
-        if (sub == 0)
+        // own rows by a warp, every entry would touch another page
+        const bool lanes = rests_by_lane(s_long, s_longest);
+        if (sub == 0 && !lanes)
             for (uint32_t left = __ballot_sync(0xffffffffu, cnt > kTileDepth); left; left &= left - 1u) {
                 const int src = __ffs(left) - 1;
                 const uint32_t li = __shfl_sync(0xffffffffu, i, src), m = __shfl_sync(0xffffffffu, cnt, src) - kTileDepth;
@@ -1117,9 +1136,8 @@ __global__ void __launch_bounds__(256) k_tile_rows(TileRowsArgs a) {
                     for (uint32_t k = lane; k < m; k += 32u)
                         a.plan.pool[at + k] = a.idx[(size_t)(kTileDepth + k) * a.stride + li];
             }
-        if (threadIdx.x == 0) {
-            a.plan.tile[tile] = make_uint4(over ? kHaloOver : halo, min(n - base, (uint32_t)T), s_rmax, 0u);
-        }
+        if (threadIdx.x == 0)
+            a.plan.tile[tile] = make_uint4(over ? kHaloOver : halo, min(n - base, (uint32_t)T), s_rmax, lanes ? 1u : 0u);
         __syncthreads();
         if (!over) {
             uint2 *out = a.plan.rows + (size_t)tile * (T * kTileDepth / 4) + s_rank[o];
@@ -1253,6 +1271,29 @@ struct WarpRow {
     }
 };
 
+// Entries k, k + L, ... below end of a list's row, walked by one thread: four gathers in
+// flight with the four entries behind them.
+template <uint32_t L, typename G, typename F>
+__device__ __forceinline__ void lane_row(const uint32_t *row, size_t stride, uint32_t k, uint32_t end, G load, F f) {
+    if (k >= end) return;
+    uint32_t j[4];
+#pragma unroll
+    for (uint32_t u = 0; u < 4; ++u) j[u] = k + u * L < end ? row[(k + u * L) * stride] : 0u;
+#pragma unroll 1
+    for (; k < end; k += 4u * L) {
+        int4 q[4];
+        uint32_t nj[4];
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u) q[u] = load(j[u]);
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u) nj[u] = k + (4u + u) * L < end ? row[(k + (4u + u) * L) * stride] : 0u;
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u)
+            if (k + u * L < end) f(j[u], q[u]);
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u) j[u] = nj[u];
+    }
+}
 
 // A tile's density pass: T particles, L threads each.  At a million particles in a
 // waterfall (13.4 M pairs) 62 us against 92 us for the direct kernel, 26 against 35 us at
@@ -1368,14 +1409,13 @@ __global__ void __launch_bounds__(T *L, 1024 / (T * L)) k_density_tiles(PassA a,
                 add(q, __int_as_float(q.w));
             }
         }
-        const uint32_t shallow = min(cnt, (uint32_t)kTileDepth);
-#pragma unroll 2
-        for (uint32_t k = depth + sub; k < shallow; k += L) {  // a tile whose halo did not fit
-            const int4 q = a.pos[a.idx[(size_t)k * a.stride + i]];
-            add(q, __int_as_float(q.w) * APBF_FIX);
-        }
-        // what is left of the long rows: one row after the other, by the whole warp
-        for (uint32_t left = __ballot_sync(0xffffffffu, sub == 0u && cnt > kTileDepth); left; left &= left - 1u) {
+        // what the tile does not hold: all of the rows where its halo did not fit, and the rest
+        // of the long ones, by their threads or one row after the other by the whole warp
+        const bool by_warp = head.w == 0u && cnt > kTileDepth;
+        const uint32_t end = by_warp ? (uint32_t)kTileDepth : cnt;
+        lane_row<L>(a.idx + i, a.stride, depth + sub, end, [&](uint32_t j) { return a.pos[j]; },
+                    [&](uint32_t, const int4 &q) { add(q, __int_as_float(q.w) * APBF_FIX); });
+        for (uint32_t left = __ballot_sync(0xffffffffu, sub == 0u && by_warp); left; left &= left - 1u) {
             const int src = __ffs(left) - 1;
             const WarpRow w(plan, a.idx, a.stride, i, cnt, p, src);
             const GaussPair gw = gauss_pair(__shfl_sync(0xffffffffu, gp.ivd36, src), __shfl_sync(0xffffffffu, gp.norm, src));
@@ -1428,11 +1468,11 @@ __global__ void __launch_bounds__(T *L, 1024 / (T * L)) k_density_tiles(PassA a,
                     for (uint32_t u = 0; u < 4; ++u)
                         hit = hit || gauss_filter_hit(ed, fdiff(p, tile_record(s_pos, row_offset(now, u))));
                 }
-#pragma unroll 2
-                for (uint32_t k = depth; k < shallow && !hit; ++k)
-                    hit = gauss_filter_hit(ed, fdiff(p, a.pos[a.idx[(size_t)k * a.stride + i]]));
+                if (!hit)
+                    lane_row<1>(a.idx + i, a.stride, depth, end, [&](uint32_t j) { return a.pos[j]; },
+                                [&](uint32_t, const int4 &q) { hit = hit || gauss_filter_hit(ed, fdiff(p, q)); });
             }
-            for (uint32_t left = __ballot_sync(0xffffffffu, ask && !hit && cnt > kTileDepth); left; left &= left - 1u) {
+            for (uint32_t left = __ballot_sync(0xffffffffu, ask && !hit && by_warp); left; left &= left - 1u) {
                 const int src = __ffs(left) - 1;
                 const WarpRow w(plan, a.idx, a.stride, i, cnt, p, src);
                 const float3 ew = make_float3(__shfl_sync(0xffffffffu, ed.x, src), __shfl_sync(0xffffffffu, ed.y, src),
@@ -1691,16 +1731,14 @@ __global__ void __launch_bounds__(T *L, 896 / (T * L)) k_delta_tiles(PassB a, Ti
                 add(q, __int_as_float(q.w), gauss_pair(kk.x, kk.y), false);
             }
         }
-        const uint32_t shallow = min(cnt, (uint32_t)kTileDepth);
-#pragma unroll 2
-        for (uint32_t k = depth + sub; k < shallow; k += L) {  // a tile whose halo did not fit
-            const uint32_t g = idx_arr[(size_t)k * a.stride + j] & ~kNoDelta;
-            const float2 kk = h.packed ? kcj : a.kc[g];
-            const int4 q = a.pk[g];
-            add(q, __int_as_float(q.w) * APBF_FIX, gauss_pair(kk.x, kk.y), true);
-        }
-        // what is left of the long rows: one row after the other, by the whole warp
-        for (uint32_t left = __ballot_sync(0xffffffffu, sub == 0u && cnt > kTileDepth); left; left &= left - 1u) {
+        // what the tile does not hold, as in k_density_tiles
+        const bool by_warp = head.w == 0u && cnt > kTileDepth;
+        lane_row<L>(idx_arr + j, a.stride, depth + sub, by_warp ? (uint32_t)kTileDepth : cnt,
+                    [&](uint32_t g) { return a.pk[g & ~kNoDelta]; }, [&](uint32_t g, const int4 &q) {
+                        const float2 kk = h.packed ? kcj : a.kc[g & ~kNoDelta];
+                        add(q, __int_as_float(q.w) * APBF_FIX, gauss_pair(kk.x, kk.y), true);
+                    });
+        for (uint32_t left = __ballot_sync(0xffffffffu, sub == 0u && by_warp); left; left &= left - 1u) {
             const int src = __ffs(left) - 1;
             const WarpRow w(plan, idx_arr, a.stride, j, cnt, p, src);
             const float2 kw = make_float2(__shfl_sync(0xffffffffu, kcj.x, src), __shfl_sync(0xffffffffu, kcj.y, src));
