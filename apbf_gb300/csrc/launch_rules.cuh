@@ -25,11 +25,19 @@ inline PassShape pass_shape_rule(PassShape tuned, uint32_t capacity, bool featur
         // threads, 32 768 particles 2107 / 1742 / 1756, 64 019 506 / 501 / 520, 119 771
         // 2625 / 2751 / 3227.
         sh.lanes = capacity > 98304u ? 1u : capacity > 32768u ? 2u : 4u;
-        sh.per_sm = 32u;  // a thread per particle (or lane) up to 1.2 million of them
+        sh.per_sm = 32u;  // a thread per particle and lane
     }
     // The features' float sums keep the row's order: one thread per particle under any shape,
     // or the applied lambda of a learned pass would depend on the tuning.
     if (features) sh.lanes = 1u;
+    // One thread per particle: blocks that are all resident and take several particles per
+    // thread, as every block begins with the sums of the pass before it.  Density and position
+    // pass at 262 144 particles 75.8 us with blocks of 256, a particle per thread, 73.1 so; at
+    // a million 250.5 and 234.4, with 6 neighbours instead of 32 102.1 and 85.7.
+    if (automatic && sh.lanes == 1u) {
+        sh.block = 128u;
+        sh.per_sm = 8u;
+    }
     return sh;
 }
 
