@@ -577,7 +577,7 @@ __device__ __forceinline__ void reset_search(Status *st, unsigned long long *tot
 }
 
 // The transfer list behind a reorder (indexed_list.h:288-308); every thread of the grid.
-__device__ __forceinline__ void remap_transfers(const TransferBufs &t, const uint32_t *__restrict__ inv_perm,
+__device__ __forceinline__ void remap_transfers(const TransferBufs &t, const uint32_t *inv_perm,
                                                 const uint32_t *d_len, Status *st) {
     const uint32_t nt = d_len[kLenTransfers], n = d_len[kLenParticles];
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nt; k += gridDim.x * blockDim.x) {

@@ -167,7 +167,7 @@ __global__ void k_sorted_codes(const int4 *pos, const float *width, float scale,
 // for a prefix of the list; searched outward from `hint` with doubling steps and then
 // bisected: cells near a particle are mostly near it in the sorted order.
 template <typename F>
-__device__ __forceinline__ uint32_t first_not(const ulonglong2 *__restrict__ code, uint32_t n, uint32_t hint, F before) {
+__device__ __forceinline__ uint32_t first_not(const ulonglong2 *code, uint32_t n, uint32_t hint, F before) {
     uint32_t lo, hi;  // the answer lies in [lo, hi]
     if (before(code[hint])) {
         uint32_t a = hint, step = 1;  // before(code[a])

@@ -352,7 +352,7 @@ __device__ __forceinline__ bool density_finish(const PassA &a, const int4 *pos, 
 // incompressibility_0..2 and the boundariness filter of incompressibility_3.
 // Every lane of the group must call it (group shuffles).
 template <bool GAUSS, int L, bool XTRA>
-__device__ __forceinline__ void density_one(const PassA &a, const int4 *__restrict__ pos, uint32_t i_raw, uint32_t n,
+__device__ __forceinline__ void density_one(const PassA &a, const int4 *pos, uint32_t i_raw, uint32_t n,
                                             uint32_t sub, bool defer, bool write_rec, PassSums &ps) {
     {
         const bool valid = i_raw < n;
@@ -667,7 +667,7 @@ __device__ __forceinline__ int3 pair_delta(const PassB &a, int4 q, float lam, fl
 // records and the neighbours' Gauss constants; other kernels: the solve records
 // and the positions.
 template <bool GAUSS, int L, bool PACKED>
-__device__ __forceinline__ int3 delta_row(const PassB &a, const int4 *__restrict__ pos, const uint32_t *row, uint32_t cnt,
+__device__ __forceinline__ int3 delta_row(const PassB &a, const int4 *pos, const uint32_t *row, uint32_t cnt,
                                           uint32_t fcnt, uint32_t j, uint32_t sub, int4 p, const GaussPair &cj,
                                           bool fil, float3 ed, bool &hit, int4 start) {
     int32_t ax = start.x, ay = start.y, az = start.z;
@@ -736,7 +736,7 @@ __device__ __forceinline__ int3 delta_row(const PassB &a, const int4 *__restrict
 // j), the others added (they hold j, j's radius does not reach them).  Lane sub of
 // the group of L takes entries sub, sub + L, ...
 template <bool GAUSS, int L, bool PACKED>
-__device__ __forceinline__ int3 delta_corrections(const PassB &a, const int4 *__restrict__ pos, uint32_t m, uint32_t j,
+__device__ __forceinline__ int3 delta_corrections(const PassB &a, const int4 *pos, uint32_t m, uint32_t j,
                                                   uint32_t sub, int4 p, const GaussPair &cj, int3 acc) {
     for (uint32_t k = sub; k < m; k += L) {
         const uint32_t e = a.ridx[(size_t)k * a.stride + j];
@@ -792,7 +792,7 @@ __device__ __forceinline__ void delta_finish(const PassB &a, int4 *pos_out, uint
 // collision (nboxes > 0) and the lambda bookkeeping.  Every lane of the group
 // must call it (group shuffles).
 template <bool GAUSS, int L>
-__device__ __forceinline__ void delta_one(const PassB &a, const int4 *__restrict__ pos, int4 *pos_out, uint32_t j_raw,
+__device__ __forceinline__ void delta_one(const PassB &a, const int4 *pos, int4 *pos_out, uint32_t j_raw,
                                           uint32_t n, uint32_t sub, bool packed, bool filter, const uint32_t *cnt_arr,
                                           const uint32_t *idx_arr, bool corr, uint32_t nboxes) {
     {
@@ -849,7 +849,7 @@ __device__ __forceinline__ void delta_one(const PassB &a, const int4 *__restrict
 
 // A converged pass (no position update) of particle j: the deferred filter still
 // belongs to it, the positions are copied through and nothing is applied.
-__device__ __forceinline__ void delta_skip_filter(const PassB &a, const int4 *__restrict__ pos, uint32_t j) {
+__device__ __forceinline__ void delta_skip_filter(const PassB &a, const int4 *pos, uint32_t j) {
     if (!a.shift[j].w) return;
     const int4 fj = a.filt[j];
     float3 ed;
