@@ -90,7 +90,7 @@ struct PassA {
     int early_exit;      // skip the pass when st->converged is set
     float rmin3;  // pow(2 * smallestTargetRadius, 3)
     int hk, gk, method, update_b;
-    float one;  // 1, as a value the assembler does not know (see F2)
+    float one;  // 1, as a value that is not known before the launch (see F2)
     float b_speed, b_sgl_factor, b_up_factor;
 };
 
@@ -1165,10 +1165,10 @@ __global__ void __launch_bounds__(256) k_tile_rows(TileRowsArgs a) {
 }
 
 // Two FP32 values in one 64-bit register pair: the packed operations round each half
-// like the scalar ones, at half the issue slots.  The assembler contracts a packed
-// product and a packed sum into one FMA whatever their rounding modifiers and -fmad say,
-// which the passes must not (dot3x): sums are written as fma(a, 1, b), which rounds
-// a + b once, with the 1 taken from the kernel's arguments so that it stays a value.
+// like the scalar ones, at half the issue slots.  A packed product followed by a packed sum
+// gave the values of one FMA, whatever the rounding modifiers and -fmad, where the passes
+// must round twice (dot3x): sums are written as fma(a, 1, b), which rounds a + b once, with
+// the 1 taken from the kernel's arguments so that it stays a value.
 struct F2 {
     unsigned long long v;
 };
@@ -1207,9 +1207,10 @@ __device__ __forceinline__ float ex2_ftz(float x) {
 }
 
 // The Gauss height W and the gradient factor s (gradient = s D) of two offsets at
-// once, as gauss_terms_r2 computes them, for exponents of at least -126: below, exp2f
-// scales around the subnormal range, which the flushing form does not.  low collects the
-// smallest exponent; a row in which it fell below is summed again by gauss_terms_r2.
+// once, as gauss_terms_r2 computes them, for exponents of at least -126: 2^-126 is the
+// smallest normal number, so down to there ex2_ftz flushes nothing, and its values are exp2f's
+// (test_gpu_exponential.py compares all of them).  low collects the smallest exponent; a row
+// in which it fell below is summed again by gauss_terms_r2.
 __device__ __forceinline__ void gauss_two(F2 r2, F2 ivd36, F2 norm, F2 k2, float &low, F2 &W, F2 &s) {
     const float2 x = f2_unpack(r2 * ivd36);
     low = fminf(fminf(low, x.x), x.y);
@@ -1401,7 +1402,7 @@ __global__ void __launch_bounds__(T *L, 1024 / (T * L)) k_density_tiles(PassA a,
             rs.sq += f2u(dot3x(g, g) * mjf);
         };
         if (L > 1) low = group_min<L>(low);  // the group sums its row again as one
-        if (low < kLowExponent) {  // far out in a narrow kernel: exp2f's own range handling
+        if (low < kLowExponent) {  // far out in a narrow kernel: subnormal results
             rs = RowSums();
 #pragma unroll 1
             for (uint32_t k = sub; k < depth; k += L) {
@@ -1721,7 +1722,7 @@ __global__ void __launch_bounds__(T *L, 896 / (T * L)) k_delta_tiles(PassB a, Ti
             acc.z = wadd(acc.z, f2i(g.z * sc));
         };
         if (L > 1) low = group_min<L>(low);  // the group sums its row again as one
-        if (low < kLowExponent) {  // far out in a narrow kernel: exp2f's own range handling
+        if (low < kLowExponent) {  // far out in a narrow kernel: subnormal results
             acc = start;
 #pragma unroll 1
             for (uint32_t k = sub; k < depth; k += L) {
