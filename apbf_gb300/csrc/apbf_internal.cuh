@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "../../include/apbf_gb300.h"
+#include "launch_rules.cuh"
 
 #define APBF_FIX 262144.0f
 #define APBF_INV_FIX (1.0f / 262144.0f)
@@ -97,8 +98,8 @@ struct PassSync {
     unsigned long long e[2][kSumStripes][16];
     uint32_t cur_density;
     uint32_t cur_update;
-    uint32_t pool_used[2];  // entries taken of the two tile plans' pools
-    uint32_t pad[28];
+    PoolCount pool_used[2];  // entries asked of the two tile plans' pools (launch_rules.cuh)
+    uint32_t pad[26];
 };
 
 // The neighbour rows of a substep rewritten for the tiled passes (solver.cu).
@@ -114,7 +115,8 @@ struct TilePlan {
                            // | row length << 8; kNoParticle past the list's end
     uint2 *rows;           // [(tile * kTileDepth / 4 + q) * T + rank]: entries 4q..4q+3 as 16-bit record offsets
     uint32_t *tail;        // per particle with a longer row: where its rest starts in the pool (all ones: not there)
-    uint32_t *pool, *pool_used;
+    uint32_t *pool;
+    PoolCount *pool_used;
     uint32_t pool_size;
 };
 

@@ -1,8 +1,14 @@
-// launch_rules.cuh -- rules that pick launch shapes from sizes and settings.  Plain C++, so
-// that a host test can go through them without a device.
+// launch_rules.cuh -- rules that pick launch shapes and places from sizes and settings.  Plain
+// C++, so that a host test can go through them without a device.
 #pragma once
 
 #include <stdint.h>
+
+#ifdef __CUDACC__
+#define APBF_RULE __host__ __device__ __forceinline__
+#else
+#define APBF_RULE inline
+#endif
 
 namespace apbf {
 
@@ -15,7 +21,7 @@ struct PassShape {
 // returned, leaves the choice where it was.
 constexpr PassShape kAutomaticShape = {1u, 256u, 8u};
 
-inline PassShape pass_shape_rule(PassShape tuned, uint32_t capacity, bool features) {
+APBF_RULE PassShape pass_shape_rule(PassShape tuned, uint32_t capacity, bool features) {
     PassShape sh = tuned;
     const bool automatic = tuned.lanes == kAutomaticShape.lanes && tuned.block == kAutomaticShape.block &&
                            tuned.per_sm == kAutomaticShape.per_sm;
@@ -39,6 +45,15 @@ inline PassShape pass_shape_rule(PassShape tuned, uint32_t capacity, bool featur
         sh.per_sm = 8u;
     }
     return sh;
+}
+
+// Where a run of m entries starts in a pool of `size`, `before` entries having been asked of it
+// (kNoRun: it does not fit).  Rows that do not fit are counted too, and a list can hold more
+// than 2^32 entries: 64 bits, so that the count never comes round to places given away.
+using PoolCount = unsigned long long;
+constexpr uint32_t kNoRun = 0xffffffffu;
+APBF_RULE uint32_t pool_run(PoolCount before, uint32_t m, uint32_t size) {
+    return before <= size && m <= size - (uint32_t)before ? (uint32_t)before : kNoRun;
 }
 
 }  // namespace apbf

@@ -26,7 +26,6 @@
 #include <type_traits>
 
 #include "apbf_internal.cuh"
-#include "launch_rules.cuh"
 
 namespace apbf {
 namespace {
@@ -1127,12 +1126,11 @@ __global__ void __launch_bounds__(256) k_tile_rows(TileRowsArgs a) {
                 const uint32_t lane = threadIdx.x & 31u;
                 uint32_t at = 0;
                 if ((int)lane == src) {
-                    at = atomicAdd(a.plan.pool_used, m);
-                    if (at > a.plan.pool_size || m > a.plan.pool_size - at) at = 0xffffffffu;
+                    at = pool_run(atomicAdd(a.plan.pool_used, (PoolCount)m), m, a.plan.pool_size);
                     a.plan.tail[i] = at;
                 }
                 at = __shfl_sync(0xffffffffu, at, src);
-                if (at != 0xffffffffu)
+                if (at != kNoRun)
                     for (uint32_t k = lane; k < m; k += 32u)
                         a.plan.pool[at + k] = a.idx[(size_t)(kTileDepth + k) * a.stride + li];
             }
@@ -1253,8 +1251,8 @@ struct WarpRow {
         p.z = __shfl_sync(0xffffffffu, p_.z, src);
         p.w = 0;
         const uint32_t at = plan.tail[i];
-        entry = at != 0xffffffffu ? plan.pool + at : idx + (size_t)kTileDepth * row_stride + i;
-        stride = at != 0xffffffffu ? 1u : row_stride;
+        entry = at != kNoRun ? plan.pool + at : idx + (size_t)kTileDepth * row_stride + i;
+        stride = at != kNoRun ? 1u : row_stride;
     }
     template <typename G, typename F>
     __device__ __forceinline__ void each(G load, F f) const {
@@ -1339,7 +1337,7 @@ __global__ void __launch_bounds__(T *L, 1024 / (T * L)) k_density_tiles(PassA a,
             if (blockIdx.x == 0 && threadIdx.x == 0) {
                 a.st->filter_tag = (!skip && defer) ? 1u : 0u;
                 a.sync->cur_update = slot;
-                a.sync->pool_used[0] = a.sync->pool_used[1] = 0u;  // for the next substep's rows
+                a.sync->pool_used[0] = a.sync->pool_used[1] = 0ull;  // for the next substep's rows
             }
             if (skip || n == 0u) return;  // uniform over the grid
         }

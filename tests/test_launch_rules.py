@@ -15,6 +15,16 @@ extern "C" void pass_shape(const unsigned *t, unsigned capacity, int features, u
     out[1] = s.block;
     out[2] = s.per_sm;
 }
+// the places given to runs of m entries each, asked one after the other from `start` entries on
+extern "C" unsigned long long pool_places(unsigned long long start, unsigned runs, unsigned m, unsigned size) {
+    apbf::PoolCount used = start;
+    unsigned long long given = 0;
+    for (unsigned k = 0; k < runs; ++k) {
+        if (apbf::pool_run(used, m, size) != apbf::kNoRun) ++given;
+        used += m;
+    }
+    return given;
+}
 """
 
 
@@ -53,3 +63,11 @@ def test_given_shapes_are_taken(rules):
                 for cap in (2197, 50_000, 1_000_000):
                     assert _shape(rules, (lanes, block, per_sm), cap) == (lanes, block, per_sm)
                     assert _shape(rules, (lanes, block, per_sm), cap, features=True) == (1, block, per_sm)
+
+
+@pytest.mark.parametrize("m,size,runs", [(1000, 2_000_000, 5_000_000), (4_000_000, 1 << 29, 2000), (7, 0, 10), (1, 5, 9)])
+def test_pool_places_are_given_once(rules, m, size, runs):
+    """However many entries are asked for in all (here up to 8e9), the pool's own are given to
+    the first that fit and to nobody else."""
+    rules.pool_places.restype = C.c_ulonglong
+    assert rules.pool_places(C.c_ulonglong(0), C.c_uint(runs), C.c_uint(m), C.c_uint(size)) == min(runs, size // m)
