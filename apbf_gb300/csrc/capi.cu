@@ -372,6 +372,7 @@ apbf_status apbf_set_scene(apbf_ctx *ctx, const apbf_scene *scene) {
         set_error("apbf_set_scene: log2res must be in [1, max_log2res]");
         return APBF_ERR_INVALID_ARG;
     }
+    if (std::memcmp(&ctx->scene, scene, sizeof(*scene)) != 0) ctx->graph_version++;  // captured substeps hold it by value
     ctx->scene = *scene;
     return APBF_OK;
 }
