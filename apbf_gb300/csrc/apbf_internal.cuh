@@ -105,7 +105,6 @@ struct PassSync {
 // The neighbour rows of a substep rewritten for the tiled passes (solver.cu).
 constexpr int kTileHalo = 640;  // halo entries of a tile; one that fills it reads the list's own rows
 constexpr int kTileDepth = 64;  // row entries rewritten as offsets; the rest of a longer row goes to the pool
-constexpr uint32_t kTileSmallest = 64;  // particles of the smaller tile shape
 constexpr uint32_t kHaloOver = 0xffffffffu, kNoParticle = 0xffffffffu;
 struct TilePlan {
     uint32_t *halo;        // [tile * kTileHalo + slot]: particles outside the tile
@@ -225,7 +224,8 @@ struct apbf_ctx {
     uint32_t *inv_perm = nullptr;
     uint32_t *cells = nullptr;             // per cell: first particle; then per cell: end
     ulonglong2 *pos_code = nullptr;        // per particle: 96-bit position code {bits 0-63, bits 64-95}
-    ulonglong2 *bs_table = nullptr;        // cells of the binary-search rows (neighborhood_bs.cu)
+    ulonglong2 *bs_table = nullptr;        // cells of the binary-search rows (neighborhood_bs.cu; null: not made)
+    uint32_t *bs_levels = nullptr;         // the range of their radii's levels
     uint32_t *bs_counts = nullptr;         // 12 x 256: the particles' code digits
     uint32_t bs_slots = 0;                 // its slots, a power of two above the capacity
     int4 *srec = nullptr;                  // per particle: search record (position xyz, fixed-point radius)
@@ -272,7 +272,7 @@ struct apbf_ctx {
     uint32_t *t_keep = nullptr;    // per transfer: kept after particle_transfer
     uint32_t *t_scan = nullptr;    // per transfer: inclusive scan of t_keep
 
-    apbf::TilePlan tile_plan[2] = {};     // of the neighbour rows, of the transposed rows
+    apbf::TilePlan tile_plan[2] = {};     // of the neighbour rows, of the transposed rows (halo null: not made)
     apbf::PassSync *pass_sync = nullptr;  // density sums on their way to the position update
     double *red_partials = nullptr;
     double *red_out = nullptr;
@@ -495,11 +495,19 @@ struct SolveOpts {
     unsigned long long loop_handle = 0;  //   (the loop's conditional handle)
 };
 apbf_status incompressibility(apbf_ctx *ctx, cudaStream_t s, const SolveOpts &o = SolveOpts());
-// The tiled passes: whether the solve qualifies, and the rewriting of the rows the
-// search left (with the transposed rows too where the update may need them).
+// The tiled passes: whether the settings ask for them, whether a substep's position updates
+// may gather over transposed rows, whether the solve runs on tiles (its plans are there), and
+// the rewriting of the rows the search left (of the transposed rows too where needed).
 apbf_status tiles_prepare_device();  // kernel attributes on the current device
+bool tiles_wanted(const apbf_ctx *ctx);
+bool transposed_rows(const apbf_ctx *ctx);
 bool tiles_eligible(const apbf_ctx *ctx);
-apbf_status tile_rows(apbf_ctx *ctx, cudaStream_t s, bool transposed);
+apbf_status tile_rows(apbf_ctx *ctx, cudaStream_t s);
+// Scratch that only some uses need, made when the first of them is set up (settings, search
+// method) or called.  Whatever does not fit in device memory is left out: the solve then runs
+// the direct passes and the binary search searches its cells, with the same results.
+void make_tile_plans(apbf_ctx *ctx);
+void make_cell_table(apbf_ctx *ctx);
 // Passes 1.. of a substep as one persistent cooperative kernel with grid barriers
 // between the density and position phases; APBF_ERR_INVALID_ARG when the solve
 // does not qualify (then the caller uses the per-pass or graph forms).

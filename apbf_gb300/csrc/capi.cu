@@ -32,7 +32,61 @@ apbf_status dalloc(T **p, size_t count, std::vector<void *> &owned) {
     return APBF_OK;
 }
 
+// Makes the buffers named by `fill` (which calls dalloc with the list it is given) all or none,
+// on the context's device and whatever streams are being captured.
+template <typename F>
+bool make_all(apbf_ctx *ctx, F fill) {
+    int device = ctx->device;
+    cudaGetDevice(&device);
+    cudaSetDevice(ctx->device);
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    std::vector<void *> made;
+    const bool ok = fill(made);
+    if (ok) {
+        ctx->owned.insert(ctx->owned.end(), made.begin(), made.end());
+    } else {
+        for (void *p : made) cudaFree(p);
+        cudaGetLastError();
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    cudaSetDevice(device);
+    return ok;
+}
+
 }  // namespace
+
+// About 160 bytes per particle and plan (180 with rows above 64 entries), 18 more with the
+// smaller tiles.
+void make_tile_plans(apbf_ctx *ctx) {
+    if (!tiles_wanted(ctx)) return;
+    const uint32_t cap = ctx->cfg.particle_capacity, T = tile_particles(cap);
+    const size_t tiles = ((size_t)cap + T - 1u) / T;
+    for (int k = 0; k < (transposed_rows(ctx) ? 2 : 1); ++k) {
+        if (ctx->tile_plan[k].halo) continue;
+        TilePlan t = {};
+        t.pool_size = ctx->cfg.max_neighbors > (uint32_t)kTileDepth ? 2u * cap : 0u;
+        t.pool_used = &ctx->pass_sync->pool_used[k];
+        if (make_all(ctx, [&](std::vector<void *> &o) {
+                return dalloc(&t.halo, tiles * kTileHalo, o) == APBF_OK && dalloc(&t.tile, tiles, o) == APBF_OK &&
+                       dalloc(&t.lane, tiles * T, o) == APBF_OK &&
+                       dalloc(&t.rows, tiles * T * (kTileDepth / 4), o) == APBF_OK &&
+                       dalloc(&t.tail, cap, o) == APBF_OK && dalloc(&t.pool, t.pool_size, o) == APBF_OK;
+            }))
+            ctx->tile_plan[k] = t;
+    }
+}
+
+// 32 to 64 bytes per particle.
+void make_cell_table(apbf_ctx *ctx) {
+    if (ctx->bs_table) return;
+    uint32_t slots = 256u;
+    while (slots < 2u * ctx->cfg.particle_capacity) slots *= 2u;
+    ulonglong2 *table = nullptr;
+    if (!make_all(ctx, [&](std::vector<void *> &o) { return dalloc(&table, slots, o) == APBF_OK; })) return;
+    ctx->bs_table = table;
+    ctx->bs_slots = slots;
+}
 
 // gpu_list::set_length from a host value, stream-ordered (no synchronisation).
 __global__ void k_set_length(uint32_t *d_len, uint32_t slot, uint32_t v) { d_len[slot] = v; }
@@ -275,9 +329,8 @@ apbf_status apbf_create(const apbf_config *cfg, apbf_ctx **out) {
     const size_t ncells = (size_t)1 << (3 * cfg->max_log2res);
     A(ctx->cells, 2 * ncells);
     A(ctx->pos_code, cap);
-    for (ctx->bs_slots = 256u; ctx->bs_slots < 2u * cap;) ctx->bs_slots *= 2u;
-    A(ctx->bs_table, (size_t)ctx->bs_slots + 1u);
     A(ctx->bs_counts, 12 * 256);
+    A(ctx->bs_levels, 2);
     A(ctx->srec, cap);
     ctx->n_cells_log2_alloc = cfg->max_log2res;
     A(ctx->lambda, cap);
@@ -310,18 +363,6 @@ apbf_status apbf_create(const apbf_config *cfg, apbf_ctx **out) {
     A(ctx->red_partials, (size_t)6 * ctx->red_blocks);
     A(ctx->red_out, 4);
     A(ctx->pass_sync, 1);
-    for (int k = 0; k < 2; ++k) {
-        TilePlan &t = ctx->tile_plan[k];
-        const size_t whole = ((size_t)cap + 255u) / 256u * 256u;  // whole tiles of every shape
-        A(t.halo, whole / kTileSmallest * kTileHalo);
-        A(t.tile, whole / kTileSmallest);
-        A(t.lane, whole);
-        A(t.rows, whole * (kTileDepth / 4));
-        t.pool_size = cfg->max_neighbors > (uint32_t)kTileDepth ? 2u * cap : 0u;
-        A(t.tail, cap);
-        A(t.pool, t.pool_size);
-        t.pool_used = &ctx->pass_sync->pool_used[k];
-    }
     A(ctx->box_min, APBF_MAX_BOXES);
     A(ctx->box_max, APBF_MAX_BOXES);
     A(ctx->box_rot, 3 * APBF_MAX_BOXES);
@@ -363,6 +404,7 @@ apbf_status apbf_set_settings(apbf_ctx *ctx, const apbf_settings *s) {
     }
     ctx->settings = *s;
     ctx->graph_version++;  // solve loop graphs hold settings by value
+    make_tile_plans(ctx);
     return APBF_OK;
 }
 
@@ -708,7 +750,7 @@ apbf_status substep_body(apbf_ctx *ctx, float dt, cudaStream_t s, bool capture, 
     const bool tiles = tiles_eligible(ctx) && !(defer_loop && batch_solve_eligible(ctx, probe)) &&
                        !solve_persistent_eligible(ctx, probe);
     if (tiles) {
-        r = tile_rows(ctx, s, spread || ctx->search_method == APBF_NEIGHBORHOOD_BINARY_SEARCH);
+        r = tile_rows(ctx, s);
         if (r != APBF_OK) return r;
     }
     const bool loop_graph = ctx->use_graphs && !ctx->prof_on && !ctx->debug && !recording &&

@@ -117,8 +117,8 @@ constexpr uint32_t kTableLevel = 11;  // from this level on a cell number has at
 // Also: the transfer list follows the reorder, the first thread resets what the search
 // and the solve behind it count from, and the particles enter the cells of their radius's
 // level into the table (the first of a cell's run its start, the last its end).  The table
-// holds every cell when all radii have one level; the levels' range tells.  (table cleared,
-// levels {all ones, 0} beforehand.)
+// holds every cell when all radii have one level; the levels' range tells: 32 less the
+// lowest, and the highest.  (table and levels cleared beforehand.)
 __global__ void k_sorted_codes(const int4 *pos, const float *width, float scale, const uint32_t *d_len,
                                ulonglong2 *code, BsCell *table, uint32_t mask, uint32_t *levels, TransferBufs tr,
                                const uint32_t *inv_perm, Status *st, unsigned long long *total) {
@@ -127,19 +127,19 @@ __global__ void k_sorted_codes(const int4 *pos, const float *width, float scale,
     const uint32_t n = d_len[kLenParticles];
     if (blockIdx.x == 0 && threadIdx.x == 0) reset_search(st, total);
     remap_transfers(tr, inv_perm, d_len, st);
-    uint32_t kmin = 32u, kmax = 0u;
+    uint32_t low = 0u, high = 0u;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int4 p = pos[i];
         code[i] = code96((uint32_t)p.x, (uint32_t)p.y, (uint32_t)p.z);
         const long long R = range_fixed(width[i], scale);
         if (R < 0) {  // no cell of its own, but it may open or close another's run
-            kmin = 0u;
+            low = 32u;
             continue;
         }
         const uint32_t k = bs_level(R);
-        kmin = min(kmin, k);
-        kmax = max(kmax, k);
-        if (k < kTableLevel) continue;
+        low = max(low, 32u - k);
+        high = max(high, k);
+        if (k < kTableLevel || !table) continue;
         const uint32_t ux = (uint32_t)p.x >> k, uy = (uint32_t)p.y >> k, uz = (uint32_t)p.z >> k;
         const auto same = [&](int4 q) {
             return (uint32_t)q.x >> k == ux && (uint32_t)q.y >> k == uy && (uint32_t)q.z >> k == uz;
@@ -155,11 +155,11 @@ __global__ void k_sorted_codes(const int4 *pos, const float *width, float scale,
             break;
         }
     }
-    kmin = __reduce_min_sync(0xffffffffu, kmin);
-    kmax = __reduce_max_sync(0xffffffffu, kmax);
+    low = __reduce_max_sync(0xffffffffu, low);
+    high = __reduce_max_sync(0xffffffffu, high);
     if ((threadIdx.x & 31u) == 0u) {  // (a bound that already holds is left alone)
-        if (kmin < *(volatile uint32_t *)&levels[0]) atomicMin(&levels[0], kmin);
-        if (kmax > *(volatile uint32_t *)&levels[1]) atomicMax(&levels[1], kmax);
+        if (low > *(volatile uint32_t *)&levels[0]) atomicMax(&levels[0], low);
+        if (high > *(volatile uint32_t *)&levels[1]) atomicMax(&levels[1], high);
     }
 }
 
@@ -227,7 +227,7 @@ struct BsArgs {
     uint32_t *count, *idx;
     unsigned long long *total;
     Status *st;
-    const BsCell *table;  // k_sorted_codes' cells, mask + 1 slots
+    const BsCell *table;  // k_sorted_codes' cells, mask + 1 slots; null: no table
     uint32_t mask;
     const uint32_t *levels;
 };
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(kBuildThreads) k_bs_rows(BsArgs a) {
     grid_dependency_wait();
     grid_dependency_trigger();
     const uint32_t n = a.d_len[kLenParticles];
-    const bool tabled = a.levels[0] == a.levels[1] && a.levels[0] >= kTableLevel;
+    const bool tabled = a.table && 32u - a.levels[0] == a.levels[1] && a.levels[1] >= kTableLevel;
     Walk w(a.pos, a.idx, a.stride, a.maxn, s_row, false);
     const uint32_t gl = w.gl;
     unsigned long long local = 0;
@@ -336,13 +336,13 @@ apbf_status neighborhood_binary_search(apbf_ctx *ctx, float range_scale, cudaStr
     const uint32_t cap = ctx->cfg.particle_capacity;
     const int g = grid_for(ctx, cap);
     // three stable passes, least significant word first
-    // the table and behind it the levels' range {all ones, 0}: cleared ahead, so that from the
-    // sort on kernel follows kernel and each starts as the one before it ends
+    // the table and the levels' range, cleared ahead, so that from the sort on
+    // kernel follows kernel and each starts as the one before it ends
     BsCell *table = reinterpret_cast<BsCell *>(ctx->bs_table);
-    uint32_t *levels = reinterpret_cast<uint32_t *>(table + ctx->bs_slots);
+    uint32_t *levels = ctx->bs_levels;
     const bool behind = !ctx->in_batch;
-    APBF_CUDA(cudaMemsetAsync(table, 0, (size_t)ctx->bs_slots * sizeof(BsCell) + 2 * sizeof(uint32_t), s));
-    APBF_CUDA(cudaMemsetAsync(levels, 0xff, sizeof(uint32_t), s));
+    if (table) APBF_CUDA(cudaMemsetAsync(table, 0, (size_t)ctx->bs_slots * sizeof(BsCell), s));
+    APBF_CUDA(cudaMemsetAsync(levels, 0, 2 * sizeof(uint32_t), s));
     const bool counted = sort_takes_counts(ctx, cap);
     if (counted) APBF_CUDA(cudaMemsetAsync(ctx->bs_counts, 0, 12 * 256 * sizeof(uint32_t), s));
     for (uint32_t w = 0; w < 3; ++w) {
@@ -418,6 +418,11 @@ extern "C" {
 
 apbf_status apbf_neighborhood_binary_search_apply(apbf_ctx *ctx, float range_scale, void *stream) {
     if (!ctx) return APBF_ERR_INVALID_ARG;
+    if (!ctx->bs_table) {  // (nothing is made while the stream is captured)
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        APBF_CUDA(cudaStreamIsCapturing((cudaStream_t)stream, &st));
+        if (st == cudaStreamCaptureStatusNone) make_cell_table(ctx);
+    }
     return neighborhood_binary_search(ctx, range_scale, (cudaStream_t)stream);
 }
 
@@ -444,6 +449,8 @@ apbf_status apbf_set_neighborhood_search(apbf_ctx *ctx, int method) {
     }
     if (method != ctx->search_method) ctx->graph_version++;  // captured substeps hold the search
     ctx->search_method = method;
+    if (method == APBF_NEIGHBORHOOD_BINARY_SEARCH) make_cell_table(ctx);
+    make_tile_plans(ctx);
     return APBF_OK;
 }
 

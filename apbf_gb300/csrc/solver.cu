@@ -2279,13 +2279,10 @@ static PassShape pass_shape(const apbf_ctx *ctx, bool features, int *grid) {
     return sh;
 }
 
-// Calls f with the tile shape (particles, threads per particle) for the list: 128 x 1, or
-// 64 x 2 where 128 would leave SMs without a tile (2 197 particles: 294 us a frame with
-// 128 x 1, 285 with 64 x 2; from 30 000 particles on the larger tile is as fast or faster:
-// 1521 / 1509 us at 32 768, 2094 / 2570 at 119 771).
+// Calls f with the tile shape (particles, threads per particle) for the list.
 template <typename F>
 static void with_tile_shape(const apbf_ctx *ctx, F &&f) {
-    if (ctx->cfg.particle_capacity <= 24576u)
+    if (tile_particles(ctx->cfg.particle_capacity) == 64u)
         f(std::integral_constant<int, 64>(), std::integral_constant<int, 2>());
     else
         f(std::integral_constant<int, 128>(), std::integral_constant<int, 1>());
@@ -2294,13 +2291,24 @@ static void with_tile_shape(const apbf_ctx *ctx, F &&f) {
 // Rewriting the rows costs as much as about two passes gain by it, less where the passes
 // are short of warps anyway: at 250 000 particles 40 us against 23 us a pass, at 2 197
 // four passes are as fast with the direct kernels (273 against 285 us a frame).
-bool tiles_eligible(const apbf_ctx *ctx) {
+bool tiles_wanted(const apbf_ctx *ctx) {
     const apbf_settings &st = ctx->settings;
     return st.height_kernel_id == 1 && st.gradient_kernel_id == 1 && st.boundariness_calculation_method != 1 &&
            st.solver_iterations >= (ctx->cfg.particle_capacity >= 65536u ? 4 : 6);
 }
 
-apbf_status tile_rows(apbf_ctx *ctx, cudaStream_t s, bool transposed) {
+bool transposed_rows(const apbf_ctx *ctx) {
+    const apbf_settings &st = ctx->settings;
+    return ctx->search_method == APBF_NEIGHBORHOOD_BINARY_SEARCH ||
+           (!st.basic_pbf && !st.base_kernel_width_on_boundary_distance);
+}
+
+bool tiles_eligible(const apbf_ctx *ctx) {
+    return tiles_wanted(ctx) && ctx->tile_plan[0].halo && (!transposed_rows(ctx) || ctx->tile_plan[1].halo);
+}
+
+apbf_status tile_rows(apbf_ctx *ctx, cudaStream_t s) {
+    const bool transposed = transposed_rows(ctx);
     apbf_status r = APBF_OK;
     with_tile_shape(ctx, [&](auto tc, auto) {
         constexpr int T = decltype(tc)::value;
