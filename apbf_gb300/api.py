@@ -46,14 +46,22 @@ def device_tensor(ptr: int, shape: tuple, dtype: torch.dtype, device: int = 0) -
     return torch.as_tensor(_CudaArray(ptr, tuple(shape), _TYPESTR[dtype]), device=f"cuda:{device}")
 
 
+# torch's current stream and device as numbers (not part of its documented interface: None
+# where a torch build has no such function)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_raw_device = getattr(torch._C, "_cuda_getDevice", None)
+
+
 def _stream_handle(stream) -> C.c_void_p:
     """The stream's handle; None: torch's current stream of the current device, asked for as
-    a number (building the Stream object cost 3 us, a third of a stage call)."""
-    if stream is not None:
-        return C.c_void_p(stream.cuda_stream)
-    if not torch.cuda.is_initialized():
-        torch.cuda.init()
-    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    a number where torch can (building the Stream object cost 3 us, a third of a stage call)."""
+    if stream is None:
+        if _raw_stream is not None and _raw_device is not None:
+            if not torch.cuda.is_initialized():
+                torch.cuda.init()
+            return C.c_void_p(_raw_stream(_raw_device()))
+        stream = torch.cuda.current_stream()
+    return C.c_void_p(stream.cuda_stream)
 
 
 def default_settings() -> N.Settings:
