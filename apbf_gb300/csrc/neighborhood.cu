@@ -187,10 +187,10 @@ __global__ void k_corrections(BuildArgs a) {
 // in z, y, x order and their particles in list order.
 //
 // A thread per particle (as this kernel once was) is a chain of dependent loads, 120 us
-// however few the particles (now 10 us at 2 197, 39 at 32 768), and idles at 12 of 32 lanes
-// where their cells differ in length (250 000: 260 against 185 us, a million: 795 against
-// 606; bound by instruction issue).  Here a group's threads load the ranges of G pairs of
-// cells at once and then test the joined ranges together (RowWalk).
+// however few the particles (now 12 us at 2 197, 39 at 32 768), and idles at 12 of 32 lanes
+// where their cells differ in length (the drop of 250 000: 260 against 176 us, the waterfall's
+// million: 795 against 576; bound by instruction issue).  Here a group's threads load the
+// ranges of G pairs of cells at once and then test the joined ranges together (RowWalk).
 //
 // Correction rows (uni, when the search radii differ): the position update of
 // particle i sums over the particles k whose rows hold i (|x_i - x_k| <= R_k),
@@ -210,15 +210,44 @@ struct SmallDiv {
     }
 };
 
+// The cells of a particle's box axis by axis: pairs along x, then cells along y and z.
+struct CellBox {
+    uint32_t x0, y0, z0, nx, ny;
+    bool inside;  // the box touches no edge cell of the grid
+};
+// Cell e of that list: how far the particle is from it along its axis (0 when the box is not
+// inside the grid) and its share of the key.
+__device__ __forceinline__ uint2 axis_cell(const Bounds &b, uint32_t L, const CellBox &box, int4 p, uint32_t e) {
+    const uint32_t d = e < box.nx ? 0u : e < box.nx + box.ny ? 1u : 2u;
+    const uint32_t c = d == 0u ? 2u * ((box.x0 >> 1) + e) : d == 1u ? box.y0 + (e - box.nx) : box.z0 + (e - box.nx - box.ny);
+    uint32_t gap = 0u;
+    if (box.inside) {
+        const int x = d == 0u ? p.x : d == 1u ? p.y : p.z;
+        const long long lo64 = d == 0u ? b.lo[0] : d == 1u ? b.lo[1] : b.lo[2];
+        const uint32_t span = (uint32_t)((d == 0u ? b.hi[0] : d == 1u ? b.hi[1] : b.hi[2]) - lo64);
+        const int lo = (int)lo64;
+        const int first = lo + (int)(((unsigned long long)c * span) >> L),
+                  behind = lo + (int)(((unsigned long long)(c + (d == 0u ? 2u : 1u)) * span) >> L);
+        gap = (uint32_t)max(max(first - x, x - behind), 0);
+    }
+    return make_uint2(gap, spread3(c) << d);
+}
+
 // The cells are taken in pairs along x: cells 2k and 2k + 1 have neighbouring keys, so their
 // particles are one run, in the order the cells would give.  Pairs that lie beyond the
 // radius (a lower bound of the distance from the pair's box) bring nothing; a quarter of
 // the candidates are in such cells.
+// A pair's distance and key come from a table of the box's cells per axis: worked out anew for
+// every pair they were half of a sparse list's instructions (a million particles with 14
+// neighbours each 825 us, 640 with the table; with 6 each 507 and 428; the thread per particle
+// took 745 and 364).  The table holds boxes of up to 17 cells an axis; larger ones do without.
+constexpr uint32_t kAxisCells = 48;  // cells along x (pairs), y and z together
 template <int G>
 __global__ void __launch_bounds__(kBuildThreads, 6) k_build_rows(BuildArgs a) {
     constexpr uint32_t P = RowWalk<G>::kParticles;
     __shared__ uint32_t s_row[kRowStage * RowWalk<G>::kPad];
     __shared__ uint32_t s_cnt[P];
+    __shared__ uint2 s_axis[P * kAxisCells];
     grid_dependency_wait();
     grid_dependency_trigger();
     const uint32_t n = a.d_len[kLenParticles];
@@ -255,7 +284,11 @@ __global__ void __launch_bounds__(kBuildThreads, 6) k_build_rows(BuildArgs a) {
         w.start(i, p, (uint32_t)max(p.w, 0));
         const bool big = npair >= (1u << 22);
         const SmallDiv by_x(nx), by_y(ny);
-        // gap of a coordinate to cells [c, e) of an axis (inside the grid)
+        const CellBox box = {x0, y0, z0, nx, ny, fast};
+        uint2 *axis = s_axis + w.slot * kAxisCells;
+        const uint32_t ncells = npair == 0u ? 0u : nx + ny + nz;
+        const uint32_t most = __reduce_max_sync(0xffffffffu, npair);  // the warp's groups go on together
+        // gap of a coordinate to cells [c, e) of an axis (inside the grid), where the table is too short
         const auto gap = [&](int x, int d, uint32_t c, uint32_t e) {
             const uint32_t span = (uint32_t)(a.b.hi[d] - a.b.lo[d]);
             const int lo = (int)a.b.lo[d];
@@ -263,31 +296,51 @@ __global__ void __launch_bounds__(kBuildThreads, 6) k_build_rows(BuildArgs a) {
                       behind = lo + (int)(((unsigned long long)e * span) >> a.L);
             return (uint32_t)max(max(first - x, x - behind), 0);
         };
-        const auto range = [&](uint32_t c, uint32_t &s, uint32_t &len) {  // of the c-th pair of the box
-            s = len = 0u;
-            if (c >= npair) return;
-            const uint32_t t = by_x(c, big), u = by_y(t, big);
-            const uint32_t cx = 2u * ((x0 >> 1) + (c - t * nx)), cy = y0 + (t - u * ny), cz = z0 + u;
-            if (all_fast) {
-                const uint32_t gx = gap(p.x, 0, cx, cx + 2u), gy = gap(p.y, 1, cy, cy + 1u), gz = gap(p.z, 2, cz, cz + 1u);
+        const auto walk = [&](auto tabled) {
+            const auto range = [&](uint32_t c, uint32_t &s, uint32_t &len) {  // of the c-th pair of the box
+                s = len = 0u;
+                if (c >= npair) return;
+                const uint32_t t = by_x(c, big), u = by_y(t, big), ix = c - t * nx, iy = t - u * ny;
+                const uint32_t cx = 2u * ((x0 >> 1) + ix);
+                uint32_t gx = 0u, gy = 0u, gz = 0u, key;
+                if (decltype(tabled)::value) {
+                    const uint2 ex = axis[ix], ey = axis[nx + iy], ez = axis[nx + ny + u];
+                    gx = ex.x;
+                    gy = ey.x;
+                    gz = ez.x;
+                    key = ex.y | ey.y | ez.y;
+                } else {
+                    const uint32_t cy = y0 + iy, cz = z0 + u;
+                    if (all_fast) {
+                        gx = gap(p.x, 0, cx, cx + 2u);
+                        gy = gap(p.y, 1, cy, cy + 1u);
+                        gz = gap(p.z, 2, cz, cz + 1u);
+                    }
+                    key = morton3(cx, cy, cz);
+                }
                 if ((unsigned long long)gx * gx + (unsigned long long)gy * gy + (unsigned long long)gz * gz > w.R2) return;
+                const uint2 st = *reinterpret_cast<const uint2 *>(a.cstart + key), en = *reinterpret_cast<const uint2 *>(a.cend + key);
+                const uint32_t n0 = cx >= x0 ? en.x - st.x : 0u, n1 = cx + 1u <= x1 ? en.y - st.y : 0u;
+                s = n0 ? st.x : st.y;
+                len = n0 + n1;
+            };
+            uint32_t s, len;
+            range(gl, s, len);
+            for (uint32_t c0 = 0; c0 < most; c0 += G) {
+                uint32_t ns, nlen;
+                range(c0 + G + gl, ns, nlen);  // in flight while this round's candidates are tested
+                if (all_fast) w.template take<true>(s, len);
+                else w.template take<false>(s, len);
+                s = ns;
+                len = nlen;
             }
-            const uint32_t key = morton3(cx, cy, cz);
-            const uint2 st = *reinterpret_cast<const uint2 *>(a.cstart + key), en = *reinterpret_cast<const uint2 *>(a.cend + key);
-            const uint32_t n0 = cx >= x0 ? en.x - st.x : 0u, n1 = cx + 1u <= x1 ? en.y - st.y : 0u;
-            s = n0 ? st.x : st.y;
-            len = n0 + n1;
         };
-        const uint32_t most = __reduce_max_sync(0xffffffffu, npair);  // the warp's groups go on together
-        uint32_t s, len;
-        range(gl, s, len);
-        for (uint32_t c0 = 0; c0 < most; c0 += G) {
-            uint32_t ns, nlen;
-            range(c0 + G + gl, ns, nlen);  // in flight while this round's candidates are tested
-            if (all_fast) w.template take<true>(s, len);
-            else w.template take<false>(s, len);
-            s = ns;
-            len = nlen;
+        if (__all_sync(0xffffffffu, ncells <= kAxisCells)) {
+            for (uint32_t e = gl; e < ncells; e += G) axis[e] = axis_cell(a.b, a.L, box, p, e);
+            __syncwarp();
+            walk(std::true_type());
+        } else {
+            walk(std::false_type());
         }
         if (uni) {
             const uint32_t one_sided = group_total<G>(w.one_sided);

@@ -110,12 +110,17 @@ struct RowWalk {
             return __shfl_sync(0xffffffffu, adj, k, G) + f;
         };
         for (uint32_t w = 0; w < rounds; w += 2 * G) {  // two candidates of each thread in flight
-            const uint32_t f0 = w + gl, f1 = f0 + G;
-            const uint32_t j0 = candidate(f0), j1 = candidate(f1);
+            const uint32_t f0 = w + gl, f1 = f0 + G, j0 = candidate(f0);
             const bool in0 = f0 < total, in1 = f1 < total;
-            const int4 q0 = in0 ? rec[j0] : p, q1 = in1 ? rec[j1] : p;
-            test<FAST>(in0, j0, q0);
-            test<FAST>(in1, j1, q1);
+            const int4 q0 = in0 ? rec[j0] : p;
+            if (w + G < rounds) {
+                const uint32_t j1 = candidate(f1);
+                const int4 q1 = in1 ? rec[j1] : p;
+                test<FAST>(in0, j0, q0);
+                test<FAST>(in1, j1, q1);
+            } else {  // (of short runs, as sparse lists have, the last round holds one)
+                test<FAST>(in0, j0, q0);
+            }
         }
     }
     // The block's rows, entries [0, s_cnt[slot]) of each (after a barrier behind the walks).
