@@ -1467,9 +1467,9 @@ __global__ void __launch_bounds__(T *L, 1024 / (T * L)) k_density_tiles(PassA a,
                     for (uint32_t u = 0; u < 4; ++u)
                         hit = hit || gauss_filter_hit(ed, fdiff(p, tile_record(s_pos, row_offset(now, u))));
                 }
-                if (!hit)
-                    lane_row<1>(a.idx + i, a.stride, depth, end, [&](uint32_t j) { return a.pos[j]; },
-                                [&](uint32_t, const int4 &q) { hit = hit || gauss_filter_hit(ed, fdiff(p, q)); });
+#pragma unroll 2
+                for (uint32_t k = depth; k < end && !hit; ++k)
+                    hit = gauss_filter_hit(ed, fdiff(p, a.pos[a.idx[(size_t)k * a.stride + i]]));
             }
             for (uint32_t left = __ballot_sync(0xffffffffu, ask && !hit && by_warp); left; left &= left - 1u) {
                 const int src = __ffs(left) - 1;
