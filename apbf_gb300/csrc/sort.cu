@@ -10,7 +10,7 @@
 // the keys; then one kernel per 8-bit digit ranks a tile of 2048 keys (8 warps x
 // 8 keys per lane, warp-striped so loads coalesce), publishes the tile's digit
 // counts, looks back over earlier tiles for its global offsets and writes the tile
-// out digit by digit.  A list of at most 16 384 pairs takes one block (k_sort_small).
+// out digit by digit.  A list of at most 4 096 pairs takes one block (k_sort_small).
 // Stability: inside a warp the keys are ranked in index order by votes; warps are combined in index order; tiles in tile order.
 // Every wait on another tile is bounded (kSpinLimit) and records
 // APBF_FLAG_SPIN_LIMIT instead of hanging.
@@ -350,46 +350,46 @@ __global__ void __launch_bounds__(kSortThreads) k_digit_scatter(const uint32_t *
 constexpr uint32_t kWaitFree = 1u << 18;
 
 // Every 8-bit pass of a short list in one block: the pairs stay in registers and shared
-// memory between the passes.  One launch (12 us at 2 197 pairs of 21 bits, 35 us before)
-// instead of a histogram, three clears and a launch per digit, whose latencies are all that a
-// short sort costs.
-template <int THREADS, int ITEMS>
+// memory between the passes.  One launch (14 us at 4 096 pairs of 21 bits, 44 us before)
+// instead of a histogram, a clear and a launch per digit, whose latencies are all that a
+// short sort costs.  With four times the threads and pairs it took 41 us at 5 000 pairs and 49
+// at 16 384, the overlapped tiles 23 and 25.
+constexpr int kSmallThreads = 256, kSmallItems = 16;
+constexpr uint32_t kSmallKeys = kSmallThreads * kSmallItems;
 struct SmallSort {
-    static constexpr uint32_t kKeys = THREADS * ITEMS;
-    uint32_t keys[kKeys], vals[kKeys];
-    uint16_t cnt[THREADS / 32][256];
+    uint32_t keys[kSmallKeys], vals[kSmallKeys];
+    uint16_t cnt[kSmallThreads / 32][256];
     uint32_t off[256], part[8];
 };
-template <int THREADS, int ITEMS>
-__global__ void __launch_bounds__(THREADS) k_sort_small(const uint32_t *kin, const uint32_t *vin, uint32_t *kout,
+__global__ void __launch_bounds__(kSmallThreads) k_sort_small(const uint32_t *kin, const uint32_t *vin, uint32_t *kout,
                                                         uint32_t *vout, const uint32_t *d_count, uint32_t max_count,
                                                         uint32_t key_mask, int passes) {
     extern __shared__ unsigned char s_raw[];
-    SmallSort<THREADS, ITEMS> &s = *reinterpret_cast<SmallSort<THREADS, ITEMS> *>(s_raw);
+    SmallSort &s = *reinterpret_cast<SmallSort *>(s_raw);
     grid_dependency_wait();
     grid_dependency_trigger();
     const uint32_t t = threadIdx.x, w = t >> 5, l = t & 31u;
     const uint32_t n = min(*d_count, max_count);
-    uint32_t keys[ITEMS], vals[ITEMS], digit[ITEMS], rank[ITEMS];
+    uint32_t keys[kSmallItems], vals[kSmallItems], digit[kSmallItems], rank[kSmallItems];
 #pragma unroll
-    for (int k = 0; k < ITEMS; ++k) {
-        const uint32_t idx = w * (32 * ITEMS) + k * 32 + l;
+    for (int k = 0; k < kSmallItems; ++k) {
+        const uint32_t idx = w * (32 * kSmallItems) + k * 32 + l;
         keys[k] = idx < n ? kin[idx] : 0u;
         vals[k] = idx < n ? vin[idx] : 0u;
     }
     for (int p = 0; p < passes; ++p) {
-        for (uint32_t k = t; k < THREADS / 32 * 128; k += THREADS) reinterpret_cast<uint32_t *>(&s.cnt[0][0])[k] = 0u;
+        for (uint32_t k = t; k < kSmallThreads / 32 * 128; k += kSmallThreads) reinterpret_cast<uint32_t *>(&s.cnt[0][0])[k] = 0u;
         __syncthreads();
 #pragma unroll
-        for (int k = 0; k < ITEMS; ++k) {
-            const uint32_t idx = w * (32 * ITEMS) + k * 32 + l;
+        for (int k = 0; k < kSmallItems; ++k) {
+            const uint32_t idx = w * (32 * kSmallItems) + k * 32 + l;
             digit[k] = idx < n ? ((keys[k] & key_mask) >> (8 * p)) & 255u : 256u + l;
         }
         rank_digits<256u>(digit, rank, s.cnt[w]);
         __syncthreads();
         uint32_t run = 0;
         if (t < 256u)
-            for (int k = 0; k < THREADS / 32; ++k) {
+            for (int k = 0; k < kSmallThreads / 32; ++k) {
                 const uint32_t c = s.cnt[k][t];
                 s.cnt[k][t] = (uint16_t)run;
                 run += c;
@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(THREADS) k_sort_small(const uint32_t *kin, con
         if (t < 256u) s.off[t] = off;
         __syncthreads();
 #pragma unroll
-        for (int k = 0; k < ITEMS; ++k) {
+        for (int k = 0; k < kSmallItems; ++k) {
             if (digit[k] >= 256u) continue;
             const uint32_t pos = s.off[digit[k]] + s.cnt[w][digit[k]] + rank[k];
             s.keys[pos] = keys[k];
@@ -406,8 +406,8 @@ __global__ void __launch_bounds__(THREADS) k_sort_small(const uint32_t *kin, con
         }
         __syncthreads();
 #pragma unroll
-        for (int k = 0; k < ITEMS; ++k) {
-            const uint32_t idx = w * (32 * ITEMS) + k * 32 + l;
+        for (int k = 0; k < kSmallItems; ++k) {
+            const uint32_t idx = w * (32 * kSmallItems) + k * 32 + l;
             if (idx >= n) continue;
             keys[k] = s.keys[idx];
             vals[k] = s.vals[idx];
@@ -418,8 +418,6 @@ __global__ void __launch_bounds__(THREADS) k_sort_small(const uint32_t *kin, con
         }
     }
 }
-using SmallSort4k = SmallSort<256, 16>;
-using SmallSort16k = SmallSort<1024, 16>;
 
 // Single-pass inclusive scan with decoupled look-back; tile = 256 threads x 16.
 constexpr int kScanItems = 16;
@@ -512,10 +510,7 @@ __global__ void __launch_bounds__(256) k_scan(uint32_t *data, const uint32_t *d_
 
 constexpr int kSortCarveout = 75;  // percent
 apbf_status sort_prepare_device() {
-    APBF_CUDA(cudaFuncSetAttribute(k_sort_small<256, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)sizeof(SmallSort4k)));
-    APBF_CUDA(cudaFuncSetAttribute(k_sort_small<1024, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)sizeof(SmallSort16k)));
+    APBF_CUDA(cudaFuncSetAttribute(k_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmallSort)));
     // kernels that overlap want the same split of an SM's memory, or it drains between them
     APBF_CUDA(cudaFuncSetAttribute(k_digit_count<8>, cudaFuncAttributePreferredSharedMemoryCarveout, kSortCarveout));
     APBF_CUDA(cudaFuncSetAttribute(k_digit_scatter<8>, cudaFuncAttributePreferredSharedMemoryCarveout, kSortCarveout));
@@ -539,7 +534,7 @@ static apbf_status launch_hist(apbf_ctx *ctx, const uint32_t *keys_in, const uin
 
 bool sort_takes_counts(const apbf_ctx *ctx, uint32_t max_count) {
     const uint32_t d = ctx->tuning.sort_digit_bits;
-    return d != 6u && d != 7u && max_count > SmallSort16k::kKeys && max_count <= kWaitFree;
+    return d != 6u && d != 7u && max_count > kSmallKeys && max_count <= kWaitFree;
 }
 
 // Stable sort by the low key_bits bits of the keys (rounded up to whole 4-bit
@@ -567,14 +562,10 @@ apbf_status sort_pairs_device(apbf_ctx *ctx, const uint32_t *keys_in, const uint
         APBF_CUDA(cudaMemcpyAsync(vals_out, vals_in, (size_t)max_count * 4, cudaMemcpyDeviceToDevice, s));
         return APBF_OK;
     }
-    if (dbits == 8u && max_count <= SmallSort16k::kKeys) {
+    if (dbits == 8u && max_count <= kSmallKeys) {
         APBF_BEFORE_LAUNCH(ctx, s, "k_sort_small");
-        if (max_count <= SmallSort4k::kKeys)
-            APBF_CUDA(launch_behind(behind_kernel && !ctx->in_batch, k_sort_small<256, 16>, 1, 256, sizeof(SmallSort4k), s, keys_in,
-                                    vals_in, keys_out, vals_out, d_count, max_count, key_mask, passes));
-        else
-            APBF_CUDA(launch_behind(behind_kernel && !ctx->in_batch, k_sort_small<1024, 16>, 1, 1024, sizeof(SmallSort16k), s, keys_in,
-                                    vals_in, keys_out, vals_out, d_count, max_count, key_mask, passes));
+        APBF_CUDA(launch_behind(behind_kernel && !ctx->in_batch, k_sort_small, 1, kSmallThreads, sizeof(SmallSort), s, keys_in,
+                                vals_in, keys_out, vals_out, d_count, max_count, key_mask, passes));
         APBF_AFTER_LAUNCH(ctx, s, "k_sort_small");
         return APBF_OK;
     }

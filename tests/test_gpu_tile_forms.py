@@ -118,3 +118,30 @@ def test_tiles_equal_direct_passes(capacity, case, filter_in_density):
         for k in want:
             assert got[k].tobytes() == want[k].tobytes(), (mode, k)
         ctx.close()
+
+
+def test_blocks_that_take_a_second_tile():
+    """More tiles than the passes have blocks (152 x 64): each block goes on to another tile."""
+    from apbf_gb300.api import Context, SubstepStages
+
+    side = 110
+    n = side ** 3
+    rng = np.random.default_rng(1)
+    st = scenes.make_state(scenes.lattice([4.0, 4.0, 4.0], [side] * 3, 1.9, 0.3, rng))
+    st["kernel_width"] = (st["kernel_width"] * rng.uniform(0.9, 1.1, size=n)).astype(np.float32)
+    out = []
+    for fused in (True, False):
+        ctx = Context(particle_capacity=n, max_neighbors=96, max_log2res=6)
+        ctx.set_settings(basic_pbf=1, solver_iterations=4)
+        ctx.set_scene((-4.0,) * 3, (252.0,) * 3, 6, (0.0, -392.4, 0.0))
+        ctx.set_boxes(np.array([[-2.0, -2.0, -2.0, 0.0]], np.float32), np.array([[250.0, 5.0, 250.0, 0.0]], np.float32))
+        ctx.upload(st)
+        if fused:
+            ctx.substep(DT)
+        else:
+            SubstepStages(ctx).update(DT)
+        ctx.check_status()
+        out.append(ctx.download()[0])
+        ctx.close()
+    for k in out[0]:
+        assert out[0][k].tobytes() == out[1][k].tobytes(), k
