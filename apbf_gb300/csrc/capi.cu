@@ -604,6 +604,7 @@ apbf_status apbf_fluid_write(apbf_ctx *ctx, const apbf_host_fluid *in, uint32_t 
     }
     cudaSetDevice(ctx->device);
     cudaStream_t s = (cudaStream_t)stream;
+    APBF_BOUND_LENGTHS(ctx, s);
     const FluidBufs &f = ctx->fl[ctx->fcur];
     void *const dev[] = {f.pos, f.vel, f.inv_mass, f.radius, f.pos_backup, f.transferring, f.target_radius,
                          f.kernel_width, f.boundariness, f.boundary_distance, f.lambda_prev};
@@ -619,6 +620,7 @@ apbf_status apbf_fluid_read(apbf_ctx *ctx, apbf_host_fluid *out, uint32_t max_co
     if (!ctx || !out || !h_count) return APBF_ERR_INVALID_ARG;
     cudaSetDevice(ctx->device);
     cudaStream_t s = (cudaStream_t)stream;
+    APBF_BOUND_LENGTHS(ctx, s);
     const FluidBufs &f = ctx->fl[ctx->fcur];
     const size_t n = std::min(max_count, ctx->cfg.particle_capacity);
     APBF_CUDA(cudaMemcpyAsync(h_count, ctx->d_len + kLenParticles, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));

@@ -197,6 +197,7 @@ extern "C" apbf_status apbf_sphere_collision_apply(apbf_ctx *ctx, const float ce
                                                    void *stream) {
     if (!ctx || !center) return APBF_ERR_INVALID_ARG;
     cudaStream_t s = (cudaStream_t)stream;
+    APBF_BOUND_LENGTHS(ctx, s);
     FluidBufs &f = ctx->fl[ctx->fcur];
     APBF_BEFORE_LAUNCH(ctx, s, "k_sphere_collision");
     k_sphere_collision<<<grid_for(ctx, ctx->cfg.particle_capacity), kBlock, 0, s>>>(
@@ -208,6 +209,7 @@ extern "C" apbf_status apbf_sphere_collision_apply(apbf_ctx *ctx, const float ce
 extern "C" apbf_status apbf_inter_particle_collision_apply(apbf_ctx *ctx, void *stream) {
     if (!ctx) return APBF_ERR_INVALID_ARG;
     cudaStream_t s = (cudaStream_t)stream;
+    APBF_BOUND_LENGTHS(ctx, s);
     const uint32_t cap = ctx->cfg.particle_capacity;
     FluidBufs &f = ctx->fl[ctx->fcur];
     FluidBufs &alt = ctx->fl[ctx->fcur ^ 1];
@@ -227,6 +229,7 @@ extern "C" apbf_status apbf_inter_particle_collision_apply(apbf_ctx *ctx, void *
 extern "C" apbf_status apbf_glue_generate(apbf_ctx *ctx, uint32_t capacity, void *stream) {
     if (!ctx || !capacity) return APBF_ERR_INVALID_ARG;
     cudaStream_t s = (cudaStream_t)stream;
+    APBF_BOUND_LENGTHS(ctx, s);
     const uint32_t cap = ctx->cfg.particle_capacity;
     if (capacity > ctx->glue_cap) {  // the glue list grows on demand, like a gpu_list request
         APBF_CUDA(cudaStreamSynchronize(s));

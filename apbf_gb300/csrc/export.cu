@@ -20,6 +20,7 @@ extern "C" apbf_status apbf_save_particle_info(apbf_ctx *ctx, const char *folder
     if (!ctx || !folder || !center) return APBF_ERR_INVALID_ARG;
     cudaSetDevice(ctx->device);
     cudaStream_t s = (cudaStream_t)stream;
+    APBF_BOUND_LENGTHS(ctx, s);
     uint32_t n = 0;
     APBF_CUDA(cudaMemcpyAsync(&n, ctx->d_len + kLenParticles, sizeof(n), cudaMemcpyDeviceToHost, s));
     APBF_CUDA(cudaStreamSynchronize(s));

@@ -15,6 +15,7 @@
 // roles at capture time (current fluid set, current position buffer), the pass
 // limit and the solve modes; up to four are cached per context and every change of
 // settings or boxes drops them.
+#include <deque>
 #include <vector>
 
 #include "apbf_internal.cuh"
@@ -378,6 +379,11 @@ extern "C" apbf_status apbf_batch_substep(apbf_batch *b, float dt, void *stream)
             if (r != APBF_OK) return r;
         }
         return APBF_OK;
+    }
+    std::deque<BoundLengths> lengths;  // of contexts whose lists are the caller's: in before the graph, out after it
+    for (auto *c : b->ctx) {
+        lengths.emplace_back(c, s);
+        if (lengths.back().status != APBF_OK) return lengths.back().status;
     }
     std::vector<HostState> before(n);
     std::vector<unsigned long long> version(n), mode(n);

@@ -423,6 +423,7 @@ apbf_status apbf_neighborhood_binary_search_apply(apbf_ctx *ctx, float range_sca
         APBF_CUDA(cudaStreamIsCapturing((cudaStream_t)stream, &st));
         if (st == cudaStreamCaptureStatusNone) make_cell_table(ctx);
     }
+    APBF_BOUND_LENGTHS(ctx, (cudaStream_t)stream);
     return neighborhood_binary_search(ctx, range_scale, (cudaStream_t)stream);
 }
 
@@ -433,6 +434,7 @@ apbf_status apbf_calculate_position_code(apbf_ctx *ctx, const uint32_t *d_index_
         return APBF_ERR_INVALID_ARG;
     }
     cudaStream_t s = (cudaStream_t)stream;
+    APBF_BOUND_LENGTHS(ctx, s);
     const FluidBufs &f = ctx->fl[ctx->fcur];
     APBF_BEFORE_LAUNCH(ctx, s, "k_code_word");
     k_code_word<<<grid_for(ctx, ctx->cfg.particle_capacity), kBlock, 0, s>>>(f.pos, ctx->d_len, code_section,

@@ -65,6 +65,7 @@ extern "C" apbf_status apbf_autotune(apbf_ctx *ctx, void *stream, apbf_tuning *c
     if (!ctx) return APBF_ERR_INVALID_ARG;
     cudaSetDevice(ctx->device);
     cudaStream_t s = (cudaStream_t)stream;
+    APBF_BOUND_LENGTHS(ctx, s);
     const size_t cap = ctx->cfg.particle_capacity;
     FluidBufs &f = ctx->fl[ctx->fcur];
     // save what the passes change: positions, boundariness, the status block
@@ -171,6 +172,7 @@ extern "C" apbf_status apbf_autotune_search(apbf_ctx *ctx, void *stream, apbf_tu
     }
     cudaSetDevice(ctx->device);
     cudaStream_t s = (cudaStream_t)stream;
+    APBF_BOUND_LENGTHS(ctx, s);
     const uint32_t cap = ctx->cfg.particle_capacity, tcap = ctx->cfg.transfer_capacity;
     const apbf_tuning before = ctx->tuning;
     const uint32_t L0 = before.search_log2res ? before.search_log2res : ctx->scene.log2res;
