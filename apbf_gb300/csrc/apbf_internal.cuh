@@ -486,7 +486,7 @@ struct SolveOpts {
     bool learned = false;     // the network's lambda replaces the computed one in this update
     int prev_mode = 0;        // lambda_prev: 0 off, 1 reset, 2 add the applied lambda
     bool projected = false;   // with prev_mode 2: pull-back up to the substep's accumulated push
-    bool later_pass = false;  // not the first pass of a substep (the widths' uniformity is known)
+    bool later_pass = false;  // not the first pass of a substep
     bool behind = true;       // a pass behind another one's position update in the stream
     bool tiles = false;       // over the tiles of tile_rows (the substep's rows, unchanged since)
     int loop_offset = -1;     // >= 0: a pass of the solve loop graph, number = pass_start + offset;
@@ -797,19 +797,6 @@ __device__ __forceinline__ long long range_fixed(float kw, float scale) {
     if (!(r >= 0.0)) return -1;
     if (r > 2147483647.0) r = 2147483647.0;
     return (long long)floor(r);
-}
-
-// |b - a|^2 <= R^2 exactly.  Once every |d| <= R < 2^31 is known, each square is
-// one 32x32 -> 64-bit multiply and the sum cannot overflow 64 bits.
-__device__ __forceinline__ bool within(int4 a, int4 b, long long R) {
-    long long dx = (long long)b.x - a.x, dy = (long long)b.y - a.y, dz = (long long)b.z - a.z;
-    dx = dx < 0 ? -dx : dx;
-    dy = dy < 0 ? -dy : dy;
-    dz = dz < 0 ? -dz : dz;
-    if (dx > R || dy > R || dz > R) return false;
-    const uint32_t ux = (uint32_t)dx, uy = (uint32_t)dy, uz = (uint32_t)dz, ur = (uint32_t)R;
-    unsigned long long s = (unsigned long long)ux * ux + (unsigned long long)uy * uy + (unsigned long long)uz * uz;
-    return s <= (unsigned long long)ur * ur;
 }
 
 

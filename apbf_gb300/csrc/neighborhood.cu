@@ -127,11 +127,9 @@ __global__ void k_cell_ranges(const uint32_t *skeys, const uint32_t *d_len, uint
 struct BuildArgs {
     const int4 *pos;
     int4 *pos_box;  // when non-null: receives box_collision(pos) (the first Jacobi iteration's box pass)
-    const float *range;
     const float *radius;
     const float4 *bmin, *bmax, *rot;
     uint32_t nboxes;
-    float scale;
     const uint32_t *d_len;
     Bounds b;
     uint32_t L;
@@ -490,13 +488,11 @@ apbf_status neighborhood_green(apbf_ctx *ctx, float range_scale, const float min
     ba.pos = f.pos;
     FluidBufs &spare = ctx->fl[ctx->fcur ^ 1];
     ba.pos_box = fuse_box ? spare.pos : nullptr;
-    ba.range = f.kernel_width;
     ba.radius = f.radius;
     ba.bmin = ctx->box_min;
     ba.bmax = ctx->box_max;
     ba.rot = ctx->box_rot;
     ba.nboxes = ctx->n_boxes;
-    ba.scale = range_scale;
     ba.d_len = ctx->d_len;
     ba.b = b;
     ba.L = L;

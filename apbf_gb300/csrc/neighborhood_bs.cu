@@ -8,10 +8,11 @@
 //     calculate_position_code.comp:22-72).
 //  2. reorder_particles: gather every attribute, remap the transfer and glue lists
 //     (neighborhood_binary_search.cpp:49-50).
-//  3. k_sorted_codes: the codes of the sorted particles (:52-56).
+//  3. k_sorted_codes: the codes of the sorted particles (:52-56), and the cells of their
+//     radii's level into a hash table.
 //  4. k_bs_rows: per particle, the 27 cells of edge 2^k around its own cell; each
-//     cell's particles are one run of the sorted codes, found by a lower-bound search
-//     (neighborhood_binary_search.comp:186-275).
+//     cell's particles are one run of the sorted codes, found in the table when all radii
+//     have one level, else by two searches (neighborhood_binary_search.comp:186-275).
 //
 // Canonical rules where the reference's arithmetic is not exact:
 //  * the level k is the smallest with 2^k >= R, R the canonical fixed-point search

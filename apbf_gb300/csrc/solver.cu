@@ -562,7 +562,6 @@ __global__ void __launch_bounds__(256, GAUSS ? 4 : 3) k_density_lambda(PassA a) 
     if (skip) return;  // uniform over the grid
     const uint32_t n = a.d_len[kLenParticles];
     const uint32_t sub = threadIdx.x % L;
-    // passes after the first: the widths' uniformity of the first pass still holds
     // the position update of the Gauss kernel gathers the packed records and widths;
     // the other kernels gather the solve records, written every pass
     const bool write_rec = !GAUSS;
@@ -1606,7 +1605,7 @@ __global__ void __launch_bounds__(T *L, 896 / (T * L)) k_delta_tiles(PassB a, Ti
         // everything the particle needs to its end, so that no load waits behind the row
         const int4 shj = valid ? a.shift[j] : make_int4(0, 0, 0, 0), fj = a.filt[j];
         const float2 kcj = a.kc[j];
-        const int4 p = a.pk[j];  // w: the applied (learned) lambda
+        const int4 p = a.pk[j];  // w: the applied lambda
         const int pw = a.pos[j].w;  // the mass rides along
         const float pushed = a.prev_mode == 2 ? a.lam_prev[j] : 0.0f;
         const auto stage = [&](uint32_t k, uint32_t g) {
@@ -2336,8 +2335,8 @@ apbf_status tile_rows(apbf_ctx *ctx, cudaStream_t s) {
 }
 
 // One Jacobi pass over the tiles of the substep's rows.
+// (The learned warm start's first pass gathers features and takes the direct kernels.)
 static apbf_status launch_tiles(apbf_ctx *ctx, cudaStream_t s, const PassA &a, const PassB &b, const SolveOpts &o) {
-    const bool learned = o.learned;
     apbf_status r = APBF_OK;
     with_tile_shape(ctx, [&](auto tc, auto lc) {
         constexpr int T = decltype(tc)::value, L = decltype(lc)::value;
@@ -2353,12 +2352,8 @@ static apbf_status launch_tiles(apbf_ctx *ctx, cudaStream_t s, const PassA &a, c
             APBF_CUDA(launch_behind(o.later_pass && o.behind && !ctx->in_batch, k_density_tiles<T, L>, grid, T * L, rec * sizeof(int4), s, a,
                                     ctx->tile_plan[0]));
             APBF_AFTER_LAUNCH(ctx, s, "k_density_tiles");
-            if (learned) {  // the network's lambda replaces the plain one in this update
-                apbf_status q = mlp_lambda(ctx, s, a.target, a.target_m, a.target_s);
-                if (q != APBF_OK) return q;
-            }
             APBF_BEFORE_LAUNCH(ctx, s, "k_delta_tiles");
-            APBF_CUDA(launch_behind(!learned && !ctx->in_batch, k_delta_tiles<T, L>, grid, T * L, rec * (sizeof(int4) + sizeof(float2)), s, b,
+            APBF_CUDA(launch_behind(!ctx->in_batch, k_delta_tiles<T, L>, grid, T * L, rec * (sizeof(int4) + sizeof(float2)), s, b,
                                     ctx->tile_plan[0], ctx->tile_plan[1]));
             APBF_AFTER_LAUNCH(ctx, s, "k_delta_tiles");
             return APBF_OK;

@@ -1,17 +1,21 @@
-// sort.cu -- parallel primitives: stable LSD radix sort of (key, value) pairs and
-// inclusive prefix sum, both single-pass per digit / per scan with decoupled
-// look-back between tiles.
+// sort.cu -- parallel primitives: stable LSD radix sort of (key, value) pairs, and an
+// inclusive prefix sum in a single pass with decoupled look-back between tiles.
 //
 // Replaces algorithms::sort (source/algorithms.cpp:59-91, 4-bit digits, three
 // dispatches per digit plus a recursive scan) and algorithms::prefix_sum
 // (source/algorithms.cpp:93-118, recursive three-kernel block scan).
 //
-// Radix sort: one histogram kernel counts the digits of every pass in one read of
-// the keys; then one kernel per 8-bit digit ranks a tile of 2048 keys (8 warps x
-// 8 keys per lane, warp-striped so loads coalesce), publishes the tile's digit
-// counts, looks back over earlier tiles for its global offsets and writes the tile
-// out digit by digit.  A list of at most 4 096 pairs takes one block (k_sort_small).
-// Stability: inside a warp the keys are ranked in index order by votes; warps are combined in index order; tiles in tile order.
+// Radix sort, by the list's capacity:
+//  * up to 4 096 pairs: every pass in one block (k_sort_small);
+//  * up to 2^18: one histogram kernel counts the digits of every pass in one read of the
+//    keys; then one kernel per 8-bit digit (k_onesweep) ranks a tile of 2048 keys (8 warps x
+//    8 keys per lane, warp-striped so loads coalesce), publishes the tile's digit counts,
+//    looks back over earlier tiles for its global offsets and writes the tile out digit by
+//    digit (6- and 7-bit digits: at every size);
+//  * above: per digit a kernel that counts the tiles' digits (k_digit_count) and one that
+//    ranks and writes the tiles (k_digit_scatter), without any wait on another tile.
+// Stability: inside a warp the keys are ranked in index order by votes; warps are combined
+// in index order; tiles in tile order.
 // Every wait on another tile is bounded (kSpinLimit) and records
 // APBF_FLAG_SPIN_LIMIT instead of hanging.
 #include <algorithm>
@@ -244,13 +248,13 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const uint32_t *kin, 
 }
 
 // The same digit pass without any wait, for lists above kWaitFree keys (a million pairs of
-// 30 bits: 76 us, with the look-back 105 us, 121 us before either): k_digit_count
+// 30 bits: 58 us, with the look-back 105, 122 before either): k_digit_count
 // leaves the digit counts of every tile and, added up, of every group of kSortGroup tiles;
 // k_digit_scatter's tile reads the groups and the tiles of its own group in one round of
 // loads while its keys arrive.  The look-back's chain grows with the number of tiles (they
 // all run at once and read back eight at a time); this does not.  The keys that the scatter
 // ranks are older than the counts, so it loads and ranks them while the counts are taken and
-// waits for these only then: a million pairs take 59 us, 74 without.
+// waits for these only then (74 us without).
 template <int BITS>
 __global__ void __launch_bounds__(kSortThreads) k_digit_count(const uint32_t *kin, const uint32_t *d_count,
                                                               uint32_t max_count, uint32_t key_mask, int shift,
