@@ -1269,8 +1269,8 @@ struct WarpRow {
     }
 };
 
-// Entries k, k + L, ... below end of a list's row, walked by one thread: four gathers in
-// flight with the four entries behind them.
+// Entries k, k + L, ... below end of a list's row, walked by one thread: four gathers (`load`)
+// in flight with the four entries behind them.
 template <uint32_t L, typename G, typename F>
 __device__ __forceinline__ void lane_row(const uint32_t *row, size_t stride, uint32_t k, uint32_t end, G load, F f) {
     if (k >= end) return;
@@ -1279,7 +1279,7 @@ __device__ __forceinline__ void lane_row(const uint32_t *row, size_t stride, uin
     for (uint32_t u = 0; u < 4; ++u) j[u] = k + u * L < end ? row[(k + u * L) * stride] : 0u;
 #pragma unroll 1
     for (; k < end; k += 4u * L) {
-        int4 q[4];
+        decltype(load(0u)) q[4];
         uint32_t nj[4];
 #pragma unroll
         for (uint32_t u = 0; u < 4; ++u) q[u] = load(j[u]);
@@ -1287,7 +1287,7 @@ __device__ __forceinline__ void lane_row(const uint32_t *row, size_t stride, uin
         for (uint32_t u = 0; u < 4; ++u) nj[u] = k + (4u + u) * L < end ? row[(k + (4u + u) * L) * stride] : 0u;
 #pragma unroll
         for (uint32_t u = 0; u < 4; ++u)
-            if (k + u * L < end) f(j[u], q[u]);
+            if (k + u * L < end) f(q[u]);
 #pragma unroll
         for (uint32_t u = 0; u < 4; ++u) j[u] = nj[u];
     }
@@ -1412,7 +1412,7 @@ __global__ void __launch_bounds__(T *L, 1024 / (T * L)) k_density_tiles(PassA a,
         const bool by_warp = head.w == 0u && cnt > kTileDepth;
         const uint32_t end = by_warp ? (uint32_t)kTileDepth : cnt;
         lane_row<L>(a.idx + i, a.stride, depth + sub, end, [&](uint32_t j) { return a.pos[j]; },
-                    [&](uint32_t, const int4 &q) { add(q, __int_as_float(q.w) * APBF_FIX); });
+                    [&](const int4 &q) { add(q, __int_as_float(q.w) * APBF_FIX); });
         for (uint32_t left = __ballot_sync(0xffffffffu, sub == 0u && by_warp); left; left &= left - 1u) {
             const int src = __ffs(left) - 1;
             const WarpRow w(plan, a.idx, a.stride, i, cnt, p, src);
@@ -1731,10 +1731,17 @@ __global__ void __launch_bounds__(T *L, 896 / (T * L)) k_delta_tiles(PassB a, Ti
         }
         // what the tile does not hold, as in k_density_tiles
         const bool by_warp = head.w == 0u && cnt > kTileDepth;
+        struct Gathered {
+            int4 q;
+            float2 k;
+        };
         lane_row<L>(idx_arr + j, a.stride, depth + sub, by_warp ? (uint32_t)kTileDepth : cnt,
-                    [&](uint32_t g) { return a.pk[g & ~kNoDelta]; }, [&](uint32_t g, const int4 &q) {
-                        const float2 kk = h.packed ? kcj : a.kc[g & ~kNoDelta];
-                        add(q, __int_as_float(q.w) * APBF_FIX, gauss_pair(kk.x, kk.y), true);
+                    [&](uint32_t e) {
+                        const uint32_t g = e & ~kNoDelta;
+                        return Gathered{a.pk[g], h.packed ? kcj : a.kc[g]};
+                    },
+                    [&](const Gathered &x) {
+                        add(x.q, __int_as_float(x.q.w) * APBF_FIX, gauss_pair(x.k.x, x.k.y), true);
                     });
         for (uint32_t left = __ballot_sync(0xffffffffu, sub == 0u && by_warp); left; left &= left - 1u) {
             const int src = __ffs(left) - 1;
