@@ -967,7 +967,9 @@ __global__ void __launch_bounds__(256, 4) k_delta(PassB a) {
 // own rows, or from the pool (rests_by_lane).
 
 // Eight neighbouring particles, whose records share a line, keep together in the table and
-// so in the halo, which takes its order; the groups are spread.
+// so in the halo, which takes its order; the groups are spread.  A group that finds its eight
+// slots taken looks at the next eight, so that its keys take a step each and not eight (a tile
+// of many outside particles 68 -> 28 us, all tiles of a drop of 250 000 42 -> 35).
 __device__ __forceinline__ uint32_t tile_hash(uint32_t j, uint32_t mask) {
     return (((j >> 3) * 2654435761u >> 16) << 3 | (j & 7u)) & mask;
 }
@@ -1042,7 +1044,7 @@ __global__ void __launch_bounds__(256) k_tile_rows(TileRowsArgs a) {
                 uint32_t was = *(volatile uint32_t *)&s_key[h];
                 if (was == 0xffffffffu) was = atomicCAS(&s_key[h], 0xffffffffu, j);
                 if (was == j || was == 0xffffffffu) return 0x8000u | h;
-                h = (h + 1u) & (kSlots - 1);
+                h = (h + 8u) & (kSlots - 1);
             }
             s_full = 1u;  // far more outside particles than the halo holds
             return 0u;
