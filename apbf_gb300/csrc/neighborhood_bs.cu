@@ -236,7 +236,7 @@ struct BsArgs {
 // neighborhood_binary_search.comp:180-275 by groups of G threads (RowWalk): a thread per
 // cell finds its run, in the table of cells when all radii have one level, else by two
 // searches of the sorted codes.  The searches are about 40 dependent loads for each of 27
-// cells: 178 us at 64 019 particles, with the table 60.
+// cells: 178 us at 64 019 particles, with the table 55.
 template <int G>
 __global__ void __launch_bounds__(kBuildThreads) k_bs_rows(BsArgs a) {
     using Walk = RowWalk<G>;
@@ -395,7 +395,7 @@ apbf_status neighborhood_binary_search(apbf_ctx *ctx, float range_scale, cudaStr
     a.mask = ctx->bs_slots - 1u;
     a.levels = levels;
     APBF_BEFORE_LAUNCH(ctx, s, "k_bs_rows");
-    // threads per particle as in the Green search: 8 / 16 / 32 take 50 / 60 / 88 us at 64 019
+    // threads per particle as in the Green search: 8 / 16 / 32 take 56 / 66 / 93 us at 64 019
     if (cap <= 12288u)
         APBF_CUDA(launch_behind(behind, k_bs_rows<32>, grid_for(ctx, cap, RowWalk<32>::kParticles, 64), kBuildThreads, 0, s, a));
     else if (cap <= 32768u)

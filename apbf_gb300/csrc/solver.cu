@@ -1296,7 +1296,7 @@ __device__ __forceinline__ void lane_row(const uint32_t *row, size_t stride, uin
 }
 
 // A tile's density pass: T particles, L threads each.  At a million particles in a
-// waterfall (13.4 M pairs) 62 us against 92 us for the direct kernel, 26 against 35 us at
+// waterfall (13.4 M pairs) 55 us against 96 us for the direct kernel, 25 against 35 us at
 // 250 000 (4.45 M pairs).  Bound by the latency of a tile's own loads (three rounds: the
 // plan's words, the records, the barrier): half of a block's time, while the pair loop
 // issues at 55 % of the cycles; so the plan's words come in one round and before the
@@ -1563,7 +1563,7 @@ __device__ __noinline__ int4 box_push_from(int4 ip, float r, uint32_t id, const 
 }
 
 // A tile's position update.  fwd: the plan of the own rows, rev: that of the
-// transposed rows.  84 us at a million particles against 125 us for the direct kernel, 30
+// transposed rows.  79 us at a million particles against 127 us for the direct kernel, 29
 // against 37 us at 250 000.  Of its instructions the deferred filter's row tests took a
 // quarter and the boxes a fifth; both now reject by cheap bounds first.
 template <int T, int L>

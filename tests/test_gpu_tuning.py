@@ -199,3 +199,25 @@ def test_learned_substeps_identical_for_every_shape():
     for r in results[1:]:
         for k in r:
             assert np.array_equal(r[k], results[0][k]), k
+
+
+@pytest.mark.parametrize("lanes", [1, 2, 4, 8])
+def test_deferred_filter_identical_in_direct_passes(lanes):
+    """The same for solves of too few passes for the tiled kernels: the direct density and
+    position pass, each number of threads per particle."""
+    spec = scenes.water_drop(total=30_000, seed=8, basic_pbf=True)
+    out = []
+    for inline in (1, 0):
+        ctx = _ctx(spec, 4, maxn=192)
+        ctx.set_tuning(gather_lanes=lanes, pass_block=128, filter_in_density=inline)
+        ctx.profile_enable(True)
+        for _ in range(25):
+            ctx.substep(spec.dt)
+        names, _ = ctx.profile_read()
+        assert "k_density_lambda" in names and "k_density_tiles" not in names
+        ctx.check_status()
+        out.append(ctx.download()[0])
+        ctx.close()
+    assert np.any(out[0]["boundariness"] == 0) and np.any(out[0]["boundariness"] > 0)
+    for k in out[0]:
+        assert np.array_equal(out[0][k], out[1][k]), k
